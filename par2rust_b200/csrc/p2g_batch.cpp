@@ -35,10 +35,11 @@ namespace {
 // costs 0.62 us per slice plus 0.433 ns per symbol and slice (1.49 ms for
 // 1027 slices x 1920 symbols, 0.187 ms for 256 x 256), a folded tail item
 // 15 % more, an accumulating item 4 % more; a scan chain steps 64 bytes in
-// 0.76 us, a packet chain in 0.81 us; CRC32 streams at ~10 GB/s per CTA.
+// 0.44 us, a packet chain in 0.47 us; CRC32 streams at ~10 GB/s per CTA.
 constexpr double kEncRate = 2.309e6;    // symbols per ms per CTA, per slice
 constexpr double kBuildCost = 1430.0;   // per-slice fixed cost (table build, barrier, copy wait) in symbols
-constexpr double kChainMs = 7.6e-4;         // one MD5 chain step of 64 bytes
+constexpr double kChainMs = 4.4e-4;         // one MD5 chain step of 64 bytes, at most 128 lanes on the SM
+constexpr double kWideChain = 1.5;          // the same with 256
 constexpr double kFoldCost = 1.15, kAccCost = 1.04;
 // A finer tiling or a tail split must beat the current plan by 3 % in the
 // simulation: the model is good to a few percent, and smaller pieces cost
@@ -72,6 +73,7 @@ struct PlanJob {
     // Encode on the tensor cores: 16-row x 240-symbol items (kItemEncodeMma);
     // RG then counts 16-row tiles and ts is fixed at 240.
     bool mma = false;
+    uint32_t scan_slices = kScanSlices;  // slices per scan item
 };
 
 double finish_ms(const PlanJob& j) { return est_set_id_ms(j.n) + est_packet_item_ms(j.slice, j.R); }
@@ -106,7 +108,7 @@ void job_bands(const PlanJob& j, uint32_t* band_tiles, uint32_t* n_bands) {
     *band_tiles = bt;
     *n_bands = (j.tiles + bt - 1) / bt;
 }
-// one chain segment of every 256-row block over one band's bytes
+// one chain segment of every kChainRows-row block over one band's bytes
 inline double chain_ms(const PlanJob& j, uint32_t band_syms) {
     return ceil(j.R / (double)kChainRows) * md5_ms(2ull * band_syms) * 1.07 + kItemMs;
 }
@@ -134,10 +136,10 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
             pre.push_back({1e30, {ji, kItemSetId, 0, 0, 0, 0}});
             p.n_setid++;
         }
-        for (uint32_t f = 0; j.file_bytes && f < j.n; f += kScanSlices)  // longest chains: right after set ids
-            pre.push_back({1e29, {ji, kItemFileHash, f, std::min(kScanSlices, j.n - f), 0, 0}});
-        for (uint32_t s = 0; j.scans && s < j.S; s += kScanSlices) {
-            const uint32_t cnt = std::min(kScanSlices, j.S - s);
+        for (uint32_t f = 0; j.file_bytes && f < j.n; f += kHashFiles)  // longest chains: right after set ids
+            pre.push_back({1e29, {ji, kItemFileHash, f, std::min(kHashFiles, j.n - f), 0, 0}});
+        for (uint32_t s = 0; j.scans && s < j.S; s += j.scan_slices) {
+            const uint32_t cnt = std::min(j.scan_slices, j.S - s);
             pre.push_back({scan_ms(j, cnt), {ji, kItemScan, s, cnt, 0, 0}});
             p.n_scan++;
         }
@@ -323,7 +325,7 @@ Plan plan_tiles(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
             // alone on the GPU, equal items run in rounds of the CTAs that
             // the (long) MD5 scan items leave free: take the tile count with
             // the fewest, fullest rounds (choose_tiles)
-            const uint32_t scans = j.scans ? (j.S + kScanSlices - 1) / kScanSlices : 0;
+            const uint32_t scans = j.scans ? (j.S + j.scan_slices - 1) / j.scan_slices : 0;
             const uint32_t free_ctas = ctas > scans + 16 ? ctas - scans : ctas;
             uint32_t ts = 0, tiles = 0;
             choose_tiles(j.Np, j.RG, free_ctas, &ts, &tiles, tail_fold(j.R));
@@ -401,17 +403,16 @@ double est_encode_item_ms(uint32_t slices, uint32_t syms) {
     return (double)slices * (round_up(syms, 8) + kBuildCost) / kEncRate + kItemMs;
 }
 double est_scan_item_ms(uint64_t slice, uint32_t count) {
-    (void)count;  // the lanes run their chains side by side
-    return md5_ms(slice) + kItemMs;
+    return md5_ms(slice) * (count > kLoneScanSlices ? kWideChain : 1.0) + kItemMs;
 }
 // CRC32 streams from DRAM at ~10 GB/s per SM (16 warps)
 double est_crc_item_ms(uint64_t slice, uint32_t count) { return (double)slice * count / 1e7 + kItemMs; }
 double est_set_id_ms(uint32_t files) {
-    const double hashes = ceil(files / 256.0) * (md5_ms(P2G_HASH16K_LEN) + md5_ms(24 + 256));
+    const double hashes = ceil(files / 256.0) * (md5_ms(P2G_HASH16K_LEN) * kWideChain + md5_ms(24 + 256));
     const double sort = (double)files * files / 512.0 * 4e-6;
     return hashes + sort + md5_ms(12 + 16ull * files) + kItemMs;
 }
-double est_packet_item_ms(uint64_t slice, uint32_t rows) { return ceil(rows / 256.0) * md5_ms(36 + slice) + kItemMs; }
+double est_packet_item_ms(uint64_t slice, uint32_t rows) { return ceil(rows / (double)kChainRows) * md5_ms(36 + slice) + kItemMs; }
 
 // Plans depend only on the job's shape, and the search (tilings, tail
 // splits, each simulated) costs milliseconds of host time, so single-job
@@ -467,6 +468,7 @@ SingleJobPlan plan_single_job_uncached(uint64_t slice, uint32_t S, uint32_t R, u
     jobs[0].R = R;
     jobs[0].n = std::max(1u, n_files);
     jobs[0].scans = scans;
+    jobs[0].scan_slices = kLoneScanSlices;
     jobs[0].set_id = set_id;
     jobs[0].chains = chains && R;
     jobs[0].file_bytes = file_bytes;
@@ -711,7 +713,7 @@ extern "C" p2g_status p2g_batch_create(const p2g_batch_job* jobs, uint32_t n, ui
     const size_t o_jobs = take(sizeof(BatchJob) * n);
     const size_t o_items = take(sizeof(BatchItem) * b->n_items);
     // control block, zeroed before each run: queue head, each job's chain
-    // state (band counts, next band and token per 256-row block, set-id flag),
+    // state (band counts, next band and token per kChainRows-row block, set-id flag),
     // then the error word
     std::vector<uint64_t> bstate_off(n);
     uint64_t ctl_words = 1;

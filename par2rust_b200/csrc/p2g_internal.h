@@ -163,8 +163,16 @@ enum BatchItemKind : uint32_t {
 constexpr uint64_t kCrcItemBytes = 4u << 20;  // source bytes per CRC item
 constexpr uint32_t kItemKindMask = 0x7Fu;
 constexpr uint32_t kItemAccumulate = 0x80u;  // encode: XOR partial sums into zeroed rows
-constexpr uint32_t kScanSlices = 256;        // one slice per MD5 lane
-constexpr uint32_t kChainRows = 256;         // recovery rows per packet-MD5 chain token
+// One MD5 lane per slice, row or file.  128 lanes keep one warp on each of an
+// SM's four schedulers, where a chain runs at its latency (806 cycles a
+// block); 256 share them (1,244), which costs a little less SM time in all.
+// So a job alone, which waits for its chains, scans 128 slices an item; a
+// batch, which waits for the SMs, 256.
+constexpr uint32_t kScanSlices = 256;
+constexpr uint32_t kLoneScanSlices = 128;
+constexpr uint32_t kHashFiles = 128;         // files per whole-file MD5 item
+constexpr uint32_t kChainRows = 128;         // recovery rows per packet-MD5 chain token
+constexpr uint32_t kCrcMaxSlices = 256;      // slices per CRC32 item
 
 // Encode item fields: kind_rg = kItemEncode | acc | rg << 8 | log2(fold) << 24;
 // b = band << 16 | symbols.
@@ -208,7 +216,7 @@ struct BatchJob {
     uint8_t* scratch;          // 16*n file ids, then the 12+16*n main-packet body
     // Recovery-packet MD5 in chain segments: the symbol range is cut into
     // n_bands bands of band_syms; when the last encode item of a band
-    // completes, the chains of every 256-row block advance over that band's
+    // completes, the chains of every kChainRows-row block advance over that band's
     // bytes (n_bands 0: packets are separate items, as in the serving loop).
     uint32_t* bstate;            // per run, zeroed: [n_bands] items done, [Q] next band, [Q] token, [1] set id ready
     const uint32_t* band_items;  // [n_bands] encode items per band
@@ -235,7 +243,7 @@ struct SingleJobPlan {
     uint32_t zero_from_sym = 0;
     double predicted_ms = 0;
 };
-// file_bytes: largest file (non-zero: whole-file MD5 items, 256 files each);
+// file_bytes: largest file (non-zero: whole-file MD5 items, kHashFiles files each);
 // split_tail: the caller zeroes the columns from zero_from_sym, so the last
 // bands' encode items may be cut into accumulating slice ranges.
 // mma: encode items on the tensor cores (kItemEncodeMma).
@@ -263,10 +271,10 @@ double encode_cost_ms(uint64_t slice, uint32_t S, uint32_t R, bool mma);
 bool prefer_mma(uint64_t slice, uint32_t S, uint32_t R);
 double est_scan_item_ms(uint64_t slice, uint32_t count);
 double est_crc_item_ms(uint64_t slice, uint32_t count);
-// slices per CRC item: ~kCrcItemBytes, at least 1, at most kScanSlices
+// slices per CRC item: ~kCrcItemBytes, at least 1, at most kCrcMaxSlices
 inline uint32_t crc_item_slices(uint64_t slice) {
     const uint64_t n = kCrcItemBytes / slice;
-    return (uint32_t)(n < 1 ? 1 : n > kScanSlices ? kScanSlices : n);
+    return (uint32_t)(n < 1 ? 1 : n > kCrcMaxSlices ? kCrcMaxSlices : n);
 }
 double est_set_id_ms(uint32_t files);
 double est_packet_item_ms(uint64_t slice, uint32_t rows);

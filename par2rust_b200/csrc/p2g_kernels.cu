@@ -547,16 +547,26 @@ __device__ __forceinline__ uint32_t rotl32(uint32_t x, int s) { return __funnels
 #define P2G_G(x, y, z) ((y) ^ ((z) & ((x) ^ (y))))
 #define P2G_H(x, y, z) ((x) ^ (y) ^ (z))
 #define P2G_I(x, y, z) ((y) ^ ((x) | ~(z)))
-// a + x + t does not depend on the previous step's output (b), so it is
-// formed first; the chain through b is then round function -> add ->
-// rotate -> add.
+// The chain through b is what bounds every MD5 here (one stream a lane, each
+// step needs the one before): it is the round function (one LOP3), one add
+// and rotate-plus-add (one instruction on this machine, 4 cycles).  Two
+// things keep it at that: x + t is formed on the multiply-add pipe (`one` is 1
+// at run time, so it stays a multiply-add), and a, x + t and f are summed in
+// ONE three-input add after f, which stays on the round function's pipe.  A
+// two-input add there crosses pipes and costs 2 cycles more a step.  Measured,
+// registers only, cycles a 64-byte block with 1 / 2 / 4 warps on a scheduler:
+// 806 / 1,244 / 2,459, against 1,168 / 1,222 / 1,796 with a + x + t summed
+// first.  So chains run one warp to a scheduler (kHashThreads).
+__constant__ uint32_t c_one = 1;
 #define P2G_STEP(f, a, b, c, d, x, t, s)                    \
     {                                                       \
-        const uint32_t _axt = (a) + ((x) + (t));            \
-        (a) = rotl32(_axt + f((b), (c), (d)), (s)) + (b);   \
+        const uint32_t _xt = mad1((x), one, (t));           \
+        const uint32_t _u = (a) + _xt + f((b), (c), (d));   \
+        (a) = rotl32(_u, (s)) + (b);                        \
     }
 
 __device__ __forceinline__ void md5_compress(uint32_t st[4], const uint32_t m[16]) {
+    const uint32_t one = c_one;
     uint32_t a = st[0], b = st[1], c = st[2], d = st[3];
     P2G_STEP(P2G_F, a, b, c, d, m[0], 0xd76aa478u, 7);
     P2G_STEP(P2G_F, d, a, b, c, m[1], 0xe8c7b756u, 12);
@@ -731,7 +741,11 @@ __device__ void md5_stream(uint32_t st[4], const uint32_t* pre, uint32_t pre_byt
 // Blocks that contain prefix words, padding, or data past the last whole
 // copy unit take the direct (generic) path.
 // ---------------------------------------------------------------------------
-constexpr int kHashThreads = 256;  // 8 warps: two MD5 warps per SM sub-partition keep full chain speed
+// MD5 lanes of a CTA: one warp per SM sub-partition, since two share its issue
+// rate (806 against 1,244 cycles a block, at the step above); the wide form
+// only where there are more streams than SMs x kHashThreads.
+constexpr int kHashThreads = 128;
+constexpr int kHashThreadsWide = 256;
 constexpr int kRingUnits = 8;
 constexpr int kRingAhead = 4;
 constexpr int kRingLaneBytes = kRingUnits * 64 + 16;  // +16: lanes land on distinct bank groups
@@ -828,7 +842,7 @@ __device__ void md5_range_ring(uint32_t st[4], const uint32_t* pre, const uint8_
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(kHashThreads) md5_slices_kernel(const uint8_t* __restrict__ src, uint64_t stride,
+__global__ void __launch_bounds__(kHashThreadsWide) md5_slices_kernel(const uint8_t* __restrict__ src, uint64_t stride,
                                                                   uint32_t count, uint64_t slice_size,
                                                                   p2g_slice_checksum* __restrict__ out) {
     extern __shared__ __align__(16) uint8_t ring[];
@@ -846,7 +860,7 @@ __global__ void __launch_bounds__(kHashThreads) md5_slices_kernel(const uint8_t*
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(kHashThreads) md5_files_kernel(const uint8_t* __restrict__ base,
+__global__ void __launch_bounds__(kHashThreadsWide) md5_files_kernel(const uint8_t* __restrict__ base,
                                                                  const FileSpan* __restrict__ spans, uint32_t n,
                                                                  uint8_t* __restrict__ out16) {
     extern __shared__ __align__(16) uint8_t ring[];
@@ -869,7 +883,7 @@ struct RecvPrefix {
 };
 
 template <bool VEC>
-__global__ void __launch_bounds__(kHashThreads) md5_recovery_kernel(const uint8_t* __restrict__ rec, uint64_t stride, uint32_t count,
+__global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_kernel(const uint8_t* __restrict__ rec, uint64_t stride, uint32_t count,
                                     uint64_t slice_size, RecvPrefix pfx, uint32_t first_exp,
                                     uint8_t* __restrict__ out16) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -894,7 +908,7 @@ __global__ void __launch_bounds__(kHashThreads) md5_recovery_kernel(const uint8_
 // with the chain state kept in `state` (4 words per row) between calls.
 // b_from == 0 starts a chain; `final` writes the digest instead of the state.
 template <bool VEC>
-__global__ void __launch_bounds__(kHashThreads) md5_recovery_range_kernel(const uint8_t* __restrict__ rec, uint64_t stride, uint32_t count,
+__global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_range_kernel(const uint8_t* __restrict__ rec, uint64_t stride, uint32_t count,
                                           uint64_t slice_size, RecvPrefix pfx, uint32_t first_exp,
                                           uint32_t* __restrict__ state, uint64_t b_from, uint64_t b_to, int final,
                                           uint8_t* __restrict__ out16) {
@@ -1085,7 +1099,7 @@ __global__ void gather_host_kernel(const uint64_t* __restrict__ seg, uint32_t n_
 // runs that job's finish step itself, so the launch has no inter-CTA waits.
 //
 // Shared memory: the encode region (tables, TMA ring, mbarriers), a cp.async
-// ring of kBatchRingLane bytes for each of the kHashThreads MD5 lanes, the
+// ring of kBatchRingLane bytes for each of the kHashThreadsWide MD5 lanes, the
 // CRC32 tables and a few words of per-CTA state.
 // ---------------------------------------------------------------------------
 // The persistent kernel runs its encode items on a 3-deep TMA ring (3 slices
@@ -1097,7 +1111,7 @@ constexpr size_t kBatchEncBytes = (encode_smem_bytes<kEncChunks, 4, kBatchEncSta
 constexpr int kBatchRingUnits = 6;
 constexpr int kBatchRingAhead = 4;
 constexpr int kBatchRingLane = kBatchRingUnits * 64 + 16;
-constexpr size_t kBatchRingBytes = (size_t)kHashThreads * kBatchRingLane;
+constexpr size_t kBatchRingBytes = (size_t)kHashThreadsWide * kBatchRingLane;
 // Tensor-core items reuse the encode region and the MD5 rings for their
 // operand and input rings; their barriers, the TMEM address, an abort flag,
 // the pipeline state and the G^-1 tables live past the other regions, so
@@ -1244,13 +1258,13 @@ __device__ __forceinline__ bool id_eq(const uint4& a, const uint4& b) {
 // line: their chain loops then get registers of their own rather than a
 // share of the persistent kernel's 128, which spills.
 //
-// Slice MD5 of slices [first, first+count) of job J on the kHashThreads
+// Slice MD5 of slices [first, first+count) of job J on up to kHashThreadsWide
 // lanes (one slice each, staged through the lane's ring).  The other warps
 // idle: the lanes are bound by their chains, and the SM is the item's alone.
 template <bool VEC>
 __device__ __noinline__ void batch_scan(const BatchJob& J, uint32_t first, uint32_t count, uint32_t ring) {
     const int tid = threadIdx.x;
-    if (tid < kHashThreads && (uint32_t)tid < count) {
+    if (tid < kHashThreadsWide && (uint32_t)tid < count) {
         const uint32_t s = first + tid;
         uint32_t st[4];
         md5_init(st);
@@ -1265,7 +1279,7 @@ __device__ __noinline__ void batch_scan(const BatchJob& J, uint32_t first, uint3
 template <bool VEC>
 __device__ __noinline__ void batch_file_hash(const BatchJob& J, uint32_t first, uint32_t count, uint32_t ring) {
     const int tid = threadIdx.x;
-    if (tid < kHashThreads && (uint32_t)tid < count) {
+    if (tid < kHashThreadsWide && (uint32_t)tid < count) {
         const uint32_t f = first + tid;
         uint32_t st[4];
         md5_init(st);
@@ -1302,8 +1316,8 @@ __device__ void batch_set_id(const BatchJob& J, uint32_t ring, uint32_t* sid) {
     const uint32_t n = J.n_files;
     uint4* ids = reinterpret_cast<uint4*>(J.scratch);
     uint8_t* body = J.scratch + 16 * (size_t)n;
-    if (tid < kHashThreads) {
-        for (uint32_t f = tid; f < n; f += kHashThreads) {
+    if (tid < kHashThreadsWide) {
+        for (uint32_t f = tid; f < n; f += kHashThreadsWide) {
             const uint64_t off = J.files[2 * f], len = J.files[2 * f + 1];
             uint32_t h[4];
             md5_init(h);
@@ -1477,9 +1491,12 @@ __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32
     }
 }
 
-__device__ void advance_all(const BatchJob& J, uint32_t ring, uint32_t* misc) {
+// All row blocks, starting with block `first` mod Q: the CTAs that complete
+// neighbouring bands start on different blocks, so that the blocks advance
+// side by side.
+__device__ void advance_all(const BatchJob& J, uint32_t first, uint32_t ring, uint32_t* misc) {
     const uint32_t Q = (J.R + kChainRows - 1) / kChainRows;
-    for (uint32_t q = 0; q < Q; ++q) try_advance(J, q, ring, misc);
+    for (uint32_t i = 0; i < Q; ++i) try_advance(J, (first + i) % Q, ring, misc);
 }
 
 // MMA: the launch has tensor-core items (mma_ginv set).  The variant without
@@ -1581,7 +1598,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
                     atomicExch(J.bstate + J.n_bands + 2 * ((J.R + kChainRows - 1) / kChainRows), 1u);
                 }
                 __syncthreads();
-                advance_all(J, ring, misc);
+                advance_all(J, 0, ring, misc);
             }
             continue;
         }
@@ -1609,7 +1626,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             __syncthreads();
             if (!misc[1]) continue;
             __threadfence();  // acquire: the whole band is visible from here on
-            advance_all(J, ring, misc);
+            advance_all(J, band, ring, misc);
             continue;
         }
         if (kind == kItemEncode) {
@@ -1650,7 +1667,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             __syncthreads();
             if (!misc[1]) continue;
             __threadfence();  // acquire: the whole band is visible from here on
-            advance_all(J, ring, misc);
+            advance_all(J, band, ring, misc);
         }
     }
     if (MMA) {  // every MMA issued has completed before TMEM is given back
@@ -1968,7 +1985,9 @@ struct HashGrid {
 };
 static HashGrid hash_grid(uint32_t streams) {
     const unsigned warps = (streams + 31) / 32;
-    const unsigned wpb = warps < (unsigned)(kHashThreads / 32) ? warps : (unsigned)(kHashThreads / 32);
+    const unsigned max_wpb =
+        (streams > (unsigned)sm_count() * kHashThreads ? kHashThreadsWide : kHashThreads) / 32;
+    const unsigned wpb = warps < max_wpb ? warps : max_wpb;
     HashGrid g;
     g.threads = wpb * 32;
     g.blocks = (streams + g.threads - 1) / g.threads;

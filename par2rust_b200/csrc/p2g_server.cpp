@@ -17,7 +17,7 @@
 //   set id  hash16k, file ids, set id
 //   encode  (row group, symbol tile, slice chunk); chunks of one tile XOR
 //           into zeroed rows, so no item runs longer than ~wave_ms/4
-//   packet  recovery-packet MD5s of up to 256 rows, issued once every
+//   packet  recovery-packet MD5s of up to 128 rows, issued once every
 //           encode item and the set-id item of the job have completed
 // A job is complete when its last item's wave has completed; its outputs
 // stay in device memory until the caller releases it.
@@ -208,7 +208,7 @@ void plan_job(p2g_server* s, SJob& j) {
             }
         }
     }
-    j.pkt_ms_per_item = est_packet_item_ms(j.slice, std::min(j.R, kScanSlices));
+    j.pkt_ms_per_item = est_packet_item_ms(j.slice, std::min(j.R, kChainRows));
 }
 
 // Admit queued jobs in arrival order while budget and slots allow.
@@ -427,7 +427,7 @@ p2g_status launch_wave(p2g_server* s, bool* launched) {
                 j.outstanding++;
                 got += ms;
             } else if (j.setid_done && j.enc_done == j.enc_total && j.pkt_issued < j.R) {
-                const uint32_t rows = std::min(kScanSlices, j.R - j.pkt_issued);
+                const uint32_t rows = std::min(kChainRows, j.R - j.pkt_issued);
                 w.items.push_back({&j, {j.slot, kItemPacket, j.pkt_issued, rows, 0, 0}});
                 j.pkt_issued += rows;
                 j.outstanding++;
