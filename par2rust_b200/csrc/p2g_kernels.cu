@@ -733,28 +733,37 @@ __device__ void md5_stream(uint32_t st[4], const uint32_t* pre, uint32_t pre_byt
 // ---------------------------------------------------------------------------
 // Staged MD5 streams.  With 32 lanes of a warp each hashing a different
 // stream, direct global loads leave every block waiting on 32 scattered
-// cache lines.  Instead each lane pulls its stream through a private ring of
-// kRingUnits 64-byte units in shared memory with cp.async, kRingAhead units
-// ahead of the block being compressed, and reads message words back with
-// 128-bit shared loads.  PW = prefix words (the message is PW prefix words
-// ‖ data); data must be 16-byte aligned when VEC (else 4-byte copies).
-// Blocks that contain prefix words, padding, or data past the last whole
-// copy unit take the direct (generic) path.
+// cache lines.  Instead the warp pulls its 32 streams through private rings
+// of UNITS 64-byte units in shared memory with cp.async, AHEAD units ahead.
+// It copies together: four lanes fetch one stream's unit, so an instruction
+// touches 8 runs of 64 bytes; a lane that fetched its own unit (32 scattered
+// 16-byte pieces an instruction) took four times the L1 and L2 requests, and
+// its warp's shared-memory reads queued behind them.  The next block's words
+// are read back with 128-bit shared loads before the current one is
+// compressed, so that only the MD5 steps themselves are on the chain: 8,192-
+// block slice chains inside the 538 MB job went from 0.497 us a block (976
+// cycles) to 0.44, and 200 packet chains alone from 0.50 to 0.43.  PW = prefix words (the message is PW prefix words ‖
+// data).  Data is 16-byte aligned when VEC; else 4-byte aligned, and the ring
+// holds it from the 16-byte boundary below its start, each block's words being
+// picked from 20 by the lane's offset (34 selects a block, beside the chain;
+// 4-byte copies took 16 instructions a unit and 0.77 us a block).  Blocks that
+// contain prefix words, padding, or data past the last whole copy unit take
+// the direct (generic) path.
 // ---------------------------------------------------------------------------
 // MD5 lanes of a CTA: one warp per SM sub-partition, since two share its issue
 // rate (806 against 1,244 cycles a block, at the step above); the wide form
 // only where there are more streams than SMs x kHashThreads.
 constexpr int kHashThreads = 128;
 constexpr int kHashThreadsWide = 256;
-constexpr int kRingUnits = 8;
-constexpr int kRingAhead = 4;
-constexpr int kRingLaneBytes = kRingUnits * 64 + 16;  // +16: lanes land on distinct bank groups
+// Ring depth: 8 units ahead are 3.4 us at 0.42 us a block.  UNITS >= AHEAD + 2:
+// while unit u + 1 + AHEAD is fetched, block u + 1 reads units u and u + 1.
+constexpr int kRingUnits = 12;
+constexpr int kRingAhead = 8;
+__host__ __device__ constexpr int ring_lane_bytes(int units) { return units * 64 + 16; }  // +16: lanes land on distinct bank groups
+constexpr int kRingLaneBytes = ring_lane_bytes(kRingUnits);
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -762,81 +771,126 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int PW, bool VEC, int UNITS = kRingUnits, int AHEAD = kRingAhead>
+// All 32 lanes of a warp call this together with the same b_from; a lane
+// without a stream passes len = 0 and b_to = 0.  SAME: the streams of a warp
+// have one length (lanes without one compress stale words; their state is not
+// used); with VEC they then have one last ring block too, and no state need be
+// held back.
+// `ring` is the warp's first lane's ring, the others follow
+// ring_lane_bytes(UNITS) apart.
+template <int PW, bool VEC, bool SAME, int UNITS = kRingUnits, int AHEAD = kRingAhead>
 __device__ void md5_range_ring(uint32_t st[4], const uint32_t* pre, const uint8_t* data, uint64_t len,
                                uint64_t b_from, uint64_t b_to, uint32_t ring) {
+    static_assert(UNITS >= AHEAD + 2, "a fetch must not reach the units being read");
     constexpr uint32_t pre_bytes = 4 * PW;
-    constexpr int SH = (4 - (PW & 3)) & 3;  // word offset of a block's first word in its aligned quad
-    constexpr int NQ = SH ? 5 : 4;          // quads touched per block
+    constexpr int SH = (4 - (PW & 3)) & 3;  // VEC: word offset of a block's first word in its aligned quad
+    constexpr int NQ = SH || !VEC ? 5 : 4;  // quads touched per block
+    constexpr uint32_t LO = PW ? 1 : 0;     // block b's words lie in units b - LO .. b + HI
+    constexpr uint32_t HI = VEC || PW ? 0 : 1;
+    static_assert(PW <= 13, "a shifted block's words end in its own unit");
+    constexpr uint32_t STRIDE = ring_lane_bytes(UNITS);
+    constexpr int COPIES = 4;               // cp.async instructions per unit of 32 streams
+    const uint32_t lane = threadIdx.x & 31;
+    // words between the 16-byte boundary the ring starts at and the data
+    const uint32_t k = VEC ? 0u : (uint32_t)((uintptr_t)data & 15) / 4;
+    const uint32_t sh = (k - PW) & 3;
     const uint64_t total = pre_bytes + len;
     const uint64_t nblocks = (total + 8) / 64 + 1;
     const uint64_t last_start = (nblocks - 1) * 64;
     if (b_to > nblocks) b_to = nblocks;
     // whole 64-byte units that can go through the ring
-    const uint64_t fetch_bytes = VEC ? (len & ~15ull) : (len & ~3ull);
-    const uint64_t n_units = fetch_bytes / 64;
+    const uint64_t n_units = (len + 4 * k) / 64;
     // ring-eligible blocks: no prefix word, all data words inside whole units
-    const uint64_t rb0 = (pre_bytes + 63) / 64;
-    const uint64_t rb1 = n_units * 16 >= 16 - PW ? (n_units * 16 + PW) / 16 : 0;  // blocks b with 16b+16-PW <= 16*n_units
-    uint64_t b = b_from;
-    uint32_t m[16];
+    // (blocks b with 16b + 16 - PW + k <= 16 n_units)
+    constexpr uint64_t rb0 = (pre_bytes + 63) / 64;
+    const uint64_t rb1 = n_units * 16 + PW >= k ? (n_units * 16 + PW - k) / 16 : 0;
     auto generic = [&](uint64_t blk) {
+        uint32_t m[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) m[i] = md5_stream_word(pre, pre_bytes, data, len, total, last_start, 64 * blk + 4 * i);
         md5_compress(st, m);
     };
-    for (; b < b_to && (b < rb0 || b >= rb1); ++b) generic(b);
-    const uint64_t fast_end = rb1 < b_to ? rb1 : b_to;
-    if (b < fast_end) {
-        auto fetch = [&](uint64_t u, uint32_t slot) {  // one unit = one commit group (possibly empty)
-            if (u < n_units) {
-                const uint8_t* g = data + 64 * u;
-                const uint32_t d = ring + slot * 64;
-                if (VEC) {
+    uint64_t b = b_from;
+    if (PW)
+        for (; b < b_to && b < rb0; ++b) generic(b);
+    const uint32_t b0 = (uint32_t)(b_from > rb0 ? b_from : rb0);  // the same in every lane
+    const uint32_t end = (uint32_t)(rb1 < b_to ? rb1 : b_to);     // this lane's ring blocks: [b0, end)
+    const uint32_t end_max = __reduce_max_sync(0xFFFFFFFFu, end);
+    if (end_max > b0) {
+        // copy i of a unit: stream i * (32 / COPIES) + lane / COPIES, piece lane % COPIES
+        constexpr uint32_t PIECE = 64 / COPIES;
+        const uint32_t piece = lane % COPIES, sub = lane / COPIES;
+        const uint32_t dst0 = ring + sub * STRIDE + piece * PIECE;
+        const uint8_t* src[COPIES];
+        uint32_t units[COPIES];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) cp_async16(d + 16 * q, g + 16 * q);
-                } else {
+        for (int i = 0; i < COPIES; ++i) {
+            const int from = i * (32 / COPIES) + (int)sub;
+            src[i] = reinterpret_cast<const uint8_t*>(
+                         __shfl_sync(0xFFFFFFFFu, (unsigned long long)(uintptr_t)data - 4 * k, from)) +
+                     piece * PIECE;
+            units[i] = __shfl_sync(0xFFFFFFFFu, (uint32_t)n_units, from);
+        }
+        auto fetch = [&](uint32_t u, uint32_t slot) {  // one unit of every stream = one commit group
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) cp_async4(d + 4 * q, g + 4 * q);
-                }
-            }
+            for (int i = 0; i < COPIES; ++i)
+                if (u < units[i]) cp_async16(dst0 + i * (32 / COPIES) * STRIDE + slot * 64, src[i] + 64ull * u);
             cp_async_commit();
         };
-        // units of block b: [lo(b), hi(b)] with hi(b) = floor((16b + 15 - PW) / 16)
-        const uint64_t first_w = 16 * b - PW;
-        const uint64_t u_lo = first_w / 16;
-        const uint64_t u_hi0 = (first_w + 15) / 16;
-        for (uint64_t u = u_lo; u < u_hi0 + AHEAD; ++u) fetch(u, (uint32_t)(u % UNITS));
-        // Each block moves the ring by one unit (16 words): the next unit to
-        // fetch, its slot and the slot of the block's first aligned quad are
-        // stepped as 32-bit counters, so no 64-bit remainder (the ring need
-        // not be a power of two) sits between one compress and the next.
         constexpr uint32_t RW = 16 * UNITS;  // ring size in words
-        uint64_t u_next = u_hi0 + AHEAD;
-        uint32_t f_slot = (uint32_t)(u_next % UNITS);
-        uint32_t w_slot = (uint32_t)(((16 * b - PW) & ~3ull) % RW);
-        for (; b < fast_end; ++b) {
-            fetch(u_next, f_slot);
-            ++u_next;
-            f_slot = f_slot + 1 == (uint32_t)UNITS ? 0u : f_slot + 1;
-            cp_async_wait<AHEAD>();
-            uint32_t q[NQ * 4];
+        const uint32_t my_ring = ring + lane * STRIDE;
+        uint32_t w_slot = (uint32_t)(((16ull * b0 + k - PW) & ~3ull) % RW);
+        uint32_t q[NQ * 4];
+        auto read = [&] {  // the words of the block at w_slot; steps w_slot by one block
 #pragma unroll
             for (int i = 0; i < NQ; ++i) {
                 uint32_t widx = w_slot + 4 * i;
                 if (widx >= RW) widx -= RW;
-                const uint4 v = lds128(ring + widx * 4);
+                const uint4 v = lds128(my_ring + widx * 4);
                 q[4 * i] = v.x;
                 q[4 * i + 1] = v.y;
                 q[4 * i + 2] = v.z;
                 q[4 * i + 3] = v.w;
             }
             w_slot = w_slot + 16 >= RW ? w_slot + 16 - RW : w_slot + 16;
+        };
+        __syncwarp();  // every lane is done with an earlier call's ring
+        for (uint32_t u = b0 - LO; u <= b0 + HI + AHEAD; ++u) fetch(u, u % UNITS);
+        cp_async_wait<AHEAD>();
+        __syncwarp();
+        read();
+        // slots are stepped as 32-bit counters: no remainder by the (non-
+        // power-of-two) ring size between one compress and the next
+        uint32_t f_slot = (b0 + 1 + HI + AHEAD) % UNITS;
+        for (uint32_t blk = b0; blk < end_max; ++blk) {
+            uint32_t m[16];
+            if (VEC) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) m[i] = q[SH + i];
-            md5_compress(st, m);
+                for (int i = 0; i < 16; ++i) m[i] = q[SH + i];
+            } else {
+                uint32_t h[17];
+#pragma unroll
+                for (int i = 0; i < 17; ++i) h[i] = sh & 2 ? q[i + 2] : q[i];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) m[i] = sh & 1 ? h[i + 1] : h[i];
+            }
+            cp_async_wait<AHEAD - 1>();  // unit blk + 1 + HI
+            __syncwarp();                // ... of every lane; and every lane has read block blk
+            fetch(blk + 1 + HI + AHEAD, f_slot);
+            f_slot = f_slot + 1 == (uint32_t)UNITS ? 0u : f_slot + 1;
+            read();  // block blk + 1 (past a stream's end: stale words, not used)
+            if (SAME && VEC) {
+                md5_compress(st, m);
+            } else {  // selected, not branched around: the copies above overlap the steps
+                uint32_t t[4] = {st[0], st[1], st[2], st[3]};
+                md5_compress(t, m);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) st[i] = blk < end ? t[i] : st[i];
+            }
         }
         cp_async_wait<0>();
+        __syncwarp();
+        if (b < end) b = end;
     }
     for (; b < b_to; ++b) generic(b);
 }
@@ -847,11 +901,12 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_slices_kernel(const uint
                                                                   p2g_slice_checksum* __restrict__ out) {
     extern __shared__ __align__(16) uint8_t ring[];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
+    const bool live = i < count;
     uint32_t st[4];
     md5_init(st);
-    md5_range_ring<0, VEC>(st, nullptr, src + (size_t)i * stride, slice_size, 0, ~0ull,
-                           smem_u32(ring) + threadIdx.x * kRingLaneBytes);
+    md5_range_ring<0, VEC, true>(st, nullptr, src + (live ? (size_t)i * stride : 0), live ? slice_size : 0, 0,
+                                         live ? ~0ull : 0, smem_u32(ring) + (threadIdx.x & ~31u) * kRingLaneBytes);
+    if (!live) return;
     uint32_t* o = reinterpret_cast<uint32_t*>(&out[i]);
     o[0] = st[0];
     o[1] = st[1];
@@ -865,12 +920,13 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_files_kernel(const uint8
                                                                  uint8_t* __restrict__ out16) {
     extern __shared__ __align__(16) uint8_t ring[];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const bool live = i < n;
     uint32_t st[4];
-    const FileSpan sp = spans[i];
+    const FileSpan sp = live ? spans[i] : FileSpan{0, 0};
     md5_init(st);
-    md5_range_ring<0, VEC>(st, nullptr, base + sp.offset, sp.length, 0, ~0ull,
-                           smem_u32(ring) + threadIdx.x * kRingLaneBytes);
+    md5_range_ring<0, VEC, false>(st, nullptr, base + sp.offset, sp.length, 0, live ? ~0ull : 0,
+                                         smem_u32(ring) + (threadIdx.x & ~31u) * kRingLaneBytes);
+    if (!live) return;
     uint32_t* o = reinterpret_cast<uint32_t*>(out16 + 16 * (size_t)i);
     o[0] = st[0];
     o[1] = st[1];
@@ -887,7 +943,7 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_kernel(const ui
                                     uint64_t slice_size, RecvPrefix pfx, uint32_t first_exp,
                                     uint8_t* __restrict__ out16) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= count) return;
+    const bool live = r < count;
     uint32_t pre[9];
 #pragma unroll
     for (int i = 0; i < 8; ++i) pre[i] = pfx.w[i];
@@ -895,8 +951,9 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_kernel(const ui
     extern __shared__ __align__(16) uint8_t ring[];
     uint32_t st[4];
     md5_init(st);
-    md5_range_ring<9, VEC>(st, pre, rec + (size_t)r * stride, slice_size, 0, ~0ull,
-                            smem_u32(ring) + threadIdx.x * kRingLaneBytes);
+    md5_range_ring<9, VEC, true>(st, pre, rec + (live ? (size_t)r * stride : 0), live ? slice_size : 0, 0,
+                                         live ? ~0ull : 0, smem_u32(ring) + (threadIdx.x & ~31u) * kRingLaneBytes);
+    if (!live) return;
     uint32_t* o = reinterpret_cast<uint32_t*>(out16 + 16 * (size_t)r);
     o[0] = st[0];
     o[1] = st[1];
@@ -913,14 +970,14 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_range_kernel(co
                                           uint32_t* __restrict__ state, uint64_t b_from, uint64_t b_to, int final,
                                           uint8_t* __restrict__ out16) {
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= count) return;
+    const bool live = r < count;
     uint32_t pre[9];
 #pragma unroll
     for (int i = 0; i < 8; ++i) pre[i] = pfx.w[i];
     pre[8] = first_exp + r;
     extern __shared__ __align__(16) uint8_t ring[];
     uint32_t st[4];
-    if (b_from == 0) {
+    if (b_from == 0 || !live) {
         md5_init(st);
     } else {
         const uint4 v = reinterpret_cast<const uint4*>(state)[r];
@@ -929,8 +986,9 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_range_kernel(co
         st[2] = v.z;
         st[3] = v.w;
     }
-    md5_range_ring<9, VEC>(st, pre, rec + (size_t)r * stride, slice_size, b_from, b_to,
-                            smem_u32(ring) + threadIdx.x * kRingLaneBytes);
+    md5_range_ring<9, VEC, true>(st, pre, rec + (live ? (size_t)r * stride : 0), live ? slice_size : 0, b_from,
+                                         live ? b_to : 0, smem_u32(ring) + (threadIdx.x & ~31u) * kRingLaneBytes);
+    if (!live) return;
     if (final) {
         uint32_t* o = reinterpret_cast<uint32_t*>(out16 + 16 * (size_t)r);
         o[0] = st[0];
@@ -1108,10 +1166,11 @@ __global__ void gather_host_kernel(const uint64_t* __restrict__ seg, uint32_t n_
 // that holds a folded tail item (4 tiles).
 constexpr int kBatchEncStages = 3;
 constexpr size_t kBatchEncBytes = (encode_smem_bytes<kEncChunks, 4, kBatchEncStages>() + 15) / 16 * 16;
-constexpr int kBatchRingUnits = 6;
+constexpr int kBatchRingUnits = 6;  // 256 lanes; the deeper ring of kRingUnits for 128
 constexpr int kBatchRingAhead = 4;
-constexpr int kBatchRingLane = kBatchRingUnits * 64 + 16;
+constexpr int kBatchRingLane = ring_lane_bytes(kBatchRingUnits);
 constexpr size_t kBatchRingBytes = (size_t)kHashThreadsWide * kBatchRingLane;
+static_assert((size_t)kHashThreads * kRingLaneBytes <= kBatchRingBytes, "128 lanes' deep rings fit too");
 // Tensor-core items reuse the encode region and the MD5 rings for their
 // operand and input rings; their barriers, the TMEM address, an abort flag,
 // the pipeline state and the G^-1 tables live past the other regions, so
@@ -1261,16 +1320,19 @@ __device__ __forceinline__ bool id_eq(const uint4& a, const uint4& b) {
 // Slice MD5 of slices [first, first+count) of job J on up to kHashThreadsWide
 // lanes (one slice each, staged through the lane's ring).  The other warps
 // idle: the lanes are bound by their chains, and the SM is the item's alone.
-template <bool VEC>
+template <bool VEC, int LANES>
 __device__ __noinline__ void batch_scan(const BatchJob& J, uint32_t first, uint32_t count, uint32_t ring) {
     const int tid = threadIdx.x;
-    if (tid < kHashThreadsWide && (uint32_t)tid < count) {
-        const uint32_t s = first + tid;
+    if (tid < LANES && (uint32_t)(tid & ~31) < count) {
+        const bool live = (uint32_t)tid < count;
+        const uint32_t s = first + (live ? tid : 0);
+        constexpr int UNITS = LANES > kHashThreads ? kBatchRingUnits : kRingUnits;
+        constexpr int AHEAD = LANES > kHashThreads ? kBatchRingAhead : kRingAhead;
         uint32_t st[4];
         md5_init(st);
-        md5_range_ring<0, VEC, kBatchRingUnits, kBatchRingAhead>(st, nullptr, J.src + (size_t)s * J.slice, J.slice,
-                                                                 0, ~0ull, ring + tid * kBatchRingLane);
-        store_digest(J.checks[s].md5, st);
+        md5_range_ring<0, VEC, true, UNITS, AHEAD>(st, nullptr, J.src + (size_t)s * J.slice, live ? J.slice : 0, 0,
+                                                   live ? ~0ull : 0, ring + (tid & ~31) * ring_lane_bytes(UNITS));
+        if (live) store_digest(J.checks[s].md5, st);
     }
 }
 
@@ -1279,14 +1341,14 @@ __device__ __noinline__ void batch_scan(const BatchJob& J, uint32_t first, uint3
 template <bool VEC>
 __device__ __noinline__ void batch_file_hash(const BatchJob& J, uint32_t first, uint32_t count, uint32_t ring) {
     const int tid = threadIdx.x;
-    if (tid < kHashThreadsWide && (uint32_t)tid < count) {
-        const uint32_t f = first + tid;
+    if (tid < kHashThreads && (uint32_t)(tid & ~31) < count) {
+        const bool live = (uint32_t)tid < count;
+        const uint32_t f = first + (live ? tid : 0);
         uint32_t st[4];
         md5_init(st);
-        md5_range_ring<0, VEC, kBatchRingUnits, kBatchRingAhead>(st, nullptr, J.src + J.files[2 * f],
-                                                                 J.files[2 * f + 1], 0, ~0ull,
-                                                                 ring + tid * kBatchRingLane);
-        store_digest(J.hfull + 16 * (size_t)f, st);
+        md5_range_ring<0, VEC, false>(st, nullptr, J.src + J.files[2 * f], live ? J.files[2 * f + 1] : 0, 0,
+                                      live ? ~0ull : 0, ring + (tid & ~31) * kRingLaneBytes);
+        if (live) store_digest(J.hfull + 16 * (size_t)f, st);
     }
 }
 
@@ -1317,13 +1379,16 @@ __device__ void batch_set_id(const BatchJob& J, uint32_t ring, uint32_t* sid) {
     uint4* ids = reinterpret_cast<uint4*>(J.scratch);
     uint8_t* body = J.scratch + 16 * (size_t)n;
     if (tid < kHashThreadsWide) {
-        for (uint32_t f = tid; f < n; f += kHashThreadsWide) {
-            const uint64_t off = J.files[2 * f], len = J.files[2 * f + 1];
+        for (uint32_t f0 = tid & ~31; f0 < n; f0 += kHashThreadsWide) {  // whole warps
+            const uint32_t f = f0 + (tid & 31);
+            const bool live = f < n;
+            const uint64_t off = live ? J.files[2 * f] : 0, len = live ? J.files[2 * f + 1] : 0;
             uint32_t h[4];
             md5_init(h);
-            md5_range_ring<0, VEC, kBatchRingUnits, kBatchRingAhead>(
-                h, nullptr, J.src + off, len < P2G_HASH16K_LEN ? len : P2G_HASH16K_LEN, 0, ~0ull,
-                ring + tid * kBatchRingLane);
+            md5_range_ring<0, VEC, false, kBatchRingUnits, kBatchRingAhead>(
+                h, nullptr, J.src + off, len < P2G_HASH16K_LEN ? len : P2G_HASH16K_LEN, 0, live ? ~0ull : 0,
+                ring + (tid & ~31) * kBatchRingLane);
+            if (!live) continue;
             store_digest(J.h16k + 16 * (size_t)f, h);
             const uint32_t pre[6] = {h[0], h[1], h[2], h[3], (uint32_t)len, (uint32_t)(len >> 32)};
             uint32_t id[4];
@@ -1377,15 +1442,17 @@ __device__ void batch_set_id(const BatchJob& J, uint32_t ring, uint32_t* sid) {
 __device__ __noinline__ void batch_packets(const BatchJob& J, uint32_t ring, const uint32_t* sid, uint32_t r0, uint32_t r1) {
     const int tid = threadIdx.x;
     if (tid < kHashThreads) {
-        for (uint32_t r = r0 + tid; r < r1; r += kHashThreads) {
+        for (uint32_t w0 = r0 + (tid & ~31); w0 < r1; w0 += kHashThreads) {  // whole warps
+            const bool live = w0 + (tid & 31) < r1;
+            const uint32_t r = live ? w0 + (tid & 31) : w0;
             // set id ‖ "PAR 2.0\0" "RecvSlic" as little-endian words ‖ exponent
             const uint32_t pre[9] = {sid[0], sid[1], sid[2], sid[3], 0x20524150u, 0x00302E32u, 0x76636552u,
                                      0x63696C53u, J.first_exp + r};
             uint32_t st[4];
             md5_init(st);
-            md5_range_ring<9, true, kBatchRingUnits, kBatchRingAhead>(
-                st, pre, J.rec + (size_t)r * J.rec_stride, J.slice, 0, ~0ull, ring + tid * kBatchRingLane);
-            store_digest(J.pkt + 16 * (size_t)r, st);
+            md5_range_ring<9, true, true>(st, pre, J.rec + (size_t)r * J.rec_stride, live ? J.slice : 0, 0,
+                                          live ? ~0ull : 0, ring + (tid & ~31) * kRingLaneBytes);
+            if (live) store_digest(J.pkt + 16 * (size_t)r, st);
         }
     }
     __syncthreads();
@@ -1407,8 +1474,10 @@ __device__ __noinline__ void advance_rows(const BatchJob& J, uint32_t q, uint32_
     const bool final = b_last + 1 == J.n_bands;
     const uint64_t from = b == 0 ? 0 : (36 + done_bytes(b - 1)) / 64;
     const uint64_t to = final ? nblocks : (36 + done_bytes(b_last)) / 64;
-    const uint32_t r = q * kChainRows + tid;
-    if (tid < (int)kChainRows && r < J.R) {
+    const uint32_t w0 = q * kChainRows + (tid & ~31);
+    if (tid < (int)kChainRows && w0 < J.R) {  // whole warps
+        const bool live = w0 + (tid & 31) < J.R;
+        const uint32_t r = live ? w0 + (tid & 31) : w0;
         const uint32_t pre[9] = {sid[0], sid[1], sid[2], sid[3], 0x20524150u, 0x00302E32u, 0x76636552u,
                                  0x63696C53u, J.first_exp + r};
         uint32_t st[4];
@@ -1421,11 +1490,11 @@ __device__ __noinline__ void advance_rows(const BatchJob& J, uint32_t q, uint32_
             st[2] = v.z;
             st[3] = v.w;
         }
-        md5_range_ring<9, true, kBatchRingUnits, kBatchRingAhead>(st, pre, J.rec + (size_t)r * J.rec_stride,
-                                                                  J.slice, from, to, ring + tid * kBatchRingLane);
-        if (final)
+        md5_range_ring<9, true, true>(st, pre, J.rec + (size_t)r * J.rec_stride, live ? J.slice : 0, from,
+                                      live ? to : 0, ring + (tid & ~31) * kRingLaneBytes);
+        if (final && live)
             store_digest(J.pkt + 16 * (size_t)r, st);
-        else
+        else if (live)
             __stcg(reinterpret_cast<uint4*>(J.chain) + r, make_uint4(st[0], st[1], st[2], st[3]));
         __threadfence();  // the next token holder, on another SM, reads this state
     }
@@ -1564,10 +1633,16 @@ __global__ void __launch_bounds__(kEncThreads, 1)
         const BatchJob& J = jobs[it.job];
         const uint32_t kind = it.kind_rg & kItemKindMask;
         if (kind == kItemScan) {
-            if (J.vec)
-                batch_scan<true>(J, it.a, it.b, ring);
-            else
-                batch_scan<false>(J, it.a, it.b, ring);
+            if (it.b > (uint32_t)kHashThreads) {
+                if (J.vec)
+                    batch_scan<true, kHashThreadsWide>(J, it.a, it.b, ring);
+                else
+                    batch_scan<false, kHashThreadsWide>(J, it.a, it.b, ring);
+            } else if (J.vec) {
+                batch_scan<true, kHashThreads>(J, it.a, it.b, ring);
+            } else {
+                batch_scan<false, kHashThreads>(J, it.a, it.b, ring);
+            }
             __syncthreads();
             continue;
         }
@@ -2034,7 +2109,7 @@ cudaError_t launch_md5_files(const uint8_t* base, const FileSpan* spans, uint32_
     const HashGrid g = hash_grid(n);
     cudaError_t e = allow_exclusive(md5_files_kernel<false>);
     if (e != cudaSuccess) return e;
-    // file starts are only known to be 4-byte aligned: 4-byte ring copies
+    // file starts are only known to be 4-byte aligned
     md5_files_kernel<false><<<g.blocks, g.threads, g.smem, st>>>(base, spans, n, out16);
     count_launch();
     return cudaGetLastError();
@@ -2057,7 +2132,7 @@ cudaError_t launch_md5_recovery(const uint8_t* rec, uint64_t stride, uint32_t co
     if (!count) return cudaSuccess;
     const HashGrid g = hash_grid(count);
     cudaError_t e;
-    // 16-byte ring copies only when every row starts 16-byte aligned
+    // rows that all start 16-byte aligned need no shift in the ring
     if ((uintptr_t)rec % 16 == 0 && stride % 16 == 0) {
         if ((e = allow_exclusive(md5_recovery_kernel<true>)) != cudaSuccess) return e;
         md5_recovery_kernel<true><<<g.blocks, g.threads, g.smem, st>>>(rec, stride, count, slice_size,

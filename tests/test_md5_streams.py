@@ -1,0 +1,77 @@
+"""The staged MD5 streams at the edges of their rings: message lengths around
+the 64-byte copy units, every 4-byte start within a 16-byte quad, warps whose
+lanes differ in length, and stream counts around a warp, a CTA and the
+switch to 256 lanes a CTA (more than 148 x 128 streams)."""
+import ctypes as C
+import hashlib
+import zlib
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _device(n, seed):
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return torch.randint(0, 256, (n,), dtype=torch.uint8, device="cuda", generator=g)
+
+
+# slice sizes around the ring's units (64 B), its depth (12 units, 8 ahead) and one block
+SLICES = [(1, 4, 4, 0), (31, 60, 64, 0), (33, 64, 64, 0), (129, 68, 68, 4), (40, 124, 128, 8), (200, 508, 512, 0),
+          (257, 576, 580, 12), (64, 772, 776, 4), (130, 1028, 1040, 0), (128, 4092, 4096, 0), (19000, 132, 132, 0)]
+
+
+@pytest.mark.parametrize("count,size,stride,off", SLICES)
+def test_slice_streams(p2g, gpu, count, size, stride, off):
+    import torch
+
+    src = _device(off + count * stride, count + size)
+    out = torch.zeros(20 * count, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    assert p2g.lib().p2g_slice_checksums(src.data_ptr() + off, stride, count, size, out.data_ptr(),
+                                         p2g.DEVICE_POINTERS, st) == 0
+    host = src.cpu().numpy()[off:]
+    want = b"".join(hashlib.md5(s).digest() + zlib.crc32(s).to_bytes(4, "little")
+                    for s in (host[i * stride:i * stride + size].tobytes() for i in range(count)))
+    assert out.cpu().numpy().tobytes() == want
+
+
+@pytest.mark.parametrize("count,size,stride,off", SLICES)
+def test_packet_streams(p2g, gpu, count, size, stride, off):
+    """The same rows behind the packet's 36-byte prefix (set id, type, exponent)."""
+    import torch
+
+    src = _device(off + count * stride, count + 3 * size)
+    out = torch.zeros(16 * count, dtype=torch.uint8, device="cuda")
+    sid = bytes(range(16))
+    st = torch.cuda.current_stream().cuda_stream
+    assert p2g.lib().p2g_recovery_packet_md5(sid, src.data_ptr() + off, stride, count, size, 7, out.data_ptr(),
+                                             p2g.DEVICE_POINTERS, st) == 0
+    host = src.cpu().numpy()[off:]
+    want = b"".join(hashlib.md5(sid + b"PAR 2.0\0RecvSlic" + (7 + i).to_bytes(4, "little") +
+                                host[i * stride:i * stride + size].tobytes()).digest() for i in range(count))
+    assert out.cpu().numpy().tobytes() == want
+
+
+def test_file_streams_of_mixed_lengths(p2g, gpu):
+    """Lanes of one warp with different lengths and starts 4 bytes apart."""
+    import torch
+
+    lengths = [1, 3, 55, 56, 63, 64, 65, 119, 128, 191, 1000, 4095, 16383, 16384, 16385, 40001] * 9
+    pitch = 40960 + 4
+    src = _device(len(lengths) * pitch + 16, 5)
+    n = len(lengths)
+    ptrs = (C.c_void_p * n)(*[src.data_ptr() + i * pitch for i in range(n)])
+    lens = (C.c_uint64 * n)(*lengths)
+    out = torch.zeros(32 * n, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    assert p2g.lib().p2g_file_hashes(ptrs, lens, n, out.data_ptr(), out.data_ptr() + 16 * n, p2g.DEVICE_POINTERS,
+                                     st) == 0
+    host = src.cpu().numpy()
+    data = [host[i * pitch:i * pitch + k].tobytes() for i, k in enumerate(lengths)]
+    got = out.cpu().numpy().tobytes()
+    assert got[:16 * n] == b"".join(hashlib.md5(d).digest() for d in data)
+    assert got[16 * n:] == b"".join(hashlib.md5(d[:16384]).digest() for d in data)
