@@ -35,7 +35,7 @@ namespace {
 // costs 0.62 us per slice plus 0.433 ns per symbol and slice (1.49 ms for
 // 1027 slices x 1920 symbols, 0.187 ms for 256 x 256), a folded tail item
 // 15 % more, an accumulating item 4 % more; a scan chain steps 64 bytes in
-// 0.44 us, a packet chain in 0.47 us; CRC32 streams at ~10 GB/s per CTA.
+// 0.44 us, a packet chain in 0.47 us; CRC32 streams at ~35 GB/s per CTA.
 constexpr double kEncRate = 2.309e6;    // symbols per ms per CTA, per slice
 constexpr double kBuildCost = 1430.0;   // per-slice fixed cost (table build, barrier, copy wait) in symbols
 constexpr double kChainMs = 4.4e-4;         // one MD5 chain step of 64 bytes, at most 128 lanes on the SM
@@ -405,8 +405,8 @@ double est_encode_item_ms(uint32_t slices, uint32_t syms) {
 double est_scan_item_ms(uint64_t slice, uint32_t count) {
     return md5_ms(slice) * (count > kLoneScanSlices ? kWideChain : 1.0) + kItemMs;
 }
-// CRC32 streams from DRAM at ~10 GB/s per SM (16 warps)
-double est_crc_item_ms(uint64_t slice, uint32_t count) { return (double)slice * count / 1e7 + kItemMs; }
+// CRC32 streams from DRAM at ~35 GB/s per SM (16 warps)
+double est_crc_item_ms(uint64_t slice, uint32_t count) { return (double)slice * count / 3.5e7 + kItemMs; }
 double est_set_id_ms(uint32_t files) {
     const double hashes = ceil(files / 256.0) * (md5_ms(P2G_HASH16K_LEN) * kWideChain + md5_ms(24 + 256));
     const double sort = (double)files * files / 512.0 * 4e-6;

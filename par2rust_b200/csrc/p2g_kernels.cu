@@ -1002,17 +1002,27 @@ __global__ void __launch_bounds__(kHashThreadsWide) md5_recovery_range_kernel(co
 
 // ---------------------------------------------------------------------------
 // CRC-32/IEEE (reflected polynomial 0xEDB88320, init and final xor
-// 0xFFFFFFFF), one warp per slice.  Lane l runs the table-driven register
-// update (four 256-entry tables, four bytes per step) over its contiguous
-// chunk from register value 0 (lane 0 from 0xFFFFFFFF); the chunk results
-// are then moved to the end of the slice by multiplying with x^(8*bytes
-// after the chunk) mod P and XORed together.  In the reflected register
-// bit 31 is the x^0 coefficient, so "times x" is a right shift that folds
-// the polynomial back in when bit 0 falls off.
+// 0xFFFFFFFF) of slices, by folding.  A warp reads a slice as rows of 32
+// words, word l of a row in lane l; with y = x^1024 (one row) the message is
+// sum_i row_i y^(n-1-i).  P has coefficients in GF(2), so P(x^1024) =
+// P(x)^1024 = 0 mod P: rows can be reduced modulo P(y) itself, all 32 bit
+// columns of a lane's words at once.  The state is 32 words a lane (the
+// coefficients of y^0..y^31), and eight rows cost 54 XORs: y^32..y^39 mod P(y)
+// say which of the top eight coefficients each new one takes, looked up among
+// the 16 sums of either half.  No table lookup and no dependent chain per
+// word (a lookup per byte chained through the register ran at ~10 GB/s an
+// SM: one issue per ~10 cycles a warp): 54 LOP3 a 1,024 bytes a warp is 75
+// GB/s an SM, above its 44 GB/s share of the memory.  At the end the 32
+// coefficients are summed with Horner's rule in y (four byte tables of "times
+// x^1024") and moved to the end of the slice by one multiplication.  In the
+// reflected register bit 31 is the x^0 coefficient, so "times x" is a right
+// shift that folds the polynomial back in when bit 0 falls off.
+// Measured, 4 MB items of the 538 MB job inside the persistent kernel: 404 us
+// an item (10 GB/s a CTA) -> 119 us (35 GB/s).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kCrcPoly = 0xEDB88320u;
 
-__device__ __forceinline__ uint32_t gf2_mulmod(uint32_t a, uint32_t b) {
+__host__ __device__ constexpr uint32_t gf2_mulmod(uint32_t a, uint32_t b) {
     uint32_t prod = 0;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -1022,7 +1032,7 @@ __device__ __forceinline__ uint32_t gf2_mulmod(uint32_t a, uint32_t b) {
     return prod;
 }
 
-__device__ uint32_t x_pow_8n(uint64_t n) {
+__host__ __device__ constexpr uint32_t x_pow_8n(uint64_t n) {
     uint32_t result = 0x80000000u;  // x^0
     uint32_t base = 0x00800000u;    // x^8
     while (n) {
@@ -1033,86 +1043,175 @@ __device__ uint32_t x_pow_8n(uint64_t n) {
     return result;
 }
 
-// Slicing-by-4 tables T[t][b] (T[0] the byte table) into shared memory,
-// built by all threads of the block (contains __syncthreads).
-__device__ __forceinline__ void crc_tables_build(uint32_t (*T)[256]) {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        uint32_t c = (uint32_t)i;
-        for (int b = 0; b < 8; ++b) c = (c >> 1) ^ ((c & 1u) ? kCrcPoly : 0u);
-        T[0][i] = c;
-    }
+// mul[t][v]: byte t of the register, value v, times x^1024; lane[l]:
+// x^(32 (32 - l)), from word l of the last row to the end of the message.
+struct CrcTables {
+    uint32_t mul[4][256];
+    uint32_t lane[32];
+};
+constexpr CrcTables make_crc_tables() {
+    CrcTables t{};
+    uint32_t bit[32] = {};  // register bit b times x^1024
+    for (int b = 0; b < 32; ++b) bit[b] = gf2_mulmod(1u << b, x_pow_8n(128));
+    for (int k = 0; k < 4; ++k)
+        for (int v = 0; v < 256; ++v)
+            for (int b = 0; b < 8; ++b)
+                if (v >> b & 1) t.mul[k][v] ^= bit[8 * k + b];
+    for (int l = 0; l < 32; ++l) t.lane[l] = x_pow_8n(4 * (32 - l));
+    return t;
+}
+__device__ const CrcTables d_crc = make_crc_tables();
+
+// The x^1024 tables into shared memory (all threads; ends with __syncthreads).
+__device__ __forceinline__ void crc_tables_load(uint32_t (*T)[256]) {
+    for (int i = threadIdx.x; i < 1024; i += blockDim.x) (&T[0][0])[i] = (&d_crc.mul[0][0])[i];
     __syncthreads();
-    for (int t = 1; t < 4; ++t) {
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-            const uint32_t v = T[t - 1][i];
-            T[t][i] = (v >> 8) ^ T[0][v & 0xFF];
-        }
-        __syncthreads();
-    }
 }
 
-// Lane chunk of a slice of W = slice_size/4 words: [start, end) words, and
-// K = x^(8 * bytes after the chunk) mod P that moves its partial CRC to the
-// end of the slice.
-struct CrcLane {
-    uint64_t start, end;
-    uint32_t K;
-};
-template <bool VEC>
-__device__ __forceinline__ CrcLane crc_lane(uint64_t slice_size, int lane) {
-    const uint64_t W = slice_size / 4;
-    uint64_t cw = (W + 31) / 32;
-    if (VEC) cw = (cw + 3) & ~3ull;
-    CrcLane c;
-    c.start = min((uint64_t)lane * cw, W);
-    c.end = min(c.start + cw, W);
-    c.K = x_pow_8n(slice_size - c.end * 4);
+// y^(32+m) mod P(y), bit k = the coefficient of y^k (unreflected).
+__host__ __device__ constexpr uint32_t crc_fold_taps(int m) {
+    uint32_t q = 0x04C11DB7u;
+    for (int i = 0; i < m; ++i) q = (q << 1) ^ ((q >> 31) ? 0x04C11DB7u : 0u);
+    return q;
+}
+// state * y^8 + the eight rows w[0] y^7 + .. + w[7], mod P(y)
+__device__ __forceinline__ void crc_fold8(uint32_t (&s)[32], const uint32_t (&w)[8]) {
+    uint32_t A[16], B[16];
+    A[0] = B[0] = 0;
+#pragma unroll
+    for (int v = 1; v < 16; ++v) {
+        const int hi = v & 8 ? 3 : v & 4 ? 2 : v & 2 ? 1 : 0;
+        A[v] = A[v ^ (1 << hi)] ^ s[24 + hi];
+        B[v] = B[v ^ (1 << hi)] ^ s[28 + hi];
+    }
+    uint32_t n[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+        int a = 0, b = 0;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            a |= (int)(crc_fold_taps(m) >> k & 1u) << m;
+            b |= (int)(crc_fold_taps(4 + m) >> k & 1u) << m;
+        }
+        n[k] = (k >= 8 ? s[k >= 8 ? k - 8 : 0] : w[k < 8 ? 7 - k : 0]) ^ A[a] ^ B[b];
+    }
+#pragma unroll
+    for (int k = 0; k < 32; ++k) s[k] = n[k];
+}
+
+// A slice of W words cut into `parts` runs of crc_part_words(W, parts) words
+// (whole 1,024-byte groups), one warp each; parts of at least 16 KiB, so that
+// rounding to groups leaves none of up to 16 empty.
+__host__ __device__ inline uint64_t crc_part_words(uint64_t W, uint32_t parts) {
+    return parts == 1 ? W : ((W + parts - 1) / parts + 255) / 256 * 256;
+}
+__host__ __device__ inline uint32_t crc_parts(uint64_t W, uint32_t most) {
+    uint32_t p = 1;
+    while (2 * p <= most && W / (2 * p) >= 4096) p *= 2;
+    return p;
+}
+
+// One part of the CRC of a slice by one warp: words [at, at + n) of the W at
+// p, moved to the slice's end.  The parts' results XOR to the register before
+// the final inversion.  Zeros in front of a message do not change its
+// remainder, so the first group is filled up with them; the initial register
+// is the inverse of the slice's first word.
+__device__ __noinline__ uint32_t crc_part_warp(const uint32_t* __restrict__ p, uint64_t at, uint64_t n, uint64_t W,
+                                               const uint32_t (*T)[256]) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t groups = (uint32_t)((n + 255) / 256), pad = groups * 256u - (uint32_t)n;
+    const uint32_t* q = p + at + lane;
+    auto load = [&](uint32_t (&w)[8], uint32_t g) {
+        if (g < groups) {
+            const uint32_t* r = q + ((size_t)g * 256 - pad);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = __ldg(r + 32 * i);
+        }
+    };
+    uint32_t s[32], a[8], b[8];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) s[k] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t v = 32 * i + lane;
+        a[i] = v < pad ? 0u : __ldg(p + at + (v - pad));
+        if (v == pad && at == 0) a[i] = ~a[i];
+        b[i] = 0;
+    }
+    load(b, 1);
+    for (uint32_t g = 0; g < groups; g += 2) {
+        crc_fold8(s, a);
+        load(a, g + 2);
+        if (g + 1 < groups) {
+            crc_fold8(s, b);
+            load(b, g + 3);
+        }
+    }
+    uint32_t c = 0;
+    auto horner = [&](int k) {
+        c = T[0][c & 0xFF] ^ T[1][(c >> 8) & 0xFF] ^ T[2][(c >> 16) & 0xFF] ^ T[3][c >> 24] ^ s[k];
+    };
+    if (groups > 3)
+#pragma unroll
+        for (int k = 31; k >= 24; --k) horner(k);
+    if (groups > 2)
+#pragma unroll
+        for (int k = 23; k >= 16; --k) horner(k);
+    if (groups > 1)
+#pragma unroll
+        for (int k = 15; k >= 8; --k) horner(k);
+#pragma unroll
+    for (int k = 7; k >= 0; --k) horner(k);
+    uint32_t K = d_crc.lane[lane];
+    if (at + n < W) K = gf2_mulmod(K, x_pow_8n(4 * (W - at - n)));
+    c = gf2_mulmod(c, K);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c ^= __shfl_xor_sync(0xFFFFFFFFu, c, o);
     return c;
 }
 
-// CRC32 of one slice by one warp (all 32 lanes call it with the same p).
-template <bool VEC>
-__device__ __forceinline__ uint32_t crc_slice_warp(const uint32_t* __restrict__ p, const CrcLane& cl, int lane,
-                                                   const uint32_t (*T)[256]) {
-    uint32_t c = lane == 0 ? 0xFFFFFFFFu : 0u;
-    uint64_t w = cl.start;
-    if (VEC && w + 4 <= cl.end) {
-        // the next 16 bytes are loaded before the current 16 are folded in,
-        // so a lane has two loads in flight instead of one
-        uint4 nxt = __ldg(reinterpret_cast<const uint4*>(p + w));
-        for (; w + 4 <= cl.end; w += 4) {
-            const uint4 v = nxt;
-            if (w + 8 <= cl.end) nxt = __ldg(reinterpret_cast<const uint4*>(p + w + 4));
-            const uint32_t vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                c ^= vv[q];
-                c = T[3][c & 0xFF] ^ T[2][(c >> 8) & 0xFF] ^ T[1][(c >> 16) & 0xFF] ^ T[0][c >> 24];
-            }
+// CRC32 of `count` slices `stride` bytes apart by the `warps` warps of a CTA
+// (all threads): a slice a warp, or, where there are fewer slices than warps,
+// several warps to a slice, summed in part[].
+__device__ __forceinline__ void crc_slices_cta(const uint8_t* __restrict__ src, uint64_t stride, uint32_t count,
+                                               uint64_t slice_size, p2g_slice_checksum* __restrict__ out, uint32_t warps,
+                                               const uint32_t (*T)[256], uint32_t* part) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t W = slice_size / 4;
+    const uint32_t P = count < warps ? crc_parts(W, warps / count) : 1u;
+    const uint64_t pw = crc_part_words(W, P);
+    for (uint32_t u = warp; u < count * P; u += warps) {
+        const uint32_t i = u / P;
+        const uint64_t at = (uint64_t)(u % P) * pw;
+        const uint32_t c = crc_part_warp(reinterpret_cast<const uint32_t*>(src + (size_t)i * stride), at,
+                                         at + pw < W ? pw : W - at, W, T);
+        if (lane == 0) {
+            if (P == 1)
+                out[i].crc32 = ~c;
+            else
+                part[u] = c;  // count * P <= warps: one round
         }
     }
-    for (; w < cl.end; ++w) {
-        c ^= __ldg(p + w);
-        c = T[3][c & 0xFF] ^ T[2][(c >> 8) & 0xFF] ^ T[1][(c >> 16) & 0xFF] ^ T[0][c >> 24];
+    if (P == 1) return;
+    __syncthreads();
+    if (threadIdx.x < count) {
+        uint32_t c = 0;
+        for (uint32_t k = 0; k < P; ++k) c ^= part[threadIdx.x * P + k];
+        out[threadIdx.x].crc32 = ~c;
     }
-    c = gf2_mulmod(c, cl.K);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c ^= __shfl_xor_sync(0xFFFFFFFFu, c, o);
-    return c ^ 0xFFFFFFFFu;
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(64) crc_slices_kernel(const uint8_t* __restrict__ src, uint64_t stride,
-                                                         uint32_t count, uint64_t slice_size,
+// Standalone: `per_cta` slices a CTA.
+__global__ void __launch_bounds__(512) crc_slices_kernel(const uint8_t* __restrict__ src, uint64_t stride,
+                                                         uint32_t count, uint64_t slice_size, uint32_t per_cta,
                                                          p2g_slice_checksum* __restrict__ out) {
     __shared__ uint32_t T[4][256];
-    crc_tables_build(T);
-    const int lane = threadIdx.x & 31;
-    const uint32_t wpb = blockDim.x >> 5;
-    const CrcLane cl = crc_lane<VEC>(slice_size, lane);
-    for (uint64_t s = (uint64_t)blockIdx.x * wpb + (threadIdx.x >> 5); s < count; s += (uint64_t)gridDim.x * wpb) {
-        const uint32_t c = crc_slice_warp<VEC>(reinterpret_cast<const uint32_t*>(src + (size_t)s * stride), cl, lane, T);
-        if (lane == 0) out[s].crc32 = c;
+    __shared__ uint32_t part[16];
+    crc_tables_load(T);
+    for (uint64_t s = (uint64_t)blockIdx.x * per_cta; s < count; s += (uint64_t)gridDim.x * per_cta) {
+        crc_slices_cta(src + s * stride, stride, (uint32_t)min((uint64_t)per_cta, count - s), slice_size, out + s,
+                       blockDim.x >> 5, T, part);
+        __syncthreads();  // part[] is free again
     }
 }
 
@@ -1352,19 +1451,12 @@ __device__ __noinline__ void batch_file_hash(const BatchJob& J, uint32_t first, 
     }
 }
 
-// Slice CRC32 of slices [first, first+count): one slice per warp at a time
-// over all 16 warps (CRC streams from DRAM; its items are a few MB each so
-// the work spreads over many SMs).
-template <bool VEC>
-__device__ __forceinline__ void batch_crc(const BatchJob& J, uint32_t first, uint32_t count,
-                                          const uint32_t (*T)[256]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const CrcLane cl = crc_lane<VEC>(J.slice, lane);
-    for (uint32_t i = (uint32_t)warp; i < count; i += kEncThreads / 32) {
-        const uint32_t s = first + i;
-        const uint32_t c = crc_slice_warp<VEC>(reinterpret_cast<const uint32_t*>(J.src + (size_t)s * J.slice), cl, lane, T);
-        if (lane == 0) J.checks[s].crc32 = c;
-    }
+// Slice CRC32 of slices [first, first+count) over all 16 warps (its items are
+// a few MB each so the work spreads over many SMs); `part`: 16 words.
+__device__ __noinline__ void batch_crc(const BatchJob& J, uint32_t first, uint32_t count, const uint32_t (*T)[256],
+                                       uint32_t* part) {
+    crc_slices_cta(J.src + (size_t)first * J.slice, J.slice, count, J.slice, J.checks + first, kEncThreads / 32, T,
+                   part);
 }
 
 // Set-id step of job J (all threads of the CTA): hash16k of each file and
@@ -1605,7 +1697,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
     }
     if (MMA && (tid >> 5) == 1) mma::tmem_alloc(smem_u32(mma_misc));
     if (MMA) mma::tc_fence_before();
-    crc_tables_build(T);  // ends with __syncthreads
+    crc_tables_load(T);  // ends with __syncthreads
     if (MMA) {
         mma::tc_fence_after();
         if ((tid >> 5) >= 4 && (tid >> 5) < 8) mma::sf_fill(mma_misc[0], (uint32_t)(tid >> 5) & 3u);
@@ -1655,10 +1747,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             continue;
         }
         if (kind == kItemCrc) {
-            if (J.vec)
-                batch_crc<true>(J, it.a, it.b, T);
-            else
-                batch_crc<false>(J, it.a, it.b, T);
+            batch_crc(J, it.a, it.b, T, reinterpret_cast<uint32_t*>(ring_p));  // the rings are idle here
             __syncthreads();
             continue;
         }
@@ -2091,14 +2180,13 @@ cudaError_t launch_md5_slices(const uint8_t* src, uint64_t stride, uint32_t coun
 cudaError_t launch_crc_slices(const uint8_t* src, uint64_t stride, uint32_t count, uint64_t slice_size,
                               p2g_slice_checksum* out, cudaStream_t st) {
     if (!count) return cudaSuccess;
-    const unsigned tpb = 64, wpb = tpb / 32;
-    const uint64_t want = (count + wpb - 1) / wpb;
+    // one slice to a warp, four warps to a CTA, while that fills every SM with
+    // 16 warps; else a slice to a CTA of as many warps as have 16 KiB each
+    const bool many = count >= (uint32_t)sm_count() * 16;
+    const unsigned warps = many ? 4 : crc_parts(slice_size / 4, 16), per_cta = many ? 4 : 1;
+    const uint64_t want = (count + per_cta - 1) / per_cta;
     const unsigned blocks = (unsigned)(want < (uint64_t)sm_count() * 8 ? want : (uint64_t)sm_count() * 8);
-    const bool vec = ((uintptr_t)src % 16 == 0) && (stride % 16 == 0) && (slice_size % 16 == 0);
-    if (vec)
-        crc_slices_kernel<true><<<blocks, tpb, 0, st>>>(src, stride, count, slice_size, out);
-    else
-        crc_slices_kernel<false><<<blocks, tpb, 0, st>>>(src, stride, count, slice_size, out);
+    crc_slices_kernel<<<blocks, 32 * warps, 0, st>>>(src, stride, count, slice_size, per_cta, out);
     count_launch();
     return cudaGetLastError();
 }

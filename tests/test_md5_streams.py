@@ -1,5 +1,5 @@
-"""The staged MD5 streams at the edges of their rings: message lengths around
-the 64-byte copy units, every 4-byte start within a 16-byte quad, warps whose
+"""The staged MD5 streams and the folded CRC32 at their edges: message lengths
+around the 64-byte copy units, the 1,024-byte fold groups and the 16 KiB parts, every 4-byte start within a 16-byte quad, warps whose
 lanes differ in length, and stream counts around a warp, a CTA and the
 switch to 256 lanes a CTA (more than 148 x 128 streams)."""
 import ctypes as C
@@ -75,3 +75,32 @@ def test_file_streams_of_mixed_lengths(p2g, gpu):
     got = out.cpu().numpy().tobytes()
     assert got[:16 * n] == b"".join(hashlib.md5(d).digest() for d in data)
     assert got[16 * n:] == b"".join(hashlib.md5(d[:16384]).digest() for d in data)
+
+
+# around 1, 2, 3, 4 and more fold groups of 1,024 B; around 2, 4, 8 and 16 parts of a slice (16 KiB each at least)
+CRC_SIZES = [(3, 1020), (3, 1024), (3, 1028), (2, 2048), (2, 2052), (5, 3076), (4, 4092), (4, 4100), (1, 32764),
+             (17, 32768), (2, 32772), (3, 65540), (1, 131076), (9, 262144), (2, 262148), (1, 1048580), (2400, 1032)]
+
+
+@pytest.mark.parametrize("count,size", CRC_SIZES)
+def test_slice_crc(p2g, gpu, count, size):
+    src = _device(count * size, size).cpu().numpy()
+    got = p2g.slice_checksums(src, size)
+    for i in range(count):
+        s = src[i * size:(i + 1) * size].tobytes()
+        assert got[i].crc32 == zlib.crc32(s) and got[i].md5 == hashlib.md5(s).digest(), i
+
+
+def test_slice_crc_in_device_job(p2g, gpu):
+    """CRC items of one slice to a warp and of several warps to a slice."""
+    import torch
+
+    for size, slices in ((1 << 20, 5), (16388, 300), (65536, 70)):
+        src = _device(slices * size + 16, size)
+        bufs = p2g.run_device_job(src, [slices * size - 5], [b"f"], size, 1, skip_hash_full=True)
+        torch.cuda.synchronize()
+        host = src.cpu().numpy()
+        got = bufs.checksums.cpu().numpy().reshape(slices, 20)
+        for i in range(slices):
+            s = host[i * size:(i + 1) * size].tobytes()
+            assert got[i].tobytes() == hashlib.md5(s).digest() + zlib.crc32(s).to_bytes(4, "little"), (size, i)
