@@ -426,8 +426,9 @@ p2g_status p2g_batch_plan(const p2g_batch_shape *shapes, uint32_t n, uint32_t ct
  * turns the tail split off here as it does for the job, and the encode
  * kernel is chosen as for the job (P2G_ENCODE_VARIANT, else by shape).  Lookup
  * kernel items cover 32-row groups (fold 1, 2 or 4 for a short last group);
- * tensor-core items have fold 0 and cover 16-row tiles of at most 240
- * symbols.  It returns up to `cap` encode items as (row group, fold,
+ * tensor-core plans are reported in the planner's units of 16 rows by at
+ * most 240 symbols, with fold 0 (the kernel's tiles, of up to 13 rows by 256
+ * symbols, cover the units of one band and slice range).  It returns up to `cap` encode items as (row group, fold,
  * first symbol, symbols, band, first slice, slice count, accumulate), the
  * number of encode items, and the first symbol of the columns that are
  * zeroed for accumulating items (the padded row width when there are none).

@@ -70,15 +70,17 @@ struct PlanJob {
     // into split_chunks slice ranges that XOR-accumulate into the rows.
     // split_chunks 0: the caller does not zero, never split.
     uint32_t split_bands = 0, split_chunks = 0;
-    // Encode on the tensor cores: 16-row x 240-symbol items (kItemEncodeMma);
-    // RG then counts 16-row tiles and ts is fixed at 240.
+    // Encode on the tensor cores (kItemEncodeMma).  Bands and slice ranges are
+    // cut in units of 240 symbols (ts) x 16 rows (RG counts them), which
+    // p2g_plan_device_job reports; the items are the kernel's tiles of
+    // mma_rows(R) rows x 256 symbols of a band.
     bool mma = false;
     uint32_t scan_slices = kScanSlices;  // slices per scan item
 };
 
 double finish_ms(const PlanJob& j) { return est_set_id_ms(j.n) + est_packet_item_ms(j.slice, j.R); }
 inline double encode_ms(const PlanJob& j, uint32_t syms) {
-    return j.mma ? est_mma_item_ms(j.S) : est_encode_item_ms(j.S, syms);
+    return j.mma ? est_mma_item_ms(j.S, mma_rows(j.R)) : est_encode_item_ms(j.S, syms);
 }
 inline double scan_ms(const PlanJob& j, uint32_t count) { return est_scan_item_ms(j.slice, count); }
 
@@ -99,10 +101,18 @@ struct Plan {
 
 constexpr uint32_t kMaxBands = 64;  // packet-MD5 chain segments per job (64: 10.27 ms vs 10.59 at 16 for 538 MB / R 200)
 
+constexpr uint32_t kMaxMmaBands = 72;
+
 // Bands of job j: runs of band_tiles consecutive tiles, a multiple of the
-// tail fold so that no folded item straddles two bands.
+// tail fold so that no folded item straddles two bands.  Tensor-core bands are
+// whole runs of 16 units = 15 kernel tiles of 256 symbols.
 void job_bands(const PlanJob& j, uint32_t* band_tiles, uint32_t* n_bands) {
-    const uint32_t F = j.mma ? 1u : tail_fold(j.R);
+    if (j.mma) {
+        *band_tiles = 16 * std::max<uint32_t>(1, (j.tiles + 16 * kMaxMmaBands - 1) / (16 * kMaxMmaBands));
+        *n_bands = (j.tiles + *band_tiles - 1) / *band_tiles;
+        return;
+    }
+    const uint32_t F = tail_fold(j.R);
     uint32_t bt = std::max<uint32_t>(1, (j.tiles + kMaxBands - 1) / kMaxBands);
     bt = (bt + F - 1) / F * F;
     *band_tiles = bt;
@@ -111,6 +121,12 @@ void job_bands(const PlanJob& j, uint32_t* band_tiles, uint32_t* n_bands) {
 // one chain segment of every kChainRows-row block over one band's bytes
 inline double chain_ms(const PlanJob& j, uint32_t band_syms) {
     return ceil(j.R / (double)kChainRows) * md5_ms(2ull * band_syms) * 1.07 + kItemMs;
+}
+
+// Slices of one of C ranges of a job; tensor-core ranges start on whole
+// 16-slice stages of the coefficient image.
+inline uint32_t slice_range(const PlanJob& j, uint32_t C) {
+    return j.mma ? ((j.S + C - 1) / C + 15) / 16 * 16 : (j.S + C - 1) / C;
 }
 
 // Items of all jobs in queue order: every job's set-id item (its chains wait
@@ -162,8 +178,7 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
         for (uint32_t b = 0; b < nb; ++b) {
             const uint32_t t0 = b * bt, t1 = std::min(j.tiles, t0 + bt);
             const uint32_t C = b >= first_split ? j.split_chunks : 1;
-            // tensor-core ranges start on whole 16-slice stages of the A image
-            const uint32_t cs = j.mma ? ((j.S + C - 1) / C + 15) / 16 * 16 : (j.S + C - 1) / C;
+            const uint32_t cs = slice_range(j, C);
             auto push = [&](uint32_t rg, uint32_t fold, uint32_t n0, uint32_t syms) {
                 for (uint32_t s0 = 0; s0 < j.S; s0 += cs) {
                     const uint32_t sn = C > 1 ? std::min(cs, j.S - s0) : 0;
@@ -172,17 +187,19 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
                     counts[b]++;
                 }
             };
-            if (j.mma) {  // tile-major: the row tiles of one symbol tile share its source reads in L2
-                for (uint32_t t = t0; t < t1; ++t) {
-                    const uint32_t n0 = t * j.ts, syms = std::min(j.ts, j.Np - n0);
-                    for (uint32_t rt = 0; rt < j.RG; ++rt)
-                        for (uint32_t s0 = 0; s0 < j.S; s0 += cs) {
-                            const uint32_t sn = C > 1 ? std::min(cs, j.S - s0) : 0;
-                            e.items.push_back({ji, encode_mma_kind(rt, C > 1), n0, (b << 16) | syms, s0, sn});
-                            e.key += est_mma_item_ms(sn ? sn : j.S);
-                            counts[b]++;
-                        }
-                }
+            if (j.mma) {  // row tiles kMmaRowBlock at a time, symbol tile by symbol tile (kMmaRowBlock)
+                const uint32_t end = std::min(t1 * j.ts, j.Np), RT = mma_row_tiles(j.R);
+                const double ms = est_mma_item_ms(C > 1 ? cs : j.S, mma_rows(j.R));
+                for (uint32_t r0 = 0; r0 < RT; r0 += kMmaRowBlock)
+                    for (uint32_t n0 = t0 * j.ts; n0 < end; n0 += kMmaTileSymbols)
+                        for (uint32_t rt = r0; rt < std::min(RT, r0 + kMmaRowBlock); ++rt)
+                            for (uint32_t s0 = 0; s0 < j.S; s0 += cs) {
+                                const uint32_t sn = C > 1 ? std::min(cs, j.S - s0) : 0;
+                                e.items.push_back({ji, encode_mma_kind(rt, C > 1), n0,
+                                                   (b << 16) | std::min(kMmaTileSymbols, end - n0), s0, sn});
+                                e.key += ms;
+                                counts[b]++;
+                            }
                 continue;
             }
             for (uint32_t t = t0; t < t1; ++t) {
@@ -221,7 +238,7 @@ double item_ms(const PlanJob& j, const BatchItem& it) {
     case kItemCrc: return est_crc_item_ms(j.slice, it.b);
     case kItemFileHash: return md5_ms(j.file_bytes) + kItemMs;
     case kItemEncodeMma:
-        return est_mma_item_ms(it.sn ? it.sn : j.S) * ((it.kind_rg & kItemAccumulate) ? kAccCost : 1.0);
+        return est_mma_item_ms(it.sn ? it.sn : j.S, mma_rows(j.R)) * ((it.kind_rg & kItemAccumulate) ? kAccCost : 1.0);
     case kItemEncode: {
         double ms = est_encode_item_ms(it.sn ? it.sn : j.S, std::min(j.ts, it.b & 0xFFFFu));
         if ((it.kind_rg >> 24) & 3u) ms *= kFoldCost;
@@ -313,9 +330,9 @@ Plan plan_tiles(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
 
         j.Np = (uint32_t)(round_up(j.slice, 16) / 2);
         j.finish = finish_ms(j);
-        if (j.mma) {  // fixed tile: one MMA N wide, 16 rows (two M = 128 halves) high
-            j.RG = (j.R + kMmaTileRows - 1) / kMmaTileRows;
-            j.ts = kMmaTileSymbols;
+        if (j.mma) {
+            j.RG = (j.R + kMmaUnitRows - 1) / kMmaUnitRows;
+            j.ts = kMmaUnitSymbols;
             j.tiles = (j.Np + j.ts - 1) / j.ts;
             continue;
         }
@@ -375,23 +392,22 @@ Plan plan_tiles(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
 }  // namespace
 
 double est_md5_ms(uint64_t bytes) { return md5_ms(bytes); }
-// A tensor-core item: one K-step (4 slices) of operand building and two
-// MMAs, plus the pipeline fill and the epilogue.
-// Per 4-slice K-step and per tile on one SM, from the standalone kernel on
-// 14,209 tiles of 16 rows x 240 symbols (96 per SM): 1.93 ms at 256 slices,
-// 5.38 ms at 1,024.
-constexpr double kMmaStepMs = 1.87e-4, kMmaFixedMs = 0.005;
-double est_mma_item_ms(uint32_t slices) { return (slices + 3) / 4 * kMmaStepMs + kMmaFixedMs + kItemMs; }
+// A tensor-core item: its K-steps (4 slices) of two MMAs, N / 2 cycles each
+// but at least 71 (A from TMEM), plus the pipeline fill and the epilogue.
+constexpr double kMmaCyclesPerMs = 1.9e6, kMmaFixedMs = 0.0015;
+double est_mma_item_ms(uint32_t slices, uint32_t rows) {
+    return (slices + 3) / 4 * std::max(143.0, 16.5 * rows) / kMmaCyclesPerMs + kMmaFixedMs + kItemMs;
+}
 // Whether a job's encode runs on the tensor cores: by the cost of its items
 // on a full GPU (the lookup kernel folds a short last row group; the tensor
-// tiles are 16 rows high and 240 symbols wide).
+// tiles are at most 13 rows high and 256 symbols wide).
 // CTA-milliseconds of a job's encode items on either kernel.
 double encode_cost_ms(uint64_t slice, uint32_t S, uint32_t R, bool mma) {
     if (!R || !S) return 0;
     const uint32_t Np = (uint32_t)(round_up(slice, 16) / 2);
     if (mma)
-        return (double)((Np + kMmaTileSymbols - 1) / kMmaTileSymbols) * ((R + kMmaTileRows - 1) / kMmaTileRows) *
-               est_mma_item_ms(S);
+        return (double)((Np + kMmaTileSymbols - 1) / kMmaTileSymbols) * mma_row_tiles(R) *
+               est_mma_item_ms(S, mma_rows(R));
     const uint32_t RG = (R + kRowsPerGroup - 1) / kRowsPerGroup, F = tail_fold(R);
     return (double)((Np + kEncTileSymbols - 1) / kEncTileSymbols) * (RG - 1 + (F > 1 ? kFoldCost / F : 1.0)) *
            est_encode_item_ms(S, std::min<uint32_t>(Np, kEncTileSymbols));
@@ -479,7 +495,9 @@ SingleJobPlan plan_single_job_uncached(uint64_t slice, uint32_t S, uint32_t R, u
     if (jobs[0].split_chunks > 1 && jobs[0].split_bands) {
         const uint32_t nb = (uint32_t)p.band_items[0].size();
         out.zero_from_sym = (nb - std::min(nb, jobs[0].split_bands)) * p.band_syms[0];
+        out.split_slices = slice_range(jobs[0], jobs[0].split_chunks);
     }
+    out.mma = jobs[0].mma;
     out.items = std::move(p.items);
     out.band_items = p.band_items[0];
     out.band_syms = p.band_syms[0];
@@ -508,7 +526,7 @@ struct p2g_batch {
     uint64_t err_word = 0;      // index of the error word in d_ctl
     size_t ctl_bytes = 0;
     uint64_t max_basis_words = 0;
-    uint64_t max_aimg_bytes = 0;  // tensor-core jobs: largest A image to fill per run
+    uint64_t max_aimg_bytes = 0;  // tensor-core jobs: largest coefficient image to fill per run
     struct Realign {
         const uint8_t* src;
         uint8_t* dst;
@@ -583,11 +601,24 @@ extern "C" p2g_status p2g_plan_device_job(uint64_t slice_size, uint32_t input_sl
                                              true, true, with_chains && recovery_count, ctas, 0, split_tail,
                                              mma && recovery_count);
     uint32_t n = 0;
+    if (pl.mma) {
+        // tensor-core plans are reported in the planner's units of 16 rows x
+        // 240 symbols of a band and slice range, which the kernel's tiles cover
+        const uint32_t Np = (uint32_t)(round_up(slice_size, 16) / 2);
+        const uint32_t RG = (recovery_count + kMmaUnitRows - 1) / kMmaUnitRows;
+        for (uint32_t n0 = 0; n0 < Np; n0 += kMmaUnitSymbols)
+            for (uint32_t rg = 0; rg < RG; ++rg)
+                for (uint32_t s0 = 0, cs = n0 >= pl.zero_from_sym ? pl.split_slices : input_slices; s0 < input_slices;
+                     s0 += cs, ++n)
+                    if (n < cap)
+                        items[n] = {rg, 0u, n0, std::min(kMmaUnitSymbols, Np - n0),
+                                    pl.band_syms ? n0 / pl.band_syms : 0u, s0, std::min(cs, input_slices - s0),
+                                    cs < input_slices ? 1u : 0u};
+    }
     for (const BatchItem& it : pl.items) {
-        const uint32_t kind = it.kind_rg & kItemKindMask;
-        if (kind != kItemEncode && kind != kItemEncodeMma) continue;
+        if ((it.kind_rg & kItemKindMask) != kItemEncode) continue;
         if (n < cap)
-            items[n] = {(it.kind_rg >> 8) & 0xFFFFu, kind == kItemEncodeMma ? 0u : 1u << ((it.kind_rg >> 24) & 3u),
+            items[n] = {(it.kind_rg >> 8) & 0xFFFFu, 1u << ((it.kind_rg >> 24) & 3u),
                         it.a, it.b & 0xFFFFu, it.b >> 16, it.s0, it.sn ? it.sn : input_slices,
                         (it.kind_rg & kItemAccumulate) ? 1u : 0u};
         ++n;
@@ -803,7 +834,7 @@ extern "C" p2g_status p2g_batch_create(const p2g_batch_job* jobs, uint32_t n, ui
         }
         if (shape[i].mma) {
             d.mma = 1;
-            d.Rpad = (d.R + kMmaTileRows - 1) / kMmaTileRows * kMmaTileRows;
+            d.rows = mma_rows(d.R);
             d.ksteps = mma_image_steps(d.S);
             d.aimg = A + o_aimg[i];
             b->max_aimg_bytes = std::max<uint64_t>(b->max_aimg_bytes, mma_aimg_bytes(d.S, d.R));

@@ -99,7 +99,7 @@ struct Context {
     cudaEvent_t ev_scratch = nullptr;
     bool scratch_pending = false;
     DevBuf src, src_al, rec, basis, checks, h16k, hfull, pkt, spans, err, tmp_in, tmp_out, md5_state;
-    DevBuf aimg;       // A operand image of the tensor-core encode
+    DevBuf aimg;       // coefficient image of the tensor-core encode
     DevBuf gseg;       // segment table of the one-launch upload of page-locked inputs
     DevBuf persist;    // single-job persistent run: descriptor, items, chain state, tables
     PinBuf h_spans, h_h16k, h_err, h_stage, h_persist, h_gseg;
@@ -429,7 +429,7 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     const size_t o_scratch = take(32ull * n + 12), o_sid = take(16);
     const size_t host_bytes = o_ctl;  // descriptor and items staged together
     // the staging buffer may still feed the previous call's copies, and the
-    // device scratch (descriptor, A image, bases) its kernels, on any stream
+    // device scratch (descriptor, coefficient image, bases) its kernels, on any stream
     if (c.scratch_pending) P2G_CU(cudaEventSynchronize(c.ev_scratch));
     P2G_CU(cudaStreamSynchronize(st));
     P2G_CU(c.persist.ensure(off));
@@ -437,7 +437,7 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     uint8_t* D = c.persist.as<uint8_t>();
     uint8_t* H = c.h_persist.as<uint8_t>();
     // basis (precomputed unless P2G_ENCODE_BASIS=derive) and 16-byte aligned slices
-    const bool gen = generate_basis() || mma;  // the tensor-core items read their A image instead
+    const bool gen = generate_basis() || mma;  // the tensor-core items read their coefficient image instead
     if (j.R && j.S && !gen) P2G_CU(c.basis.ensure(basis_bytes(j.S, RG)));
     if (mma) P2G_CU(c.aimg.ensure(mma_aimg_bytes(j.S, j.R)));
     const uint8_t* esrc = j.d_src;
@@ -480,7 +480,7 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     if (mma) {
         d.mma = 1;
         d.aimg = c.aimg.as<uint8_t>();
-        d.Rpad = (j.R + kMmaTileRows - 1) / kMmaTileRows * kMmaTileRows;
+        d.rows = mma_rows(j.R);
         d.ksteps = mma_image_steps(j.S);
         P2G_CU(make_src_map(&d.src_map, esrc, estride, j.S, (uint32_t)(estride / 2)));
     }
@@ -1180,7 +1180,7 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
             P2G_CU(cudaMemset2DAsync(jb.recovery, jb.recovery_stride, 0, jb.slice_size, R, s));
             return P2G_OK;
         }
-        // the error word, bases and A image are the library's: a call on
+        // the error word, bases and coefficient image are the library's: a call on
         // another stream must not overwrite them while an earlier call reads
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         P2G_CU(cudaStreamIsCapturing(s, &cap));

@@ -129,13 +129,36 @@ cudaError_t launch_encode_noheap(const uint8_t* src, uint64_t src_stride, uint32
 cudaError_t gf_device_tables(const uint16_t** antilog, const uint16_t** logbase);
 
 // The encode on the tensor cores (p2g_mma.cu): a_image_kernel fills `aimg`
-// (mma_aimg_bytes(S, R) of scratch) with the A operand of every 16-row tile
-// and K-step, then the persistent tcgen05 kernel accumulates 16-row x
-// 240-symbol tiles over all S slices.  src rows are read in whole 16-byte
+// (mma_aimg_bytes(S, R) of scratch) with the coefficient operand of every row
+// tile and K-step, then the persistent tcgen05 kernel accumulates tiles of
+// mma_rows(R) rows x 256 symbols over all S slices.  src rows are read in whole 16-byte
 // units, as by launch_encode, through a 2-D tensor map (16-byte aligned src
 // and src_stride).
 size_t mma_aimg_bytes(uint32_t S, uint32_t R);
-// K-steps (4 slices) per 16-row tile in that image: whole 16-slice stages.
+// A tensor-core tile: 256 symbols x up to 13 recovery rows (TMEM's 512 columns
+// hold two accumulators of 16 columns a row, the scale factors and the symbol
+// stages).  R rows take the fewest row tiles of at most 13, evenly: mma_rows(R)
+// rows each.
+constexpr uint32_t kMmaTileSymbols = 256;
+constexpr uint32_t kMmaMaxRows = 13;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr uint32_t mma_rows(uint32_t R) {
+    const uint32_t tiles = (R + kMmaMaxRows - 1) / kMmaMaxRows;
+    return tiles ? (R + tiles - 1) / tiles : 1;
+}
+constexpr uint32_t mma_row_tiles(uint32_t R) { return R ? (R + mma_rows(R) - 1) / mma_rows(R) : 0; }
+// Row tiles that run side by side over one symbol tile before the next: the
+// ~148 tiles at work are then about 8 x 19, and share their coefficients (6.6
+// KB a K-step, 19 ways) and source symbols (2 KB, 8 ways) in L2.
+constexpr uint32_t kMmaRowBlock = 8;
+// The planner's unit of tensor-core work: bands and slice ranges are cut, and
+// p2g_plan_device_job reports, in units of 16 rows x 240 symbols (one M = 256 x
+// N = 240 accumulator); 15 tiles' symbols make 16 units.
+constexpr uint32_t kMmaUnitSymbols = 240;
+constexpr uint32_t kMmaUnitRows = 16;
+// K-steps (4 slices) per row tile in that image: whole 16-slice stages.
 constexpr uint32_t mma_image_steps(uint32_t S) { return (S + 15) / 16 * 4; }
 // The source as a 2-D tensor map of Np u16 symbols x S slices for the
 // tensor-core tiles (cuTensorMapEncodeTiled, found through the runtime).
@@ -158,7 +181,7 @@ enum BatchItemKind : uint32_t {
     kItemPacket = 4,  // packet MD5s of recovery rows [a, a+b) (set id already written)
     kItemCrc = 5,     // slice CRC32 of slices [a, a+b)
     kItemFileHash = 6,  // whole-file MD5 (hash_full) of files [a, a+b), one lane each
-    kItemEncodeMma = 7,  // one (16-row tile, 240-symbol tile) of the accumulator on the tensor cores
+    kItemEncodeMma = 7,  // one (row tile, 256-symbol tile) of the accumulator on the tensor cores
 };
 constexpr uint64_t kCrcItemBytes = 4u << 20;  // source bytes per CRC item
 constexpr uint32_t kItemKindMask = 0x7Fu;
@@ -181,12 +204,10 @@ inline uint32_t encode_kind(uint32_t rg, uint32_t fold, bool acc) {
 }
 
 // Tensor-core encode item: kind_rg = kItemEncodeMma | acc | row tile << 8;
-// a = first symbol, b = band << 16 | symbols (<= 240), s0/sn as for kItemEncode.
+// a = first symbol, b = band << 16 | symbols (<= 256), s0/sn as for kItemEncode.
 inline uint32_t encode_mma_kind(uint32_t rt, bool acc) {
     return kItemEncodeMma | (acc ? kItemAccumulate : 0u) | (rt << 8);
 }
-constexpr uint32_t kMmaTileSymbols = 240;  // symbols of a tensor-core tile (its MMA N)
-constexpr uint32_t kMmaTileRows = 16;      // recovery rows of a tensor-core tile
 
 struct BatchItem {
     uint32_t job;
@@ -227,8 +248,8 @@ struct BatchJob {
     uint32_t ts, first_exp;  // ts: tile width (sub-tile width of folded items)
     uint32_t vec;            // slices and file starts of src are 16-byte aligned
     uint32_t mma;            // encode items run on the tensor cores (kItemEncodeMma)
-    uint8_t* aimg;           // mma: the A operand image (mma_aimg_bytes)
-    uint32_t Rpad, ksteps;   // mma: R rounded up to whole 16-row tiles; the image's K-steps per tile
+    uint8_t* aimg;           // mma: the coefficient image (mma_aimg_bytes)
+    uint32_t rows, ksteps;   // mma: recovery rows per row tile (mma_rows); the image's K-steps per tile
     CUtensorMap src_map;     // mma: esrc as a 2-D tensor (make_src_map); 64-byte aligned
 };
 
@@ -241,6 +262,8 @@ struct SingleJobPlan {
     // recovery columns [zero_from_sym, Np) are written by XOR-accumulating
     // items: the caller zeroes them first (Np: none)
     uint32_t zero_from_sym = 0;
+    uint32_t split_slices = 0;  // slices of each range there
+    bool mma = false;           // the encode items are tensor-core tiles
     double predicted_ms = 0;
 };
 // file_bytes: largest file (non-zero: whole-file MD5 items, kHashFiles files each);
@@ -264,7 +287,7 @@ cudaError_t launch_seeded_fill(uint8_t* base, const uint64_t* spans, const uint6
 // (milliseconds of one CTA).
 double est_md5_ms(uint64_t bytes);
 double est_encode_item_ms(uint32_t slices, uint32_t syms);
-double est_mma_item_ms(uint32_t slices);
+double est_mma_item_ms(uint32_t slices, uint32_t rows);
 // CTA-milliseconds of a job's encode on the lookup or the tensor-core kernel
 // (cost model), and whether the tensor cores are the cheaper.
 double encode_cost_ms(uint64_t slice, uint32_t S, uint32_t R, bool mma);
@@ -280,14 +303,13 @@ double est_set_id_ms(uint32_t files);
 double est_packet_item_ms(uint64_t slice, uint32_t rows);
 // Sets the batch kernel's shared-memory attribute (call before stream capture).
 cudaError_t prepare_batch_kernel();
-// mma: the batch has tensor-core encode items (the CTAs allocate TMEM and
-// need the G^-1 tables of mma_tables_ready()).
+// mma: the batch has tensor-core encode items (the CTAs allocate TMEM) and no
+// lookup ones.
 cudaError_t launch_batch(const BatchJob* jobs, const BatchItem* items, uint32_t n_items, uint32_t* ctl, int* err,
                          uint32_t ctas, cudaStream_t st, bool mma = false);
-// Device address of the 512 G^-1 table entries (256 for the low byte, 256 for
-// the high) after a one-time set-up of the tensor-core tables on this device.
-cudaError_t mma_tables_ready(const uint16_t** ginv);
-// Fills every tensor-core job's A image (blockIdx.y = job); max_bytes: the
+// One-time set-up of the tensor-core tables on this device.
+cudaError_t mma_prepare();
+// Fills every tensor-core job's coefficient image (blockIdx.y = job); max_bytes: the
 // largest image.
 cudaError_t launch_a_image_batch(const BatchJob* jobs, uint32_t n_jobs, uint64_t max_bytes, cudaStream_t st);
 int device_sm_count();

@@ -91,10 +91,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-// Ends an mbarrier object's life, so that its bytes may hold other data.
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
@@ -803,7 +799,8 @@ __device__ void md5_range_ring(uint32_t st[4], const uint32_t* pre, const uint8_
     // ring-eligible blocks: no prefix word, all data words inside whole units
     // (blocks b with 16b + 16 - PW + k <= 16 n_units)
     constexpr uint64_t rb0 = (pre_bytes + 63) / 64;
-    const uint64_t rb1 = n_units * 16 + PW >= k ? (n_units * 16 + PW - k) / 16 : 0;
+    const uint64_t words = n_units * 16 + PW;
+    const uint64_t rb1 = words > k ? (words - k) / 16 : 0;
     auto generic = [&](uint64_t blk) {
         uint32_t m[16];
 #pragma unroll
@@ -811,7 +808,7 @@ __device__ void md5_range_ring(uint32_t st[4], const uint32_t* pre, const uint8_
         md5_compress(st, m);
     };
     uint64_t b = b_from;
-    if (PW)
+    if constexpr (PW > 0)
         for (; b < b_to && b < rb0; ++b) generic(b);
     const uint32_t b0 = (uint32_t)(b_from > rb0 ? b_from : rb0);  // the same in every lane
     const uint32_t end = (uint32_t)(rb1 < b_to ? rb1 : b_to);     // this lane's ring blocks: [b0, end)
@@ -1270,56 +1267,54 @@ constexpr int kBatchRingAhead = 4;
 constexpr int kBatchRingLane = ring_lane_bytes(kBatchRingUnits);
 constexpr size_t kBatchRingBytes = (size_t)kHashThreadsWide * kBatchRingLane;
 static_assert((size_t)kHashThreads * kRingLaneBytes <= kBatchRingBytes, "128 lanes' deep rings fit too");
-// Tensor-core items reuse the encode region and the MD5 rings for their
-// operand and input rings; their barriers, the TMEM address, an abort flag,
-// the pipeline state and the G^-1 tables live past the other regions, so
-// they persist across items.  The MD5 rings start past the tensor-core input
-// stages: a tile's producer issues the next tile's first input stages before
-// the CTA has counted the tile's band, and the packet-MD5 chains that a band
-// completes run on the rings meanwhile (the rings then overlap only operand
-// stages, which are idle between tiles).
-constexpr size_t kBatchRingOff = ((kBatchEncBytes > (size_t)mma::kInStages * mma::kInStageBytes
-                                       ? kBatchEncBytes
-                                       : (size_t)mma::kInStages * mma::kInStageBytes) + 15) / 16 * 16;
-constexpr size_t kBatchMmaBarsOff = kBatchRingOff + kBatchRingBytes + 4 * 256 * 4 + 64;
-// the G^-1 tables of tensor-core items, copied once per launch, after the
-// pipeline state words
-constexpr size_t kBatchGinvOff = kBatchMmaBarsOff + mma::kBarBytes + 32;
-// the next tile a tensor-core tile's producer claimed (one mma::Tile)
-constexpr size_t kBatchNextTileOff = (kBatchGinvOff + mma::kGinvBytes + 15) / 16 * 16;
-constexpr size_t kBatchSmem = kBatchNextTileOff + 64;
-static_assert(sizeof(mma::Tile) <= 64 && kBatchNextTileOff % 16 == 0, "next-tile slot");
-static_assert(kBatchEncBytes % 16 == 0 && kBatchRingOff % 16 == 0, "MD5 rings must start 16-byte aligned");
-static_assert(mma::kRingBytes <= kBatchRingOff + kBatchRingBytes,
-              "tensor-core rings fit the encode region and the MD5 rings");
-static_assert(kBatchMmaBarsOff % 8 == 0 && kBatchSmem <= 227 * 1024, "batch shared memory");
-size_t batch_smem_bytes() { return kBatchSmem; }
+constexpr size_t kBatchRingOff = (kBatchEncBytes + 15) / 16 * 16;
+constexpr size_t kBatchTabOff = kBatchRingOff + kBatchRingBytes;  // CRC tables, then 16 words of CTA state
+constexpr size_t kBatchSmem = kBatchTabOff + 4 * 256 * 4 + 64;
+// Launches with tensor-core items (and no lookup ones) lay it out otherwise:
+// five input stages first.  A tile's producer issues the next tile's first
+// stages before the CTA has counted the tile's band, and the packet-MD5 chains
+// that a band completes run meanwhile; so those chains have rings of their own
+// past the stages (128 lanes, 6 units), while the other MD5 items, which never
+// run with a stage in flight, use the stages' bytes.  Then the CRC tables and
+// state words as above, the pipeline's barriers, TMEM address, abort flag and
+// state.
+constexpr int kBatchInStages = 5;
+constexpr size_t kBatchMmaChainOff = (size_t)kBatchInStages * mma::kInStageBytes;
+constexpr size_t kBatchMmaTabOff = kBatchMmaChainOff + (size_t)kHashThreads * kBatchRingLane;
+constexpr size_t kBatchMmaBarsOff = kBatchMmaTabOff + 4 * 256 * 4 + 64;
+constexpr size_t kBatchMmaSmem = kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages) + 32;
+static_assert(kBatchEncBytes % 16 == 0 && kBatchRingOff % 16 == 0 && kBatchMmaChainOff % 16 == 0,
+              "MD5 rings must start 16-byte aligned");
+static_assert(kBatchRingBytes <= kBatchMmaChainOff, "the wide MD5 rings fit the tensor-core input stages");
+static_assert(kBatchMmaBarsOff % 8 == 0 && kBatchSmem <= 227 * 1024 && kBatchMmaSmem <= 227 * 1024,
+              "batch shared memory");
+size_t batch_smem_bytes() { return kBatchSmem > kBatchMmaSmem ? kBatchSmem : kBatchMmaSmem; }
 
 // The tile of a tensor-core item.
 __device__ __forceinline__ mma::Tile batch_mma_tile_of(const BatchJob& J, const BatchItem& it) {
     mma::Tile T;
     T.src_map = &J.src_map;
-    T.aimg = J.aimg;
+    const uint32_t rt = (it.kind_rg >> 8) & 0xFFFFu;
+    T.aimg = J.aimg + (size_t)rt * J.ksteps * J.rows * mma::kRowStepBytes;
     T.rec = J.rec;
     T.rec_stride = J.rec_stride;
     T.s0 = it.s0;
     T.sn = it.sn ? it.sn : J.S - it.s0;
-    T.ksteps = J.ksteps;
+    T.rows = J.rows;
     T.R = J.R;
-    T.r0 = ((it.kind_rg >> 8) & 0xFFFFu) * kMmaTileRows;
+    T.r0 = rt * J.rows;
     T.n0 = it.a;
     T.syms = it.b & 0xFFFFu;
     T.accumulate = (it.kind_rg & kItemAccumulate) ? 1u : 0u;
     return T;
 }
 
-// One tensor-core item of the batch kernel, all threads: 14 operand-building
-// warps (warps 2..15).  Kept out of line, with its pipeline state in shared
-// memory (words [2..6] past the barriers: operand stages, tiles, drains,
-// input stages, stages issued ahead), so that it adds no registers to the
-// other item kinds.
+// One tensor-core item of the batch kernel, all threads.  Kept out of line,
+// with its pipeline state in shared memory (words [3], [5], [6] past the
+// barriers: tiles, input stages, stages issued ahead), so that it adds no
+// registers to the other item kinds.
 //
-// The CTA's next item is claimed from the queue here, by the producer thread
+// The CTA's next item is claimed from the queue here, by one thread of warp 0
 // once it has issued this tile's last input stage (a few K-steps before the
 // tile ends, about when the CTA would otherwise claim it); its index goes to
 // *held (shared memory, read by every thread after this returns) and its
@@ -1334,8 +1329,7 @@ __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, c
                                             uint32_t n_items, uint32_t* __restrict__ ctl, const int* err,
                                             uint32_t idx, uint32_t* held) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint32_t* mm = reinterpret_cast<uint32_t*>(smem + kBatchMmaBarsOff + mma::kBarBytes);
-    const uint16_t* gsm = reinterpret_cast<const uint16_t*>(smem + kBatchGinvOff);  // filled at launch start
+    uint32_t* mm = reinterpret_cast<uint32_t*>(smem + kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages));
     // Earlier items stored to this shared memory through the generic proxy;
     // the tile's bulk and tensor copies write it through the async proxy.
     // Order the two before any copy is issued.
@@ -1347,42 +1341,36 @@ __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, c
     P.ring = smem_u32(smem);
     P.bars = smem_u32(smem + kBatchMmaBarsOff);
     P.tmem = mm[0];
-    P.ginv = gsm;
     P.abort_flag = mm + 1;
-    P.g = mm[2];
     P.tcount = mm[3];
-    P.drains = mm[4];
     P.gi = mm[5];
     P.pre = mm[6];
-    if (threadIdx.x == 0) mma::tensormap_acquire(&J.src_map);  // written by the host's upload of the jobs
+    if (threadIdx.x < 32) mma::tensormap_acquire(&J.src_map);  // written by the host's upload of the jobs
     const mma::Tile T = batch_mma_tile_of(J, it);
-    // producer thread only (thread 0); the tile goes to its shared-memory slot
-    auto claim_next = [&]() -> const mma::Tile* {
+    // one thread of warp 0
+    auto claim_next = [&](mma::Tile& next) {
         *held = kNoHeldItem;
-        if (*reinterpret_cast<const volatile int*>(err)) return nullptr;
+        if (*reinterpret_cast<const volatile int*>(err)) return false;
         if (J.n_bands) {
             const uint32_t band = it.b >> 16;
             const uint32_t done = *reinterpret_cast<const volatile uint32_t*>(&J.bstate[band]);
-            if (done + kClaimMargin >= J.band_items[band]) return nullptr;
+            if (done + kClaimMargin >= J.band_items[band]) return false;
         }
         const uint32_t h = *reinterpret_cast<const volatile uint32_t*>(&ctl[0]);
-        if (h >= n_items || (items[h].kind_rg & kItemKindMask) != kItemEncodeMma) return nullptr;
+        if (h >= n_items || (items[h].kind_rg & kItemKindMask) != kItemEncodeMma) return false;
         const uint32_t nidx = atomicAdd(&ctl[0], 1u);
         *held = nidx;
-        if (nidx >= n_items) return nullptr;
+        if (nidx >= n_items) return false;
         const BatchItem nit = items[nidx];
-        if ((nit.kind_rg & kItemKindMask) != kItemEncodeMma) return nullptr;
+        if ((nit.kind_rg & kItemKindMask) != kItemEncodeMma) return false;
         const BatchJob& Jn = jobs[nit.job];
         mma::tensormap_acquire(&Jn.src_map);
-        mma::Tile* slot = reinterpret_cast<mma::Tile*>(smem + kBatchNextTileOff);
-        *slot = batch_mma_tile_of(Jn, nit);
-        return slot;
+        next = batch_mma_tile_of(Jn, nit);
+        return true;
     };
-    const bool ok = mma::run_tile<14>(P, T, claim_next);  // ends with a CTA barrier
+    const bool ok = mma::run_tile<kBatchInStages>(P, T, claim_next);  // ends with a CTA barrier
     if (threadIdx.x == 0) {
-        mm[2] = P.g;
         mm[3] = P.tcount;
-        mm[4] = P.drains;
         mm[5] = P.gi;
         mm[6] = P.pre;
     }
@@ -1553,6 +1541,7 @@ __device__ __noinline__ void batch_packets(const BatchJob& J, uint32_t ring, con
 // Chain segment: rows of block q advance over the message blocks that bands
 // b..b_last completed (set id ‖ type ‖ exponent ‖ row bytes; the last band
 // also pads and writes the digests).  State between passes lives in J.chain.
+template <int UNITS, int AHEAD>
 __device__ __noinline__ void advance_rows(const BatchJob& J, uint32_t q, uint32_t b, uint32_t b_last, uint32_t ring,
                                           const uint32_t* sid) {
     const int tid = threadIdx.x;
@@ -1582,8 +1571,8 @@ __device__ __noinline__ void advance_rows(const BatchJob& J, uint32_t q, uint32_
             st[2] = v.z;
             st[3] = v.w;
         }
-        md5_range_ring<9, true, true>(st, pre, J.rec + (size_t)r * J.rec_stride, live ? J.slice : 0, from,
-                                      live ? to : 0, ring + (tid & ~31) * kRingLaneBytes);
+        md5_range_ring<9, true, true, UNITS, AHEAD>(st, pre, J.rec + (size_t)r * J.rec_stride, live ? J.slice : 0,
+                                                    from, live ? to : 0, ring + (tid & ~31) * ring_lane_bytes(UNITS));
         if (final && live)
             store_digest(J.pkt + 16 * (size_t)r, st);
         else if (live)
@@ -1599,6 +1588,7 @@ __device__ __noinline__ void advance_rows(const BatchJob& J, uint32_t q, uint32_
 // pass either advances at least one band or returns, so this ends.  No CTA
 // waits for another: a busy token means its holder will see the new band.
 constexpr uint32_t kChainBandsPerPass = 16;
+template <int UNITS, int AHEAD>
 __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32_t* misc) {
     const int tid = threadIdx.x;
     const uint32_t nb = J.n_bands, Q = (J.R + kChainRows - 1) / kChainRows;
@@ -1632,7 +1622,7 @@ __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32
             __syncthreads();
             if (!k) break;
             __threadfence();  // acquire: the bands' rows and the set id
-            advance_rows(J, q, b, b + k - 1, ring, misc + 4);
+            advance_rows<UNITS, AHEAD>(J, q, b, b + k - 1, ring, misc + 4);
             if (tid == 0) {
                 __threadfence();
                 atomicExch(&next[q], b + k);
@@ -1655,43 +1645,43 @@ __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32
 // All row blocks, starting with block `first` mod Q: the CTAs that complete
 // neighbouring bands start on different blocks, so that the blocks advance
 // side by side.
+template <bool MMA>
 __device__ void advance_all(const BatchJob& J, uint32_t first, uint32_t ring, uint32_t* misc) {
+    constexpr int UNITS = MMA ? kBatchRingUnits : kRingUnits, AHEAD = MMA ? kBatchRingAhead : kRingAhead;
     const uint32_t Q = (J.R + kChainRows - 1) / kChainRows;
-    for (uint32_t i = 0; i < Q; ++i) try_advance(J, (first + i) % Q, ring, misc);
+    for (uint32_t i = 0; i < Q; ++i) try_advance<UNITS, AHEAD>(J, (first + i) % Q, ring, misc);
 }
 
-// MMA: the launch has tensor-core items (mma_ginv set).  The variant without
-// them keeps the other item kinds' code free of the tensor pipeline's
+// MMA: the launch has tensor-core items and no lookup ones.  The variant
+// without them keeps the lookup items' code free of the tensor pipeline's
 // registers.
 template <bool MMA>
 __global__ void __launch_bounds__(kEncThreads, 1)
     batch_kernel(const BatchJob* __restrict__ jobs, const BatchItem* __restrict__ items, uint32_t n_items,
-                 uint32_t* __restrict__ ctl, int* __restrict__ err, const uint16_t* __restrict__ mma_ginv) {
+                 uint32_t* __restrict__ ctl, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* enc = smem;
     uint64_t* bars = reinterpret_cast<uint64_t*>(enc + encode_bars_offset<kEncChunks, 4, kBatchEncStages>());
-    uint8_t* ring_p = smem + kBatchRingOff;
-    uint32_t(*T)[256] = reinterpret_cast<uint32_t(*)[256]>(ring_p + kBatchRingBytes);
+    uint8_t* ring_p = smem + (MMA ? 0 : kBatchRingOff);  // MD5 rings, but for the chains of
+    const uint32_t chain_ring = smem_u32(smem + (MMA ? kBatchMmaChainOff : kBatchRingOff));
+    uint8_t* tab_p = smem + (MMA ? kBatchMmaTabOff : kBatchTabOff);
+    uint32_t(*T)[256] = reinterpret_cast<uint32_t(*)[256]>(tab_p);
     // [0] item [1] last [2..3] chain tokens [4..7] set id [8] item claimed ahead by a tensor-core tile
-    uint32_t* misc = reinterpret_cast<uint32_t*>(ring_p + kBatchRingBytes + 4 * 256 * 4);
+    uint32_t* misc = reinterpret_cast<uint32_t*>(tab_p + 4 * 256 * 4);
     const uint32_t ring = smem_u32(ring_p);
     const int tid = threadIdx.x;
-    // tensor-core items (mma_ginv set): TMEM for the whole launch, barriers
-    // and scale factors set up once.  mma_misc: [0] TMEM address, [1] abort
-    // flag, [2..6] pipeline state.
-    uint32_t* mma_misc = reinterpret_cast<uint32_t*>(smem + kBatchMmaBarsOff + mma::kBarBytes);
+    // tensor-core launches: TMEM for the whole launch, barriers and scale
+    // factors set up once.  mma_misc: [0] TMEM address, [1] abort flag, [3..6]
+    // pipeline state.
+    uint32_t* mma_misc = reinterpret_cast<uint32_t*>(smem + kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages));
     const uint32_t mma_bars = smem_u32(smem + kBatchMmaBarsOff);
-    // The lookup items' barriers lie inside the tensor-core input stages.
-    // Launches with tensor-core items set them up only around a lookup item
-    // and invalidate them after it (an mbarrier's bytes may hold other data
-    // only once it is invalidated); such launches plan no lookup items.
     if (tid == 0) {
         misc[8] = kNoHeldItem;
         if (!MMA)
             for (int st = 0; st < kBatchEncStages; ++st) mbar_init(&bars[st], 1);
         if (MMA) {
-            mma::init_bars(mma_bars, 14);
-            mma_misc[1] = mma_misc[2] = mma_misc[3] = mma_misc[4] = mma_misc[5] = mma_misc[6] = 0;
+            mma::init_bars<kBatchInStages>(mma_bars);
+            mma_misc[1] = mma_misc[3] = mma_misc[5] = mma_misc[6] = 0;
         }
         fence_mbar_init();
     }
@@ -1701,8 +1691,6 @@ __global__ void __launch_bounds__(kEncThreads, 1)
     if (MMA) {
         mma::tc_fence_after();
         if ((tid >> 5) >= 4 && (tid >> 5) < 8) mma::sf_fill(mma_misc[0], (uint32_t)(tid >> 5) & 3u);
-        uint16_t* gsm = reinterpret_cast<uint16_t*>(smem + kBatchGinvOff);
-        for (int i = tid; i < 512; i += kEncThreads) gsm[i] = mma_ginv[i];
         mma::tc_fence_before();
         __syncthreads();
         mma::tc_fence_after();
@@ -1762,7 +1750,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
                     atomicExch(J.bstate + J.n_bands + 2 * ((J.R + kChainRows - 1) / kChainRows), 1u);
                 }
                 __syncthreads();
-                advance_all(J, 0, ring, misc);
+                advance_all<MMA>(J, 0, chain_ring, misc);
             }
             continue;
         }
@@ -1774,10 +1762,6 @@ __global__ void __launch_bounds__(kEncThreads, 1)
         }
         if (MMA && kind == kItemEncodeMma) {
             const bool ok = batch_mma_tile(jobs, items, n_items, ctl, err, idx, misc + 8);
-            // the builders' generic stores come before any later item's bulk
-            // copies (async proxy) into the same bytes
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
             if (!ok) {
                 if (tid == 0) atomicOr(err, 1);
                 break;
@@ -1790,18 +1774,10 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             __syncthreads();
             if (!misc[1]) continue;
             __threadfence();  // acquire: the whole band is visible from here on
-            advance_all(J, band, ring, misc);
+            advance_all<MMA>(J, band, chain_ring, misc);
             continue;
         }
-        if (kind == kItemEncode) {
-            if (MMA) {  // its barriers, set up for this item alone (nothing is in flight now)
-                if (tid == 0) {
-                    for (int st = 0; st < kBatchEncStages; ++st) mbar_init(&bars[st], 1);
-                    fence_mbar_init();
-                }
-                phase = 0;
-                __syncthreads();
-            }
+        if (!MMA && kind == kItemEncode) {
             // the job's precomputed basis when it has one, else derived per slice
             const uint32_t rg = (it.kind_rg >> 8) & 0xFFFFu, sn = it.sn ? it.sn : J.S;
             const uint32_t fold = 1u << ((it.kind_rg >> 24) & 3u);
@@ -1813,13 +1789,6 @@ __global__ void __launch_bounds__(kEncThreads, 1)
                                     : encode_tile<kEncChunks, true, 4, kBatchEncStages>(J.esrc, J.estride, sn, nullptr, J.RG, rg, J.R,
                                                                         it.a, syms, J.rec, J.rec_stride, enc, phase,
                                                                         J.first_exp, it.s0, acc, fold, J.ts);
-            if (MMA) {  // the barriers' bytes go back to the tensor-core input stages
-                __syncthreads();
-                if (tid == 0)
-                    for (int st = 0; st < kBatchEncStages; ++st) mbar_inval(&bars[st]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncthreads();
-            }
             if (!ok) {
                 if (tid == 0) atomicOr(err, 1);
                 break;
@@ -1831,7 +1800,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             __syncthreads();
             if (!misc[1]) continue;
             __threadfence();  // acquire: the whole band is visible from here on
-            advance_all(J, band, ring, misc);
+            advance_all<MMA>(J, band, chain_ring, misc);
         }
     }
     if (MMA) {  // every MMA issued has completed before TMEM is given back
@@ -1841,15 +1810,15 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             // input stages issued ahead for a tile that did not run (the loop
             // always runs a claimed tile, so this stays idle): they land before
             // the CTA exits
-            const mma::Bars B(mma_bars);
+            const mma::Bars<kBatchInStages> B(mma_bars);
             for (uint32_t q = mma_misc[5]; q < mma_misc[5] + mma_misc[6]; ++q)
-                mma::bar_drain(B.in_full + 8 * (q % mma::kInStages), (q / mma::kInStages) & 1u);
+                mma::bar_drain(B.in_full + 8 * (q % kBatchInStages), (q / kBatchInStages) & 1u);
         }
         if ((tid >> 5) == 1) {
             if ((tid & 31) == 0) {
-                const mma::Bars B(mma_bars);
+                const mma::Bars<kBatchInStages> B(mma_bars);
                 mma::mma_commit(B.drain);
-                mma::bar_drain(B.drain, mma_misc[4] & 1u);
+                mma::bar_drain(B.drain, 0);
             }
             __syncwarp();
             mma::tc_fence_after();
@@ -2301,7 +2270,8 @@ cudaError_t prepare_batch_kernel() {
         cudaError_t e =
             cudaFuncSetAttribute(batch_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem);
+            e = cudaFuncSetAttribute(batch_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kBatchMmaSmem);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 256) attr_set[dev] = true;
     }
@@ -2313,12 +2283,10 @@ cudaError_t launch_batch(const BatchJob* jobs, const BatchItem* items, uint32_t 
     if (!n_items) return cudaSuccess;
     cudaError_t e = prepare_batch_kernel();
     if (e != cudaSuccess) return e;
-    const uint16_t* ginv = nullptr;
-    if (mma && (e = mma_tables_ready(&ginv)) != cudaSuccess) return e;
     if (mma)
-        batch_kernel<true><<<ctas, kEncThreads, kBatchSmem, st>>>(jobs, items, n_items, ctl, err, ginv);
+        batch_kernel<true><<<ctas, kEncThreads, kBatchMmaSmem, st>>>(jobs, items, n_items, ctl, err);
     else
-        batch_kernel<false><<<ctas, kEncThreads, kBatchSmem, st>>>(jobs, items, n_items, ctl, err, nullptr);
+        batch_kernel<false><<<ctas, kEncThreads, kBatchSmem, st>>>(jobs, items, n_items, ctl, err);
     count_launch();
     return cudaGetLastError();
 }

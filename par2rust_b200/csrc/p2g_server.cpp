@@ -168,21 +168,20 @@ void plan_job(p2g_server* s, SJob& j) {
     j.todo.push_back({j.slot, kItemSetId, 0, 0, 0, 0});
     j.todo_ms.push_back(est_set_id_ms(j.n));
     if (j.R && j.mma) {
-        // tensor-core items: 16-row tiles x 240 symbols, slice chunks on whole
-        // 16-slice stages of the A image, again at most ~wave_ms/4 each
-        const double per_stage = est_mma_item_ms(16) - est_mma_item_ms(0);
+        // tensor-core items: row tiles x 256 symbols, slice chunks on whole
+        // 16-slice stages of the coefficient image, again at most ~wave_ms/4 each
+        const uint32_t rows = mma_rows(j.R), RT = mma_row_tiles(j.R);
+        const double per_stage = est_mma_item_ms(16, rows) - est_mma_item_ms(0, rows);
         uint32_t mchunk = (uint32_t)std::max(1.0, floor(s->wave_ms / 4.0 / per_stage)) * 16;
         if (mchunk >= j.S) mchunk = j.S;
         const uint32_t mchunks = (j.S + mchunk - 1) / mchunk;
-        const uint32_t mtiles = (j.Np + kMmaTileSymbols - 1) / kMmaTileSymbols;
-        const uint32_t RT = (j.R + kMmaTileRows - 1) / kMmaTileRows;
-        for (uint32_t t = 0; t < mtiles; ++t) {
-            const uint32_t n0 = t * kMmaTileSymbols, syms = std::min(kMmaTileSymbols, j.Np - n0);
+        for (uint32_t n0 = 0; n0 < j.Np; n0 += kMmaTileSymbols) {
+            const uint32_t syms = std::min(kMmaTileSymbols, j.Np - n0);
             for (uint32_t c = 0; c < mchunks; ++c) {
                 const uint32_t s0 = c * mchunk, sn = std::min(mchunk, j.S - s0);
                 for (uint32_t rt = 0; rt < RT; ++rt) {
                     j.todo.push_back({j.slot, encode_mma_kind(rt, mchunks > 1), n0, syms, s0, sn});
-                    j.todo_ms.push_back(est_mma_item_ms(sn));
+                    j.todo_ms.push_back(est_mma_item_ms(sn, rows));
                     j.enc_total++;
                 }
             }
@@ -291,7 +290,7 @@ p2g_status admit(p2g_server* s) {
         if (j.mma) {
             d.mma = 1;
             d.aimg = take(aimg_b);
-            d.Rpad = (j.R + kMmaTileRows - 1) / kMmaTileRows * kMmaTileRows;
+            d.rows = mma_rows(j.R);
             d.ksteps = mma_image_steps(j.S);
             const cudaError_t me = make_src_map(&d.src_map, d.esrc, d.estride, j.S, (uint32_t)(d.estride / 2));
             if (me != cudaSuccess) return fail_cuda(s, me, "tensor map");
@@ -449,7 +448,7 @@ p2g_status launch_wave(p2g_server* s, bool* launched) {
     for (auto& [j, it] : w.items) {
         const uint32_t k = it.kind_rg & kItemKindMask;
         const double ms = k == kItemEncode      ? est_encode_item_ms(it.sn, std::min(it.b & 0xFFFFu, j->desc.ts))
-                          : k == kItemEncodeMma ? est_mma_item_ms(it.sn)
+                          : k == kItemEncodeMma ? est_mma_item_ms(it.sn, mma_rows(j->R))
                           : k == kItemScan ? est_scan_item_ms(j->slice, it.b)
                           : k == kItemCrc ? est_crc_item_ms(j->slice, it.b)
                           : k == kItemSetId ? est_set_id_ms(j->n)
@@ -599,7 +598,7 @@ extern "C" p2g_status p2g_server_submit(p2g_server* s, const p2g_server_job* rq,
     j->RG = (j->R + kRowsPerGroup - 1) / kRowsPerGroup;
     j->Np = (uint32_t)(round_up(j->slice, 16) / 2);
     j->footprint = S * j->slice + (uint64_t)j->R * round_up(j->slice, 16);
-    // tensor-core encode when the cost model prefers it and the A image
+    // tensor-core encode when the cost model prefers it and the coefficient image
     // (R x S x 128 B) stays within a quarter of the source bytes
     const char* ev = getenv("P2G_ENCODE_VARIANT");  // "lut" / "tensor" force a kind (tensor: if the image fits)
     const bool want_mma = ev && !strcmp(ev, "lut") ? false
