@@ -76,6 +76,7 @@ struct PlanJob {
     // mma_rows(R) rows x 256 symbols of a band.
     bool mma = false;
     uint32_t scan_slices = kScanSlices;  // slices per scan item
+    bool lone = false;                   // the launch's only job: may have chain items
 };
 
 double finish_ms(const PlanJob& j) { return est_set_id_ms(j.n) + est_packet_item_ms(j.slice, j.R); }
@@ -102,6 +103,7 @@ struct Plan {
 constexpr uint32_t kMaxBands = 64;  // packet-MD5 chain segments per job (64: 10.27 ms vs 10.59 at 16 for 538 MB / R 200)
 
 constexpr uint32_t kMaxMmaBands = 72;
+constexpr double kMaxCtas = 148;  // SMs of a B200
 
 // Bands of job j: runs of band_tiles consecutive tiles, a multiple of the
 // tail fold so that no folded item straddles two bands.  Tensor-core bands are
@@ -168,6 +170,13 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
         if (!j.R) continue;
         uint32_t bt = 0, nb = 0;
         job_bands(j, &bt, &nb);
+        // A job alone whose chains last more than half as long as its encode
+        // keeps one CTA on each row block's chains: left to the CTAs that
+        // complete bands, the blocks' last bands ran one after the other (538
+        // MB, 200 rows: encode done at 4.3 ms, chains at 5.2).
+        if (j.lone && j.chains && nb > 1 && 2 * md5_ms(j.slice + 36) * kMaxCtas > encode_cost_ms(j.slice, j.S, j.R, j.mma))
+            for (uint32_t q = 0; q < (j.R + kChainRows - 1) / kChainRows; ++q)
+                pre.push_back({9e29, {ji, kItemChain, q, 0, 0, 0}});
         const uint32_t F = j.mma ? 1u : tail_fold(j.R);
         p.band_syms[ji] = bt * j.ts;
         p.band_items[ji].assign(nb, 0);
@@ -237,6 +246,7 @@ double item_ms(const PlanJob& j, const BatchItem& it) {
     case kItemScan: return scan_ms(j, it.b);
     case kItemCrc: return est_crc_item_ms(j.slice, it.b);
     case kItemFileHash: return md5_ms(j.file_bytes) + kItemMs;
+    case kItemChain: return md5_ms(j.slice + 36) + kItemMs;
     case kItemEncodeMma:
         return est_mma_item_ms(it.sn ? it.sn : j.S, mma_rows(j.R)) * ((it.kind_rg & kItemAccumulate) ? kAccCost : 1.0);
     case kItemEncode: {
@@ -485,6 +495,7 @@ SingleJobPlan plan_single_job_uncached(uint64_t slice, uint32_t S, uint32_t R, u
     jobs[0].n = std::max(1u, n_files);
     jobs[0].scans = scans;
     jobs[0].scan_slices = kLoneScanSlices;
+    jobs[0].lone = true;
     jobs[0].set_id = set_id;
     jobs[0].chains = chains && R;
     jobs[0].file_bytes = file_bytes;

@@ -181,6 +181,7 @@ enum BatchItemKind : uint32_t {
     kItemPacket = 4,  // packet MD5s of recovery rows [a, a+b) (set id already written)
     kItemCrc = 5,     // slice CRC32 of slices [a, a+b)
     kItemFileHash = 6,  // whole-file MD5 (hash_full) of files [a, a+b), one lane each
+    kItemChain = 8,  // packet-MD5 chains of rows [128a, 128a + 128), kept by one CTA until the last band
     kItemEncodeMma = 7,  // one (row tile, 256-symbol tile) of the accumulator on the tensor cores
 };
 constexpr uint64_t kCrcItemBytes = 4u << 20;  // source bytes per CRC item

@@ -1277,12 +1277,14 @@ constexpr size_t kBatchSmem = kBatchTabOff + 4 * 256 * 4 + 64;
 // past the stages (128 lanes, 6 units), while the other MD5 items, which never
 // run with a stage in flight, use the stages' bytes.  Then the CRC tables and
 // state words as above, the pipeline's barriers, TMEM address, abort flag and
-// state.
+// state, and two tile slots.
+constexpr uint32_t kNoHeldItem = 0xFFFFFFFFu;
 constexpr int kBatchInStages = 5;
 constexpr size_t kBatchMmaChainOff = (size_t)kBatchInStages * mma::kInStageBytes;
 constexpr size_t kBatchMmaTabOff = kBatchMmaChainOff + (size_t)kHashThreads * kBatchRingLane;
 constexpr size_t kBatchMmaBarsOff = kBatchMmaTabOff + 4 * 256 * 4 + 64;
-constexpr size_t kBatchMmaSmem = kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages) + 32;
+constexpr size_t kBatchSlotOff = (kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages) + 32 + 15) / 16 * 16;
+constexpr size_t kBatchMmaSmem = kBatchSlotOff + 2 * 80;
 static_assert(kBatchEncBytes % 16 == 0 && kBatchRingOff % 16 == 0 && kBatchMmaChainOff % 16 == 0,
               "MD5 rings must start 16-byte aligned");
 static_assert(kBatchRingBytes <= kBatchMmaChainOff, "the wide MD5 rings fit the tensor-core input stages");
@@ -1309,34 +1311,39 @@ __device__ __forceinline__ mma::Tile batch_mma_tile_of(const BatchJob& J, const 
     return T;
 }
 
-// One tensor-core item of the batch kernel, all threads.  Kept out of line,
-// with its pipeline state in shared memory (words [3], [5], [6] past the
-// barriers: tiles, input stages, stages issued ahead), so that it adds no
-// registers to the other item kinds.
+// One tensor-core tile of the batch kernel, all threads: the one in slot
+// tcount & 1 of the shared-memory slots; the other slot receives the tile that
+// this CTA runs next (T.rows 0: none).  Kept out of line, with its pipeline
+// state in shared memory (mma_misc), so that it adds no registers to the other
+// item kinds.
 //
-// The CTA's next item is claimed from the queue here, by one thread of warp 0
-// once it has issued this tile's last input stage (a few K-steps before the
-// tile ends, about when the CTA would otherwise claim it); its index goes to
-// *held (shared memory, read by every thread after this returns) and its
-// first input stages are issued at once.  Nothing is claimed ahead
-// (held = kNoHeldItem) once the error flag is set, when the queue head is not
-// a tensor-core item, or when fewer than kClaimMargin other tiles of this
-// tile's band are unfinished: the CTA that completes a band runs its
-// packet-MD5 chains next, and a claimed item would wait behind them.
-constexpr uint32_t kNoHeldItem = 0xFFFFFFFFu;
+// The helper warp first counts the CTA's previous tile of the run (its slot is
+// the one about to be overwritten) in that tile's band, so that no thread
+// waits for the atomic between two tiles; a band that this completes is left
+// in adv (shared, job + 1 and band; two pairs, so that a slow warp still reads
+// this tile's while the next tile's helper writes) for the CTA to advance
+// after this tile.
+// Then it claims the CTA's next item from the queue, ~4 us before the tile
+// ends (about when the CTA would otherwise claim it), so that the tile's first
+// input stages are in flight when it starts.  Nothing is claimed ahead once the error
+// flag is set, when the queue head is not a tensor-core item, or when fewer
+// than kClaimMargin other tiles of this tile's band are unfinished: the CTA
+// that completes a band runs its packet-MD5 chains next, and a claimed item
+// would wait behind them.  In one job of 538 MB a tile took 41.6 us with the
+// count, the pop and the descriptor loads between two tiles (4,500 cycles), and
+// 36.8 us this way.
 constexpr uint32_t kClaimMargin = 8;
+struct MmaSlot {
+    mma::Tile T;
+    uint32_t job, band;
+};
+static_assert(sizeof(MmaSlot) <= 80, "slots");
 __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, const BatchItem* __restrict__ items,
                                             uint32_t n_items, uint32_t* __restrict__ ctl, const int* err,
-                                            uint32_t idx, uint32_t* held) {
+                                            uint32_t count_prev, uint32_t* adv, uint32_t* held) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint32_t* mm = reinterpret_cast<uint32_t*>(smem + kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages));
-    // Earlier items stored to this shared memory through the generic proxy;
-    // the tile's bulk and tensor copies write it through the async proxy.
-    // Order the two before any copy is issued.
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    const BatchItem it = items[idx];
-    const BatchJob& J = jobs[it.job];
+    MmaSlot* slots = reinterpret_cast<MmaSlot*>(smem + kBatchSlotOff);
     mma::Pipe P;
     P.ring = smem_u32(smem);
     P.bars = smem_u32(smem + kBatchMmaBarsOff);
@@ -1345,30 +1352,43 @@ __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, c
     P.tcount = mm[3];
     P.gi = mm[5];
     P.pre = mm[6];
-    if (threadIdx.x < 32) mma::tensormap_acquire(&J.src_map);  // written by the host's upload of the jobs
-    const mma::Tile T = batch_mma_tile_of(J, it);
-    // one thread of warp 0
-    auto claim_next = [&](mma::Tile& next) {
-        *held = kNoHeldItem;
-        if (*reinterpret_cast<const volatile int*>(err)) return false;
+    P.issued = mm + 7;
+    MmaSlot& cur = slots[P.tcount & 1u];
+    MmaSlot& nxt = slots[(P.tcount & 1u) ^ 1u];
+    P.next = &nxt.T;
+    if (threadIdx.x < 32) mma::tensormap_acquire(cur.T.src_map);  // written by the host's upload of the jobs
+    const bool ok = mma::run_tile<kBatchInStages>(P, cur.T, [&] {
+        if (threadIdx.x & 31) return;
+        const BatchJob& J = jobs[cur.job];
+        if (count_prev && jobs[nxt.job].n_bands) {
+            const BatchJob& Jp = jobs[nxt.job];
+            __threadfence();  // the tile's rows, stored before the CTA barrier at its end
+            if (atomicAdd(&Jp.bstate[nxt.band], 1u) + 1 == Jp.band_items[nxt.band]) {
+                adv[1] = nxt.band;
+                adv[0] = nxt.job + 1;
+            }
+        }
+        nxt.T.rows = 0;
+        if (*reinterpret_cast<const volatile int*>(err)) return;
         if (J.n_bands) {
-            const uint32_t band = it.b >> 16;
-            const uint32_t done = *reinterpret_cast<const volatile uint32_t*>(&J.bstate[band]);
-            if (done + kClaimMargin >= J.band_items[band]) return false;
+            const uint32_t done = *reinterpret_cast<const volatile uint32_t*>(&J.bstate[cur.band]);
+            if (done + kClaimMargin >= J.band_items[cur.band]) return;
         }
         const uint32_t h = *reinterpret_cast<const volatile uint32_t*>(&ctl[0]);
-        if (h >= n_items || (items[h].kind_rg & kItemKindMask) != kItemEncodeMma) return false;
-        const uint32_t nidx = atomicAdd(&ctl[0], 1u);
-        *held = nidx;
-        if (nidx >= n_items) return false;
-        const BatchItem nit = items[nidx];
-        if ((nit.kind_rg & kItemKindMask) != kItemEncodeMma) return false;
-        const BatchJob& Jn = jobs[nit.job];
+        if (h >= n_items || (items[h].kind_rg & kItemKindMask) != kItemEncodeMma) return;
+        const uint32_t idx = atomicAdd(&ctl[0], 1u);
+        if (idx >= n_items) return;
+        const BatchItem it = items[idx];
+        if ((it.kind_rg & kItemKindMask) != kItemEncodeMma) {  // another CTA took the tile seen at the head
+            *held = idx;
+            return;
+        }
+        const BatchJob& Jn = jobs[it.job];
         mma::tensormap_acquire(&Jn.src_map);
-        next = batch_mma_tile_of(Jn, nit);
-        return true;
-    };
-    const bool ok = mma::run_tile<kBatchInStages>(P, T, claim_next);  // ends with a CTA barrier
+        nxt.job = it.job;
+        nxt.band = it.b >> 16;
+        nxt.T = batch_mma_tile_of(Jn, it);
+    });  // ends with a CTA barrier
     if (threadIdx.x == 0) {
         mm[3] = P.tcount;
         mm[5] = P.gi;
@@ -1582,23 +1602,60 @@ __device__ __noinline__ void advance_rows(const BatchJob& J, uint32_t q, uint32_
     __syncthreads();
 }
 
+// Advance block q (its token is ours) over the bands that are ready in a row,
+// in one pass: one chain state load and store, one ring start and one
+// hand-over for all.  The bands are looked at by the lanes of a warp (a band
+// after another took ~12 us a pass).  Returns the band the chains stand at,
+// and in *moved whether they moved.
+constexpr uint32_t kChainBandsPerPass = 32;
+template <int UNITS, int AHEAD>
+__device__ uint32_t advance_ready(const BatchJob& J, uint32_t q, uint32_t ring, uint32_t* misc, bool* moved) {
+    const int tid = threadIdx.x;
+    const uint32_t nb = J.n_bands, Q = (J.R + kChainRows - 1) / kChainRows;
+    uint32_t* done = J.bstate;
+    uint32_t* next = done + nb;
+    if (tid < 32) {
+        const uint32_t b = *reinterpret_cast<volatile uint32_t*>(&next[q]) + tid;
+        const bool sid = *reinterpret_cast<volatile uint32_t*>(next + 2 * Q) != 0;
+        const bool ready = sid && b < nb && *reinterpret_cast<volatile uint32_t*>(&done[b]) == J.band_items[b];
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, ready);
+        if (tid == 0) {
+            misc[3] = b;
+            misc[2] = m == 0xFFFFFFFFu ? 32 : (uint32_t)__ffs(~m) - 1;
+        }
+    }
+    __syncthreads();
+    const uint32_t k = misc[2];
+    const uint32_t b = misc[3];
+    *moved = k != 0;
+    if (k) {
+        __threadfence();  // acquire: the bands' rows and the set id
+        if (tid < 4) misc[4 + tid] = __ldcg(reinterpret_cast<const uint32_t*>(J.set_id) + tid);
+        __syncthreads();
+        advance_rows<UNITS, AHEAD>(J, q, b, b + k - 1, ring, misc + 4);
+        if (tid == 0) {
+            __threadfence();
+            atomicExch(&next[q], b + k);
+        }
+    }
+    __syncthreads();
+    return b + k;
+}
+
 // Take block q's chain token if it is free and advance its rows over every
 // band that is ready, in order; after releasing the token, look once more
 // (a band that became ready while the token was held was left to us).  Each
 // pass either advances at least one band or returns, so this ends.  No CTA
 // waits for another: a busy token means its holder will see the new band.
-constexpr uint32_t kChainBandsPerPass = 16;
+// polls > 0: keep the token and look up to that many times, ~0.5 us apart, for
+// the next band, until the last one is done (the chain items).
 template <int UNITS, int AHEAD>
-__device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32_t* misc) {
+__device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32_t* misc, uint32_t polls = 0,
+                            const int* err = nullptr) {
     const int tid = threadIdx.x;
     const uint32_t nb = J.n_bands, Q = (J.R + kChainRows - 1) / kChainRows;
-    uint32_t* done = J.bstate;
-    uint32_t* next = done + nb;
+    uint32_t* next = J.bstate + nb;
     uint32_t* busy = next + Q;
-    uint32_t* sid_ready = busy + Q;
-    auto ready = [&](uint32_t b) {
-        return b < nb && atomicAdd(sid_ready, 0u) != 0 && atomicAdd(&done[b], 0u) == J.band_items[b];
-    };
     for (;;) {
         if (tid == 0) misc[2] = atomicCAS(&busy[q], 0u, 1u) == 0u ? 1u : 0u;
         __syncthreads();
@@ -1606,34 +1663,25 @@ __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32
         __syncthreads();
         if (!got) return;
         for (;;) {
-            // every band that is ready in a row goes in one pass: one chain
-            // state load and store, one ring start and one hand-over for all
-            if (tid == 0) {
-                const uint32_t b = atomicAdd(&next[q], 0u);
-                uint32_t k = 0;
-                while (k < kChainBandsPerPass && ready(b + k)) ++k;
-                misc[3] = b;
-                misc[2] = k;
-            }
+            bool moved;
+            const uint32_t at = advance_ready<UNITS, AHEAD>(J, q, ring, misc, &moved);
+            if (at >= nb) break;
+            if (moved) continue;
+            if (!polls) break;
+            --polls;
+            if (tid == 0) misc[2] = *reinterpret_cast<const volatile int*>(err) ? 1u : 0u;
             __syncthreads();
-            const uint32_t k = misc[2];
-            const uint32_t b = misc[3];
-            if (k && tid < 4) misc[4 + tid] = __ldcg(reinterpret_cast<const uint32_t*>(J.set_id) + tid);
+            const bool stop = misc[2] != 0;
             __syncthreads();
-            if (!k) break;
-            __threadfence();  // acquire: the bands' rows and the set id
-            advance_rows<UNITS, AHEAD>(J, q, b, b + k - 1, ring, misc + 4);
-            if (tid == 0) {
-                __threadfence();
-                atomicExch(&next[q], b + k);
-            }
-            __syncthreads();
+            if (stop) break;
+            __nanosleep(400);
         }
         if (tid == 0) {
             __threadfence();
             atomicExch(&busy[q], 0u);
             __threadfence();
-            misc[2] = ready(atomicAdd(&next[q], 0u)) ? 1u : 0u;
+            const uint32_t b = atomicAdd(&next[q], 0u);
+            misc[2] = b < nb && atomicAdd(&next[2 * Q], 0u) != 0 && atomicAdd(&J.bstate[b], 0u) == J.band_items[b] ? 1u : 0u;
         }
         __syncthreads();
         const bool again = misc[2] != 0;
@@ -1641,6 +1689,10 @@ __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32
         if (!again) return;
     }
 }
+
+// Polls of a chain item (~1 s); when they run out the block goes back to the
+// CTAs that complete its bands.
+constexpr uint32_t kChainPolls = 1u << 20;
 
 // All row blocks, starting with block `first` mod Q: the CTAs that complete
 // neighbouring bands start on different blocks, so that the blocks advance
@@ -1666,22 +1718,22 @@ __global__ void __launch_bounds__(kEncThreads, 1)
     const uint32_t chain_ring = smem_u32(smem + (MMA ? kBatchMmaChainOff : kBatchRingOff));
     uint8_t* tab_p = smem + (MMA ? kBatchMmaTabOff : kBatchTabOff);
     uint32_t(*T)[256] = reinterpret_cast<uint32_t(*)[256]>(tab_p);
-    // [0] item [1] last [2..3] chain tokens [4..7] set id [8] item claimed ahead by a tensor-core tile
+    // [0] item [1] last [2..3] chain tokens [4..7] set id [8..9], [11..12] job + 1 and band to advance [10] item held
     uint32_t* misc = reinterpret_cast<uint32_t*>(tab_p + 4 * 256 * 4);
     const uint32_t ring = smem_u32(ring_p);
     const int tid = threadIdx.x;
     // tensor-core launches: TMEM for the whole launch, barriers and scale
-    // factors set up once.  mma_misc: [0] TMEM address, [1] abort flag, [3..6]
+    // factors set up once.  mma_misc: [0] TMEM address, [1] abort flag, [3..7]
     // pipeline state.
     uint32_t* mma_misc = reinterpret_cast<uint32_t*>(smem + kBatchMmaBarsOff + mma::bar_bytes(kBatchInStages));
     const uint32_t mma_bars = smem_u32(smem + kBatchMmaBarsOff);
     if (tid == 0) {
-        misc[8] = kNoHeldItem;
+        misc[10] = kNoHeldItem;
         if (!MMA)
             for (int st = 0; st < kBatchEncStages; ++st) mbar_init(&bars[st], 1);
         if (MMA) {
             mma::init_bars<kBatchInStages>(mma_bars);
-            mma_misc[1] = mma_misc[3] = mma_misc[5] = mma_misc[6] = 0;
+            mma_misc[1] = mma_misc[3] = mma_misc[5] = mma_misc[6] = mma_misc[7] = 0;
         }
         fence_mbar_init();
     }
@@ -1698,13 +1750,10 @@ __global__ void __launch_bounds__(kEncThreads, 1)
     uint32_t phase = 0;
     for (;;) {
         if (tid == 0) {
-            // an item a tensor-core tile claimed ahead runs next whatever the
-            // error flag says: its first input copies may be in flight
-            const uint32_t h = misc[8];
-            misc[8] = kNoHeldItem;
-            misc[0] = h != kNoHeldItem ? h
-                      : *reinterpret_cast<volatile int*>(err) ? n_items
-                                                                : atomicAdd(&ctl[0], 1u);
+            // an item of another kind that a tile's helper warp popped
+            const uint32_t h = misc[10];
+            misc[10] = kNoHeldItem;
+            misc[0] = *reinterpret_cast<volatile int*>(err) ? n_items : h != kNoHeldItem ? h : atomicAdd(&ctl[0], 1u);
         }
         __syncthreads();
         const uint32_t idx = misc[0];
@@ -1754,6 +1803,12 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             }
             continue;
         }
+        if (kind == kItemChain) {
+            // this CTA keeps block it.a's chains until the last band (the
+            // other MD5 items' ring: no tensor-core stage is in flight here)
+            try_advance<kRingUnits, kRingAhead>(J, it.a, ring, misc, kChainPolls, err);
+            continue;
+        }
         if (kind == kItemPacket) {
             if (tid < 4) misc[4 + tid] = __ldcg(reinterpret_cast<const uint32_t*>(J.set_id) + tid);
             __syncthreads();
@@ -1761,20 +1816,54 @@ __global__ void __launch_bounds__(kEncThreads, 1)
             continue;
         }
         if (MMA && kind == kItemEncodeMma) {
-            const bool ok = batch_mma_tile(jobs, items, n_items, ctl, err, idx, misc + 8);
+            // a run of tiles: the one popped, then every one its helper warp
+            // claims ahead
+            MmaSlot* slots = reinterpret_cast<MmaSlot*>(smem + kBatchSlotOff);
+            if (tid == 0) {
+                MmaSlot& c = slots[mma_misc[3] & 1u];
+                c.T = batch_mma_tile_of(J, it);
+                c.job = it.job;
+                c.band = it.b >> 16;
+                misc[8] = misc[11] = 0;
+            }
+            // Earlier items stored to this shared memory through the generic proxy;
+            // the tiles' bulk and tensor copies write it through the async proxy.
+            // Order the two before any copy is issued.
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+            bool ok = true;
+            for (uint32_t n = 0;; ++n) {
+                uint32_t* adv = misc + (n & 1 ? 11 : 8);
+                ok = batch_mma_tile(jobs, items, n_items, ctl, err, n, adv, misc + 10);
+                if (!ok) break;
+                if (adv[0]) {  // the tile before this one completed its band
+                    const uint32_t aj = adv[0] - 1, ab = adv[1];
+                    __syncthreads();
+                    if (tid == 0) adv[0] = 0;
+                    __threadfence();  // acquire: the whole band is visible from here on
+                    advance_all<MMA>(jobs[aj], ab, chain_ring, misc);
+                    __syncthreads();
+                }
+                const MmaSlot& ran = slots[(mma_misc[3] & 1u) ^ 1u];
+                if (slots[mma_misc[3] & 1u].T.rows) continue;
+                const BatchJob& Jr = jobs[ran.job];
+                if (!Jr.n_bands) break;
+                if (tid == 0) {
+                    __threadfence();  // release this tile's rows before counting it
+                    misc[1] = (atomicAdd(&Jr.bstate[ran.band], 1u) + 1 == Jr.band_items[ran.band]) ? 1u : 0u;
+                }
+                __syncthreads();
+                if (misc[1]) {
+                    __threadfence();  // acquire: the whole band is visible from here on
+                    advance_all<MMA>(Jr, ran.band, chain_ring, misc);
+                }
+                break;
+            }
             if (!ok) {
                 if (tid == 0) atomicOr(err, 1);
                 break;
             }
-            if (!J.n_bands) continue;
-            const uint32_t band = it.b >> 16;
-            __threadfence();  // release this tile's rows before counting it
             __syncthreads();
-            if (tid == 0) misc[1] = (atomicAdd(&J.bstate[band], 1u) + 1 == J.band_items[band]) ? 1u : 0u;
-            __syncthreads();
-            if (!misc[1]) continue;
-            __threadfence();  // acquire: the whole band is visible from here on
-            advance_all<MMA>(J, band, chain_ring, misc);
             continue;
         }
         if (!MMA && kind == kItemEncode) {

@@ -54,7 +54,8 @@ constexpr int kInStages = 6;  // 4 K-steps each: the MMAs of 20 in reserve, 4,20
 // shared memory layout (bytes): the ring, barriers, misc
 constexpr uint32_t kOffBars = kInStages * kInStageBytes;
 constexpr uint32_t kOffMisc = kOffBars + bar_bytes(kInStages);
-constexpr uint32_t kSmemBytes = kOffMisc + 32;
+constexpr uint32_t kOffNext = kOffMisc + 32;  // the next tile
+constexpr uint32_t kSmemBytes = kOffNext + sizeof(Tile);
 static_assert(kSmemBytes > 116 * 1024, "one CTA per SM: TMEM is allocated whole");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
 static_assert(mma_image_steps(1027) == image_steps(1027) && mma_image_steps(32) == image_steps(32) &&
@@ -135,7 +136,7 @@ __device__ __forceinline__ Tile tile_of(const EncodeArgs& A, uint32_t at) {
 }
 
 // One tile, out of line with its pipeline state in shared memory (misc[0]
-// TMEM base, [1] abort flag, [2..4] state), as in the batch kernel: inlined
+// TMEM base, [1] abort flag, [2..5] state), as in the batch kernel: inlined
 // into the tile loop the compiler keeps the MMA warp's operands out of uniform
 // registers, and a K-step takes 300 cycles.
 __device__ __noinline__ bool encode_mma_tile(const EncodeArgs& A, uint32_t tile, uint32_t next) {
@@ -149,11 +150,17 @@ __device__ __noinline__ bool encode_mma_tile(const EncodeArgs& A, uint32_t tile,
     P.gi = misc[2];
     P.tcount = misc[3];
     P.pre = misc[4];
+    P.issued = misc + 5;
+    Tile* const slot = reinterpret_cast<Tile*>(smem + kOffNext);
+    P.next = slot;
     const Tile T = tile_of(A, tile);
-    const bool ok = run_tile<kInStages>(P, T, [&](Tile& n) {
-        if (next >= A.row_tiles * A.sym_tiles) return false;
-        n = tile_of(A, next);
-        return true;
+    const bool ok = run_tile<kInStages>(P, T, [&] {
+        if ((threadIdx.x & 31) == 0) {
+            if (next < A.row_tiles * A.sym_tiles)
+                *slot = tile_of(A, next);
+            else
+                slot->rows = 0;
+        }
     });  // ends with a CTA barrier
     if (threadIdx.x == 0) {
         misc[2] = P.gi;
@@ -171,7 +178,7 @@ __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_co
     uint32_t* misc = reinterpret_cast<uint32_t*>(smem + kOffMisc);
     if (tid == 0) {
         init_bars<kInStages>(smem_addr(smem + kOffBars));
-        for (int i = 1; i < 5; ++i) misc[i] = 0;
+        for (int i = 1; i < 6; ++i) misc[i] = 0;
     }
     if (warp == 1) tmem_alloc(smem_addr(misc));  // the whole of TMEM: two accumulators, A stages, scale factors
     tc_fence_before();

@@ -20,8 +20,9 @@
 // stored by the builders, read by the MMAs) a 4-slice K-step of two N = 240
 // MMAs took 430 cycles where the MMAs alone take 240; with A in TMEM a K-step
 // of two N = 208 MMAs takes 230 where they alone take 208 (538 MB, 200 rows:
-// 5.33 -> 4.00 ms with the tile's start and epilogue).  13 rows: two accumulators of 208 columns,
-// 8 for the scale factors and four A stages of 16 fit TMEM's 512.
+// 5.33 -> 3.93 ms with the tile's start and epilogue; under a steady load the
+// clock falls to 1.83-1.95 GHz at the 1,000 W limit).  13 rows: two accumulators of 208 columns,
+// 8 for the scale factors and four K-steps of A of 16 fit TMEM's 512.
 //
 // Shared memory (from `ring`, 1024-aligned): input stages of 34,816 B, each
 // covering 4 K-steps (16 input slices): their coefficient rows (4 x 512 B a
@@ -45,15 +46,15 @@ constexpr uint32_t kSrcSliceBytes = kTileSyms * 2;
 constexpr uint32_t kInBBytes = kInSteps * kMaxRows * kRowStepBytes;  // 26,624 B at most
 constexpr uint32_t kInSrcBytes = kInSlices * kSrcSliceBytes;         // 8 KiB
 constexpr uint32_t kInStageBytes = kInBBytes + kInSrcBytes;
-constexpr uint32_t kAStages = kInSteps;               // K-steps of A in TMEM, one per K-step of an input stage
+constexpr uint32_t kAStages = 2;                      // halves of an input stage (2 K-steps each) in TMEM
 constexpr uint32_t kAccCol1 = 16 * kMaxRows;          // TMEM column of the second accumulator
 constexpr uint32_t kSfCol = 2 * kAccCol1;             // scale factors (all 1.0, read as both operands')
-constexpr uint32_t kACol = kSfCol + 8;                // A stages, 16 columns each: 8 a M = 128 half
+constexpr uint32_t kACol = kSfCol + 8;                // A, 16 columns a K-step: 8 a M = 128 half
 constexpr uint32_t kEpilogueWarps = 12;               // three to a TMEM lane quadrant
-static_assert(kACol + 16 * kAStages <= 512, "TMEM columns");
+static_assert(kACol + 16 * kInSteps <= 512, "TMEM columns");
 static_assert(kInStageBytes % 1024 == 0 && kInBBytes % 128 == 0, "tensor copies land 128-byte aligned");
-// barriers: in_full/in_empty per input stage, a_full/a_empty per A stage, acc_full, acc_empty, drain
-__host__ __device__ constexpr uint32_t bar_bytes(int in_stages) { return (2 * in_stages + 2 * (int)kAStages + 3) * 8; }
+// barriers: in_full/in_empty per input stage, a_full/a_empty per A stage, acc_full, acc_empty, next_full, drain
+__host__ __device__ constexpr uint32_t bar_bytes(int in_stages) { return (2 * in_stages + 2 * (int)kAStages + 4) * 8; }
 
 // The coefficient image in global memory: for row tile rt (`rows` recovery
 // rows) and K-step k (slices 4k .. 4k+3), rows x 512 B laid out as in shared
@@ -151,8 +152,8 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
         "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
         "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Two runs of 16 columns of this warp's 32 lanes.
 __device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, uint32_t (&v)[32]) {
     asm volatile(
@@ -176,6 +177,18 @@ constexpr uint32_t kPairs = 0x22200200u;  // byte g = e2m1 pair of bits (g & 1, 
 __device__ __forceinline__ uint2 spread16(uint32_t x) {
     return make_uint2(__byte_perm(kPairs, 0u, x & 0x3333u), __byte_perm(kPairs, 0u, (x >> 2) & 0x3333u));
 }
+// 4 slices' words (symbols 2m low, 2m+1 high) -> 8 e2m1 words of either half
+__device__ __forceinline__ void spread4(const uint32_t* x, uint32_t (&v)[16]) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        // spread16 of both symbols: pairs (4q, 4q+1) from x & 0x3333, pairs (4q+2, 4q+3) from (x >> 2) & 0x3333
+        const uint32_t e = x[s] & 0x33333333u, o = (x[s] >> 2) & 0x33333333u;
+        v[2 * s] = __byte_perm(kPairs, 0u, e & 0xFFFFu);
+        v[2 * s + 1] = __byte_perm(kPairs, 0u, o & 0xFFFFu);
+        v[8 + 2 * s] = __byte_perm(kPairs, 0u, e >> 16);
+        v[8 + 2 * s + 1] = __byte_perm(kPairs, 0u, o >> 16);
+    }
+}
 __device__ __forceinline__ uint32_t lds_b32(uint32_t addr) {
     uint32_t v;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -185,10 +198,11 @@ __device__ __forceinline__ uint32_t lds_b32(uint32_t addr) {
 // Barrier block of a pipeline with IN input stages.
 template <int IN>
 struct Bars {
-    uint32_t in_full, in_empty, a_full, a_empty, acc_full, acc_empty, drain;
+    uint32_t in_full, in_empty, a_full, a_empty, acc_full, acc_empty, next_full, drain;
     __device__ explicit Bars(uint32_t b)
         : in_full(b), in_empty(b + 8 * IN), a_full(b + 16 * IN), a_empty(b + 16 * IN + 8 * kAStages),
-          acc_full(b + 16 * IN + 16 * kAStages), acc_empty(acc_full + 8), drain(acc_full + 16) {}
+          acc_full(b + 16 * IN + 16 * kAStages), acc_empty(acc_full + 8), next_full(acc_full + 16),
+          drain(acc_full + 24) {}
 };
 // One thread.  An input stage is released by the MMA warp's commit after its
 // last K-step (the builders have read it by then: the MMAs waited for their A).
@@ -200,11 +214,12 @@ __device__ __forceinline__ void init_bars(uint32_t b) {
         bar_init(B.in_empty + 8 * i, 1);
     }
     for (uint32_t i = 0; i < kAStages; ++i) {
-        bar_init(B.a_full + 8 * i, 4);  // one warp of each lane quadrant
+        bar_init(B.a_full + 8 * i, 8);  // the builder warps
         bar_init(B.a_empty + 8 * i, 1);
     }
     bar_init(B.acc_full, 1);
     bar_init(B.acc_empty, kEpilogueWarps);
+    bar_init(B.next_full, 1);
     bar_init(B.drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
@@ -248,6 +263,8 @@ struct Pipe {
     volatile uint32_t* abort_flag;
     uint32_t gi, tcount;
     uint32_t pre;  // input stages of the coming tile already issued by the previous call
+    volatile uint32_t* issued;  // shared: input stages issued so far, for the helper warp
+    const Tile* next;           // shared: the tile that follows, written by the helper warp (rows 0: none)
 };
 
 // The lane that issues a warp's asynchronous instructions.
@@ -271,18 +288,17 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // All threads of the CTA (16 warps) call this.  Warp 0 streams the inputs,
-// warp 1 issues the MMAs, warps 4..11 build A (warp w its lane quadrant w % 4
+// warp 1 issues the MMAs, warp 2 finds the next tile, warps 4..11 build A (warp w its lane quadrant w % 4
 // of every other K-step), and warps 4..15 run the epilogue (every third row of
 // their quadrant).  Returns false (uniformly, after a CTA barrier) when a
 // bounded wait gave up; copies and MMAs in flight have then landed.
-// next_fn: called once, by one thread of warp 0 alone, after the warp has
-// issued this tile's last input stage; it fills in the tile this CTA runs next
-// and returns whether there is one.  The warp then issues that tile's first
-// input stages while this tile's last K-steps and epilogue run, so the next
-// tile starts without a copy round trip.  Only warp 0's P.pre counts (the
-// stages it issued ahead); the next call must be for that same tile.  When any
-// role's wait gives up, warp 0 waits for every copy it issued, the next tile's
-// included, before this returns.
+// helper: run by warp 2 when warp 0 has kHelperLead stages of this tile left to
+// issue; it writes the tile this CTA runs next to *P.next.  Warp 0 then issues
+// that tile's first input stages while this tile's last K-steps and epilogue
+// run, so the next tile starts without a copy round trip.  Only warp 0's P.pre
+// counts (the stages it issued ahead); the next call must be for that same
+// tile.  When any role's wait gives up, warp 0 waits for every copy it issued,
+// the next tile's included, before this returns.
 //
 // Every role runs whole warps on values the compiler knows to be the same in
 // every lane (uni), with only the asynchronous instructions under the elected
@@ -295,8 +311,9 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // own: K-steps past the tile's last multiply the builders' zeros, and a role
 // whose wait gave up runs on to its end (every later wait returns at once; the
 // tile is dropped, its memory is the CTA's own and nothing is stored).
-template <int IN, class NextFn>
-__device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, NextFn&& next_fn) {
+constexpr uint32_t kHelperLead = 4;  // with 5 more in flight, about 8,000 cycles before the tile's end
+template <int IN, class Helper>
+__device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper) {
     const uint32_t warp = uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const Bars<IN> B(uni(P.bars));
     const uint32_t in0 = uni(P.ring), tmem = uni(P.tmem), rows = uni(T.rows);
@@ -332,6 +349,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, NextFn&& next_f
                     bar_expect_tx(full, bytes + kInSrcBytes);
                     tma_1d(dst, a, bytes, full);
                     tma_2d(dst + kInBBytes, reinterpret_cast<const void*>(map), (int32_t)x, (int32_t)sa, full);
+                    *P.issued = gi + 1;
                 }
                 if (++st == IN) {
                     st = 0;
@@ -340,19 +358,13 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, NextFn&& next_f
             }
         };
         issue(uni((uint64_t)(uintptr_t)T.src_map), uni((uint64_t)(uintptr_t)T.aimg), n0, s0, rows, pre, NI);
+        if (ok) ok = warp_wait(B.next_full, tc & 1u, P.abort_flag);
         if (ok) {
-            Tile U;
-            uint32_t want = 0;
-            if (lead && next_fn(U) && !(U.n0 & 7u) && !(U.s0 % kInSlices) && U.rows <= kMaxRows) {
-                const uint32_t ni = (U.sn + kInSlices - 1) / kInSlices;
-                want = ni < (uint32_t)IN ? ni : (uint32_t)IN;
-            }
-            want = __shfl_sync(0xFFFFFFFFu, want, leader);
-            if (want) {
-                auto from = [&](uint64_t v) { return (uint64_t)__shfl_sync(0xFFFFFFFFu, (unsigned long long)v, leader); };
-                issue(from((uint64_t)(uintptr_t)U.src_map), from((uint64_t)(uintptr_t)U.aimg), (uint32_t)from(U.n0),
-                      (uint32_t)from(U.s0), (uint32_t)from(U.rows), 0, want);
-            }
+            const uint32_t n_rows = uni(P.next->rows), nx = uni(P.next->n0), ns = uni(P.next->s0);
+            const uint32_t ni = (uni(P.next->sn) + kInSlices - 1) / kInSlices;
+            if (n_rows && n_rows <= kMaxRows && !(nx & 7u) && !(ns % kInSlices))
+                issue(uni((uint64_t)(uintptr_t)P.next->src_map), uni((uint64_t)(uintptr_t)P.next->aimg), nx, ns, n_rows, 0,
+                      ni < (uint32_t)IN ? ni : (uint32_t)IN);
         }
         if (!ok) {  // copies issued but maybe not consumed land before the stages are reused
             for (uint32_t q = gi > gi0 + IN ? gi - IN : gi0; q < gi; ++q)
@@ -371,16 +383,19 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, NextFn&& next_f
             ok &= warp_wait(B.in_full + 8 * si, pi, P.abort_flag);
             const uint32_t b0 = in0 + si * kInStageBytes;
 #pragma unroll
-            for (uint32_t ks = 0; ks < kInSteps; ++ks) {
-                ok &= warp_wait(B.a_full + 8 * ks, pa, P.abort_flag);
+            for (uint32_t u = 0; u < kAStages; ++u) {
+                ok &= warp_wait(B.a_full + 8 * u, pa, P.abort_flag);
                 tc_fence_after();
-                const uint64_t bdesc = smem_desc(b0 + ks * step, 128, 256);
-                const uint32_t a = tmem + kACol + 16 * ks;
                 if (lead) {
-                    mma_mxf4(tmem, a, bdesc, id, sf, k + ks);
-                    mma_mxf4(tmem + kAccCol1, a + 8, bdesc, id, sf, k + ks);
-                    mma_commit(B.a_empty + 8 * ks);
-                    if (ks == kInSteps - 1) mma_commit(B.in_empty + 8 * si);
+#pragma unroll
+                    for (uint32_t ks = 2 * u; ks < 2 * u + 2; ++ks) {
+                        const uint64_t bdesc = smem_desc(b0 + ks * step, 128, 256);
+                        const uint32_t a = tmem + kACol + 16 * ks;
+                        mma_mxf4(tmem, a, bdesc, id, sf, k + ks);
+                        mma_mxf4(tmem + kAccCol1, a + 8, bdesc, id, sf, k + ks);
+                    }
+                    mma_commit(B.a_empty + 8 * u);
+                    if (u == kAStages - 1) mma_commit(B.in_empty + 8 * si);
                 }
             }
             pa ^= 1u;
@@ -392,6 +407,12 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, NextFn&& next_f
         if (lead) mma_commit(B.acc_full);
         // every MMA issued completes before its stages or TMEM are reused
         if (!ok) bar_drain(B.acc_full, tc & 1u);
+    } else if (warp == 2) {
+        const uint32_t at = NI > kHelperLead ? gi0 + NI - kHelperLead : gi0;
+        for (uint32_t it = 0; it < (1u << 20) && (int32_t)(*P.issued - at) < 0 && !*P.abort_flag; ++it) __nanosleep(64);
+        helper();
+        __syncwarp();
+        if (lane == 0) bar_arrive(B.next_full);
     } else if (warp >= 4) {
         const uint32_t q = warp & 3u, j = (warp >> 2) - 1u;
         const uint32_t lanes = tmem + ((32 * q) << 16);
@@ -408,26 +429,24 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, NextFn&& next_f
                     x[s] = lds_b32(a + at * kSrcSliceBytes);
                     if (at >= left) x[s] = 0;
                 }
-#pragma unroll
-                for (uint32_t u = 0; u < 2; ++u) {
-                    const uint32_t ks = 2 * u + j;
-                    uint32_t v[16];
-#pragma unroll
-                    for (uint32_t s = 0; s < kKSlices; ++s) {
-                        // spread16 of both halves: pairs (4q, 4q+1) from x & 0x3333, pairs (4q+2, 4q+3) from (x >> 2) & 0x3333
-                        const uint32_t e = x[u * kKSlices + s] & 0x33333333u, o = (x[u * kKSlices + s] >> 2) & 0x33333333u;
-                        v[2 * s] = __byte_perm(kPairs, 0u, e & 0xFFFFu);
-                        v[2 * s + 1] = __byte_perm(kPairs, 0u, o & 0xFFFFu);
-                        v[8 + 2 * s] = __byte_perm(kPairs, 0u, e >> 16);
-                        v[8 + 2 * s + 1] = __byte_perm(kPairs, 0u, o >> 16);
-                    }
-                    ok &= warp_wait(B.a_empty + 8 * ks, pa, P.abort_flag);
-                    tc_fence_after();
-                    tmem_st16(lanes + kACol + 16 * ks, v);
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(B.a_full + 8 * ks);
-                }
+// the second K-step is spread while the first is stored
+                uint32_t v[16], w[16];
+                spread4(x, v);
+                ok &= warp_wait(B.a_empty + 8 * 0, pa, P.abort_flag);
+                tc_fence_after();
+                tmem_st16(lanes + kACol + 16 * j, v);
+                spread4(x + kKSlices, w);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(B.a_full + 8 * 0);
+                ok &= warp_wait(B.a_empty + 8 * 1, pa, P.abort_flag);
+                tc_fence_after();
+                tmem_st16(lanes + kACol + 16 * (j + 2), w);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(B.a_full + 8 * 1);
                 pa ^= 1u;
                 if (++si == IN) {
                     si = 0;
