@@ -859,32 +859,39 @@ __device__ void md5_range_ring(uint32_t st[4], const uint32_t* pre, const uint8_
         // slots are stepped as 32-bit counters: no remainder by the (non-
         // power-of-two) ring size between one compress and the next
         uint32_t f_slot = (b0 + 1 + HI + AHEAD) % UNITS;
-        for (uint32_t blk = b0; blk < end_max; ++blk) {
-            uint32_t m[16];
-            if (VEC) {
+        // Lanes of different lengths (!SAME, or different shifts) run in legs that
+        // end where some lanes' streams end; those set their state aside and
+        // go on over stale words.  Holding the state back block by block put
+        // four selects on every lane's chain (0.465 us a block against 0.446, 400 files
+        // of up to 1 MiB in one job).
+        uint32_t kept[4] = {st[0], st[1], st[2], st[3]};
+        uint32_t leg = SAME && VEC ? end_max : b0;
+        for (uint32_t blk = b0; blk < end_max;) {
+            if (!(SAME && VEC)) leg = __reduce_min_sync(0xFFFFFFFFu, end > blk ? end : 0xFFFFFFFFu);
+            for (; blk < leg; ++blk) {
+                uint32_t m[16];
+                if (VEC) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) m[i] = q[SH + i];
-            } else {
-                uint32_t h[17];
+                    for (int i = 0; i < 16; ++i) m[i] = q[SH + i];
+                } else {
+                    uint32_t h[17];
 #pragma unroll
-                for (int i = 0; i < 17; ++i) h[i] = sh & 2 ? q[i + 2] : q[i];
+                    for (int i = 0; i < 17; ++i) h[i] = sh & 2 ? q[i + 2] : q[i];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) m[i] = sh & 1 ? h[i + 1] : h[i];
-            }
-            cp_async_wait<AHEAD - 1>();  // unit blk + 1 + HI
-            __syncwarp();                // ... of every lane; and every lane has read block blk
-            fetch(blk + 1 + HI + AHEAD, f_slot);
-            f_slot = f_slot + 1 == (uint32_t)UNITS ? 0u : f_slot + 1;
-            read();  // block blk + 1 (past a stream's end: stale words, not used)
-            if (SAME && VEC) {
+                    for (int i = 0; i < 16; ++i) m[i] = sh & 1 ? h[i + 1] : h[i];
+                }
+                cp_async_wait<AHEAD - 1>();  // unit blk + 1 + HI
+                __syncwarp();                // ... of every lane; and every lane has read block blk
+                fetch(blk + 1 + HI + AHEAD, f_slot);
+                f_slot = f_slot + 1 == (uint32_t)UNITS ? 0u : f_slot + 1;
+                read();  // block blk + 1 (past a stream's end: stale words, not used)
                 md5_compress(st, m);
-            } else {  // selected, not branched around: the copies above overlap the steps
-                uint32_t t[4] = {st[0], st[1], st[2], st[3]};
-                md5_compress(t, m);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) st[i] = blk < end ? t[i] : st[i];
             }
+            if (!(SAME && VEC) && end == leg)
+                for (int i = 0; i < 4; ++i) kept[i] = st[i];
         }
+        if (!(SAME && VEC))
+            for (int i = 0; i < 4; ++i) st[i] = kept[i];
         cp_async_wait<0>();
         __syncwarp();
         if (b < end) b = end;
