@@ -49,6 +49,7 @@ namespace {
 
 using namespace mma;
 constexpr int kThreads = 512;
+constexpr int kImageThreads = 224;  // a K-step of 13 rows has 416 units, of 7 224
 constexpr int kInStages = 6;  // 4 K-steps each: the MMAs of 20 in reserve, 4,200 cycles
 
 // shared memory layout (bytes): the ring, barriers, misc
@@ -64,42 +65,44 @@ static_assert(mma_image_steps(1027) == image_steps(1027) && mma_image_steps(32) 
 
 }  // namespace
 
-// The coefficient image of one job (layout: image_steps in p2g_mma_tile.cuh),
-// one 16-byte K half of a B row per step of the loop: rows of recovery row
-// r >= R and slices s >= S are 0.  c(r,s) = base_s ^ (first_exp + r) =
-// 2^(logbase_s * (first_exp + r) mod 65535) (RsEncoder::coefficient,
-// src/reedsolomon.rs:56-60; gf_pow src/galois.rs:74-87).
+// The coefficient image of one job (layout: image_steps in p2g_mma_tile.cuh):
+// K-steps b0, b0 + step, .. of its row tiles, one CTA a K-step at a time, a
+// thread per 16-byte K half of a B row, so that the only divisions are one a
+// K-step.  Rows of recovery row r >= R and slices s >= S are 0.  c(r,s) =
+// base_s ^ (first_exp + r) = 2^(logbase_s * (first_exp + r) mod 65535)
+// (RsEncoder::coefficient, src/reedsolomon.rs:56-60; gf_pow
+// src/galois.rs:74-87).  Bound by the writes: 512 MB (2,000 rows x 2,000
+// slices) took 181 us with an index division a unit, 136 now.
 __device__ __forceinline__ void fill_a_image(uint8_t* __restrict__ aimg, uint32_t S, uint32_t R, uint32_t first_exp,
-                                             const uint16_t* __restrict__ logbase, uint64_t i0, uint64_t step) {
+                                             const uint16_t* __restrict__ logbase, uint32_t b0, uint32_t step) {
     const uint32_t rows = mma_rows(R), ksteps = image_steps(S), n_row = (R + rows - 1) / rows;
     const uint32_t units = rows * (kRowStepBytes / 16);  // 16-byte units of a K-step
-    const uint64_t total = (uint64_t)n_row * ksteps * units;
-    for (uint64_t i = i0; i < total; i += step) {
-        const uint32_t c = (uint32_t)(i % units);  // byte c*16 = grp*256 + kh*128 + m8*16
-        const uint64_t q = i / units;
-        const uint32_t k = (uint32_t)(q % ksteps), rt = (uint32_t)(q / ksteps);
-        const uint32_t n = (c >> 4) * 8 + (c & 7u), kh = (c >> 3) & 1u;
-        const uint32_t r = rt * rows + (n >> 4), s0 = k * kKSlices + 2 * kh;
-        const uint32_t e = (first_exp + r) % kFieldLimit, d = d_dual_log[n & 15u];
-        auto bits = [&](uint32_t s) -> uint32_t {  // row n & 15 of M_c(r,s)
-            if (r >= R || s >= S) return 0u;
-            uint32_t x = (uint32_t)logbase[s] * e;  // < 2^32
-            x = (x & 0xFFFFu) + (x >> 16);
-            x = (x & 0xFFFFu) + (x >> 16);
-            if (x >= kFieldLimit) x -= kFieldLimit;
-            x += d;
-            if (x >= kFieldLimit) x -= kFieldLimit;
-            return d_trace_bits[x];
-        };
-        const uint2 v0 = spread16(bits(s0)), v1 = spread16(bits(s0 + 1));
-        reinterpret_cast<uint4*>(aimg)[i] = make_uint4(v0.x, v0.y, v1.x, v1.y);
+    for (uint32_t q = b0; q < n_row * ksteps; q += step) {  // < 2^13 row tiles x 2^13 K-steps
+        const uint32_t rt = q / ksteps, k = q - rt * ksteps;
+        uint4* out = reinterpret_cast<uint4*>(aimg) + (size_t)q * units;
+        for (uint32_t c = threadIdx.x; c < units; c += blockDim.x) {  // byte c*16 = grp*256 + kh*128 + m8*16
+            const uint32_t n = (c >> 4) * 8 + (c & 7u), kh = (c >> 3) & 1u;
+            const uint32_t r = rt * rows + (n >> 4), s0 = k * kKSlices + 2 * kh;
+            const uint32_t e = (first_exp + r) % kFieldLimit, d = d_dual_log[n & 15u];
+            auto bits = [&](uint32_t s) -> uint32_t {  // row n & 15 of M_c(r,s)
+                if (r >= R || s >= S) return 0u;
+                uint32_t x = (uint32_t)logbase[s] * e;  // < 2^32
+                x = (x & 0xFFFFu) + (x >> 16);
+                x = (x & 0xFFFFu) + (x >> 16);
+                if (x >= kFieldLimit) x -= kFieldLimit;
+                x += d;
+                if (x >= kFieldLimit) x -= kFieldLimit;
+                return d_trace_bits[x];
+            };
+            const uint2 v0 = spread16(bits(s0)), v1 = spread16(bits(s0 + 1));
+            out[c] = make_uint4(v0.x, v0.y, v1.x, v1.y);
+        }
     }
 }
 
 __global__ void a_image_kernel(uint8_t* __restrict__ aimg, const uint16_t* __restrict__ logbase, uint32_t S, uint32_t R,
                                uint32_t first_exp) {
-    fill_a_image(aimg, S, R, first_exp, logbase, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
-                 (uint64_t)gridDim.x * blockDim.x);
+    fill_a_image(aimg, S, R, first_exp, logbase, blockIdx.x, gridDim.x);
 }
 
 struct EncodeArgs {
@@ -279,8 +282,7 @@ cudaError_t mma_prepare() {
 __global__ void a_image_batch_kernel(const BatchJob* __restrict__ jobs, const uint16_t* __restrict__ logbase) {
     const BatchJob& J = jobs[blockIdx.y];
     if (!J.mma || !J.R || !J.aimg) return;
-    fill_a_image(J.aimg, J.S, J.R, J.first_exp, logbase, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
-                 (uint64_t)gridDim.x * blockDim.x);
+    fill_a_image(J.aimg, J.S, J.R, J.first_exp, logbase, blockIdx.x, gridDim.x);
 }
 
 cudaError_t launch_a_image_batch(const BatchJob* jobs, uint32_t n_jobs, uint64_t max_bytes, cudaStream_t st) {
@@ -289,9 +291,9 @@ cudaError_t launch_a_image_batch(const BatchJob* jobs, uint32_t n_jobs, uint64_t
     if (e != cudaSuccess) return e;
     const uint16_t *antilog = nullptr, *logbase = nullptr;
     if ((e = gf_device_tables(&antilog, &logbase)) != cudaSuccess) return e;
-    const uint64_t want = (max_bytes / 16 + 255) / 256;
+    const uint64_t want = max_bytes / kRowStepBytes;  // K-steps of the largest image, at most
     const unsigned bx = (unsigned)std::min<uint64_t>(want, (uint64_t)device_sm_count() * 8);
-    a_image_batch_kernel<<<dim3(bx, n_jobs), 256, 0, st>>>(jobs, logbase);
+    a_image_batch_kernel<<<dim3(bx, n_jobs), kImageThreads, 0, st>>>(jobs, logbase);
     add_launches(1);
     return cudaGetLastError();
 }
@@ -350,10 +352,9 @@ cudaError_t launch_encode_mma(const uint8_t* src, uint64_t src_stride, uint32_t 
     A.rows = mma_rows(R);
     A.row_tiles = mma_row_tiles(R);
     A.sym_tiles = (Np + kTileSyms - 1) / kTileSyms;
-    const uint64_t chunks = mma_aimg_bytes(S, R) / 16;
     const int sms = device_sm_count();
-    const unsigned cb = (unsigned)std::min<uint64_t>((chunks + 255) / 256, (uint64_t)sms * 8);
-    a_image_kernel<<<cb, 256, 0, st>>>(aimg, logbase, S, R, first_exp);
+    const unsigned cb = (unsigned)std::min<uint64_t>((uint64_t)A.row_tiles * image_steps(S), (uint64_t)sms * 8);
+    a_image_kernel<<<cb, kImageThreads, 0, st>>>(aimg, logbase, S, R, first_exp);
     add_launches(1);
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)A.row_tiles * A.sym_tiles, (uint64_t)sms);
     encode_mma_kernel<<<grid, kThreads, kSmemBytes, st>>>(A, err);
