@@ -425,6 +425,29 @@ double encode_cost_ms(uint64_t slice, uint32_t S, uint32_t R, bool mma) {
 bool prefer_mma(uint64_t slice, uint32_t S, uint32_t R) {
     return R && S && encode_cost_ms(slice, S, R, true) < encode_cost_ms(slice, S, R, false);
 }
+// An encode alone on the GPU ends with its last wave, not with its work: the
+// tiles of either kernel in whole waves of SMs, each tile's steps and fixed
+// part, the launches and, on the tensor cores, the coefficient image at ~3
+// TB/s.  Against the two kernels timed over 266 shapes (slices 4 KiB..1 MiB, 4
+// to 1,024 of them, 1 to 200 rows) this picks the faster or one within 1 %, but
+// for two within 14 %: 4 KiB x 1,024 x 1 takes 773 us on the lookup kernel and
+// 39 on the tensor cores, 256 KiB x 64 x 32 72 and 54, 1 MiB x 16 x 100 179
+// and 303.
+bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R) {
+    if (!R || !S) return false;
+    const uint32_t Np = (uint32_t)(round_up(slice, 16) / 2), sms = (uint32_t)kMaxCtas;
+    const uint32_t rows = mma_rows(R), RT = mma_row_tiles(R);
+    const uint64_t tiles = (uint64_t)((Np + kMmaTileSymbols - 1) / kMmaTileSymbols) * RT;
+    const double mma = 8.0 + (double)((tiles + sms - 1) / sms) *
+                                 (mma_image_steps(S) * std::max(212.0, 17.6 * rows) + 3600.0) / 1900.0 +
+                       (double)RT * rows * S * 128.0 / 3.0e6;
+    const uint32_t RG = (R + kRowsPerGroup - 1) / kRowsPerGroup, fold = tail_fold(R);
+    uint32_t ts = 0, n = 0;
+    choose_tiles(Np, RG, sms, &ts, &n, fold);
+    const uint64_t ctas = (uint64_t)n * (RG - 1) + (n + fold - 1) / fold;
+    const double lut = 6.0 + (double)((ctas + sms - 1) / sms) * S * (ts + kBuildCost) / (kEncRate / 1000.0);
+    return mma < lut;
+}
 double est_encode_item_ms(uint32_t slices, uint32_t syms) {
     return (double)slices * (round_up(syms, 8) + kBuildCost) / kEncRate + kItemMs;
 }

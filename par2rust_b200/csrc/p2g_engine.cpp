@@ -218,15 +218,33 @@ static p2g_status join_into(Context& c, cudaStream_t caller) {
 // Which encode kernel runs a job: the shared-memory lookup kernel or the
 // tensor-core bit-sliced one.  P2G_ENCODE_LUT / P2G_ENCODE_TENSOR (or
 // P2G_ENCODE_VARIANT=lut|tensor) force one; otherwise the planner's cost
-// model picks by shape (prefer_mma).
-static bool use_tensor_encode(uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size) {
+// model picks by shape (prefer_mma, or prefer_mma_alone for an encode call).
+static bool use_tensor_encode(uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size, bool alone = false) {
     if (flags & P2G_ENCODE_TENSOR) return true;
     if (flags & P2G_ENCODE_LUT) return false;
     if (const char* e = getenv("P2G_ENCODE_VARIANT")) {
         if (!strcmp(e, "tensor")) return true;
         if (!strcmp(e, "lut")) return false;
     }
-    return prefer_mma(slice_size, S, R);
+    return alone ? prefer_mma_alone(slice_size, S, R) : prefer_mma(slice_size, S, R);
+}
+
+// The kernel of one encode call, with room for its coefficient image in
+// *use_tensor's case.  Where the rule alone picked the tensor cores and the
+// image does not fit the device, the lookup kernel (whose bases are a quarter
+// of it) runs instead.
+static p2g_status choose_encode(Context& c, uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size,
+                                bool* use_tensor) {
+    *use_tensor = use_tensor_encode(flags, S, R, slice_size, true);
+    if (!*use_tensor) return P2G_OK;
+    const cudaError_t e = c.aimg.ensure(mma_aimg_bytes(S, R));
+    if (e == cudaSuccess) return P2G_OK;
+    if (e == cudaErrorMemoryAllocation && !(flags & P2G_ENCODE_TENSOR) && !prefer_mma(slice_size, S, R)) {
+        cudaGetLastError();
+        *use_tensor = false;
+        return P2G_OK;
+    }
+    return cuda_fail(e, "coefficient image");
 }
 
 static bool generate_basis() {
@@ -1187,8 +1205,9 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
         const bool order = cap == cudaStreamCaptureStatusNone;  // no outside event inside a capture
         if (order && c.scratch_pending) P2G_CU(cudaStreamWaitEvent(s, c.ev_scratch, 0));
         P2G_CU(cudaMemsetAsync(c.err.p, 0, sizeof(int), s));
-        if (use_tensor_encode(jb.flags, S, R, jb.slice_size)) {
-            P2G_CU(c.aimg.ensure(mma_aimg_bytes(S, R)));
+        bool tensor = false;
+        P2G_TRY(choose_encode(c, jb.flags, S, R, jb.slice_size, &tensor));
+        if (tensor) {
             P2G_CU(launch_encode_mma(jb.src, jb.src_stride, S, jb.slice_size, R, jb.first_exponent,
                                      c.aimg.as<uint8_t>(), jb.recovery, jb.recovery_stride, c.err.as<int>(), s));
         } else {
@@ -1223,8 +1242,9 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
         P2G_CU(cudaMemcpy2DAsync(c.src.p, stride, jb.src, jb.src_stride, jb.slice_size, S, cudaMemcpyHostToDevice, s));
         if (stride != jb.slice_size)  // the 16-byte padding of each row is read: zero it
             P2G_CU(cudaMemset2DAsync(c.src.as<uint8_t>() + jb.slice_size, stride, 0, stride - jb.slice_size, S, s));
-        if (use_tensor_encode(jb.flags, S, R, jb.slice_size)) {
-            P2G_CU(c.aimg.ensure(mma_aimg_bytes(S, R)));
+        bool tensor = false;
+        P2G_TRY(choose_encode(c, jb.flags, S, R, jb.slice_size, &tensor));
+        if (tensor) {
             P2G_CU(launch_encode_mma(c.src.as<uint8_t>(), stride, S, jb.slice_size, R, jb.first_exponent,
                                      c.aimg.as<uint8_t>(), c.rec.as<uint8_t>(), stride, c.err.as<int>(), s));
         } else {
