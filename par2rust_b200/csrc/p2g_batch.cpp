@@ -133,7 +133,7 @@ inline uint32_t slice_range(const PlanJob& j, uint32_t C) {
 
 // Items of all jobs in queue order: every job's set-id item (its chains wait
 // for it), then the MD5 scan items, longest first, then the encode items job
-// by job (largest job first), band by band, tile-major within a band so a
+// by job (longest chains first), band by band, tile-major within a band so a
 // tile's row groups run together and share its source reads in L2, and last
 // the short CRC items, which fill the ragged final round of the encode.  A
 // folded item covers the last row group of `fold` adjacent tiles.
@@ -143,7 +143,7 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
     p.band_syms.assign(jobs.size(), 0);
     std::vector<std::pair<double, BatchItem>> pre, post;
     struct JobItems {
-        double key;
+        double chain, key;
         uint32_t job;
         std::vector<BatchItem> items;
     };
@@ -181,7 +181,7 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
         p.band_syms[ji] = bt * j.ts;
         p.band_items[ji].assign(nb, 0);
         std::vector<uint32_t>& counts = p.band_items[ji];
-        JobItems e{0.0, ji, {}};
+        JobItems e{j.chains ? md5_ms(j.slice + 36) : 0.0, 0.0, ji, {}};
         const uint32_t first_split = j.chains && j.split_chunks > 1 && j.split_bands
                                          ? nb - std::min(nb, j.split_bands) : nb;
         for (uint32_t b = 0; b < nb; ++b) {
@@ -230,7 +230,12 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
         enc.push_back(std::move(e));
     }
     std::stable_sort(pre.begin(), pre.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+    // Jobs with the longest packet chains first, larger jobs first among equals:
+    // a chain of 1 MiB rows runs 7.5 ms after its job's bands, and left to the
+    // end of the queue (jobs by size alone) one of 48 mixed jobs kept the
+    // launch at 33.5 ms that had run dry at 27.4.
     std::stable_sort(enc.begin(), enc.end(), [](const JobItems& a, const JobItems& b) {
+        if (a.chain != b.chain) return a.chain > b.chain;
         if (a.key != b.key) return a.key > b.key;
         return a.job < b.job;
     });
@@ -434,7 +439,7 @@ bool prefer_mma(uint64_t slice, uint32_t S, uint32_t R) {
 // 39 on the tensor cores, 256 KiB x 64 x 32 72 and 54, 1 MiB x 16 x 100 179
 // and 303.
 bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R) {
-    if (!R || !S) return false;
+    if (!R || S <= 6) return false;  // a few slices: the lookup kernel, or a tie
     const uint32_t Np = (uint32_t)(round_up(slice, 16) / 2), sms = (uint32_t)kMaxCtas;
     const uint32_t rows = mma_rows(R), RT = mma_row_tiles(R);
     const uint64_t tiles = (uint64_t)((Np + kMmaTileSymbols - 1) / kMmaTileSymbols) * RT;
