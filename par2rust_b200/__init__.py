@@ -529,7 +529,8 @@ def file_hashes(buffers: Sequence[bytes]) -> List[Tuple[bytes, bytes]]:
     """(hash_full, hash16k) per buffer, computed on the device."""
     import numpy as np
 
-    arrs = [np.frombuffer(bytes(b) + b"\0" * 4, dtype=np.uint8) for b in buffers]
+    # bytes are hashed where they lie (their data is 16-byte aligned)
+    arrs = [np.frombuffer(b if type(b) is bytes and b else bytes(b) + b"\0" * 4, dtype=np.uint8) for b in buffers]
     n = len(arrs)
     ptrs = (C.c_void_p * max(n, 1))(*[a.ctypes.data for a in arrs])
     lens = (C.c_uint64 * max(n, 1))(*[len(b) for b in buffers])

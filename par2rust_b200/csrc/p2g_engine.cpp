@@ -48,6 +48,9 @@ static inline uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m
 // slice, is encoded in 24 bits; larger tails are memset apart).
 constexpr uint32_t kGatherMinFiles = 8;
 constexpr uint64_t kGatherSegBytes = 4ull << 20;
+// Staged uploads of pageable host buffers (upload_host).
+constexpr uint64_t kUploadChunk = 1ull << 20, kUploadSlots = 8;
+constexpr uint64_t kUploadMin = 1ull << 20;  // smaller ones: one copy of the driver's
 
 // Grow-only device buffer.
 struct DevBuf {
@@ -104,6 +107,8 @@ struct Context {
     DevBuf persist;    // single-job persistent run: descriptor, items, chain state, tables
     PinBuf h_spans, h_h16k, h_err, h_stage, h_persist, h_gseg;
     PinBuf h_rec;   // host copy of the recovery rows (create calls)
+    PinBuf h_up;    // slots of the staged uploads, two to a thread
+    cudaEvent_t ev_up[8] = {};
     PinBuf h_prog;  // encode progress: the device queue head, read while a job runs
 };
 static Context& ctx() {
@@ -140,6 +145,7 @@ static p2g_status ensure_ready(Context& c) {
         P2G_CU(cudaEventCreateWithFlags(&c.ev_h16k, cudaEventDisableTiming));
         for (auto& ev : c.ev_join) P2G_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         for (auto& ev : c.ev_band) P2G_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        for (auto& ev : c.ev_up) P2G_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         P2G_CU(upload_tables());
         P2G_CU(c.err.ensure(64));
         P2G_CU(c.h_err.ensure(64));
@@ -587,7 +593,7 @@ static p2g_status run_device_job(Context& c, DeviceJob& j, cudaStream_t caller) 
             hs[n + f] = {j.files[f].first_slice * j.slice, j.files[f].length};
         }
         P2G_CU(cudaMemcpyAsync(c.spans.p, hs, sizeof(FileSpan) * 2 * n, cudaMemcpyHostToDevice, s_files));
-        P2G_CU(launch_md5_files(j.d_src, c.spans.as<FileSpan>(), n, j.d_h16k, s_files));
+        P2G_CU(launch_md5_files(j.d_src, c.spans.as<FileSpan>(), n, j.d_h16k, false, s_files));
         if (!j.have_set_id) {
             P2G_CU(c.h_h16k.ensure(16 * n));
             P2G_CU(cudaMemcpyAsync(c.h_h16k.p, j.d_h16k, 16 * n, cudaMemcpyDeviceToHost, s_files));
@@ -596,7 +602,7 @@ static p2g_status run_device_job(Context& c, DeviceJob& j, cudaStream_t caller) 
         tr.mark("hash16k + D2H", s_files);
         if (j.d_hfull) {
             P2G_CU(cudaStreamWaitEvent(s_full, c.ev_h16k, 0));  // spans uploaded
-            P2G_CU(launch_md5_files(j.d_src, c.spans.as<FileSpan>() + n, n, j.d_hfull, s_full));
+            P2G_CU(launch_md5_files(j.d_src, c.spans.as<FileSpan>() + n, n, j.d_hfull, false, s_full));
             tr.mark("hash_full", s_full);
         }
     }
@@ -1144,6 +1150,89 @@ extern "C" p2g_status p2g_check_bounded_wait(uint32_t polls) {
 }
 
 // ---- seams ----------------------------------------------------------------
+// Uploads of the calls on host buffers.  The driver copies pageable memory at
+// ~11 GB/s on one thread, and ~8 us a piece; here up to four threads copy 1 MiB
+// chunks into page-locked slots, each sent as soon as it is full (64 MiB of
+// slices with their hashes: 6.9 -> 3.3 ms; 300 files, 9.6 MB: 4.4 -> 3.2 ms).
+// Page-locked sources and small ones go by cudaMemcpyAsync.  The segments are
+// in ascending order of dst; bytes between them are left undefined.  The call
+// ends with its stream synchronised, so the slots are free for the next one.
+struct UploadSeg {
+    const uint8_t* src;
+    uint64_t dst, len;
+};
+static p2g_status upload_host(Context& c, uint8_t* dst, const std::vector<UploadSeg>& seg, cudaStream_t s) {
+    if (seg.empty()) return P2G_OK;
+    const uint64_t total = seg.back().dst + seg.back().len;
+    bool staged = seg.size() > 1 ? total >= kUploadMin / 4 : total >= kUploadMin;
+    for (size_t i = 0; staged && i < seg.size(); ++i) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, seg[i].src) != cudaSuccess) cudaGetLastError();
+        else if (a.type != cudaMemoryTypeUnregistered) staged = false;
+    }
+    if (staged && c.h_up.ensure(kUploadSlots * kUploadChunk) != cudaSuccess) {
+        cudaGetLastError();
+        staged = false;
+    }
+    if (!staged) {
+        for (const UploadSeg& g : seg) P2G_CU(cudaMemcpyAsync(dst + g.dst, g.src, g.len, cudaMemcpyHostToDevice, s));
+        return P2G_OK;
+    }
+    const uint64_t chunks = (total + kUploadChunk - 1) / kUploadChunk;
+    std::atomic<uint64_t> next{0};
+    std::atomic<uint32_t> who{0};
+    std::atomic<int> bad{(int)cudaSuccess};
+    auto work = [&]() {
+        const uint32_t t = who.fetch_add(1);
+        cudaError_t e = cudaSetDevice(c.device);
+        for (uint32_t k = 0; e == cudaSuccess && bad.load() == (int)cudaSuccess; ++k) {
+            const uint64_t i = next.fetch_add(1);
+            if (i >= chunks) break;
+            const uint32_t slot = 2 * t + (k & 1);
+            uint8_t* p = c.h_up.as<uint8_t>() + slot * kUploadChunk;
+            const uint64_t a = i * kUploadChunk, b = std::min(total, a + kUploadChunk);
+            if (k >= 2 && (e = cudaEventSynchronize(c.ev_up[slot])) != cudaSuccess) break;
+            auto g = std::upper_bound(seg.begin(), seg.end(), a, [](uint64_t v, const UploadSeg& u) { return v < u.dst + u.len; });
+            for (; g != seg.end() && g->dst < b; ++g) {
+                const uint64_t lo = std::max(a, g->dst), hi = std::min(b, g->dst + g->len);
+                memcpy(p + (lo - a), g->src + (lo - g->dst), hi - lo);
+            }
+            if ((e = cudaMemcpyAsync(dst + a, p, b - a, cudaMemcpyHostToDevice, s)) == cudaSuccess)
+                e = cudaEventRecord(c.ev_up[slot], s);
+        }
+        if (e != cudaSuccess) bad.store((int)e);
+    };
+    run_on_threads((unsigned)std::min<uint64_t>(kUploadSlots / 2, chunks), work);
+    const cudaError_t e = (cudaError_t)bad.load();
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(s);  // copies from the slots in flight
+        return cuda_fail(e, "upload of host buffers");
+    }
+    return P2G_OK;
+}
+// `count` rows of `len` bytes, src_stride apart, to rows dst_stride apart.
+static p2g_status upload_rows(Context& c, uint8_t* dst, uint64_t dst_stride, const uint8_t* src, uint64_t src_stride,
+                              uint64_t len, uint32_t count, cudaStream_t s) {
+    if (len * count < kUploadMin) {
+        P2G_CU(cudaMemcpy2DAsync(dst, dst_stride, src, src_stride, len, count, cudaMemcpyHostToDevice, s));
+        return P2G_OK;
+    }
+    std::vector<UploadSeg> seg;
+    if (src_stride == len && dst_stride == len) {
+        seg.push_back({src, 0, len * count});
+    } else {
+        seg.reserve(count);
+        for (uint32_t i = 0; i < count; ++i) seg.push_back({src + i * src_stride, i * dst_stride, len});
+    }
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, src) != cudaSuccess) cudaGetLastError();
+    else if (a.type != cudaMemoryTypeUnregistered) {
+        P2G_CU(cudaMemcpy2DAsync(dst, dst_stride, src, src_stride, len, count, cudaMemcpyHostToDevice, s));
+        return P2G_OK;
+    }
+    return upload_host(c, dst, seg, s);
+}
+
 extern "C" p2g_status p2g_gf_mul_xor(uint16_t coeff, const uint8_t* input, uint8_t* output, size_t len,
                                      uint32_t flags, void* stream) {
     Context& c = ctx();
@@ -1239,7 +1328,7 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
     P2G_CU(c.rec.ensure((size_t)stride * R));
     P2G_CU(cudaMemsetAsync(c.err.p, 0, sizeof(int), s));
     if (S) {
-        P2G_CU(cudaMemcpy2DAsync(c.src.p, stride, jb.src, jb.src_stride, jb.slice_size, S, cudaMemcpyHostToDevice, s));
+        P2G_TRY(upload_rows(c, c.src.as<uint8_t>(), stride, jb.src, jb.src_stride, jb.slice_size, S, s));
         if (stride != jb.slice_size)  // the 16-byte padding of each row is read: zero it
             P2G_CU(cudaMemset2DAsync(c.src.as<uint8_t>() + jb.slice_size, stride, 0, stride - jb.slice_size, S, s));
         bool tensor = false;
@@ -1289,7 +1378,7 @@ extern "C" p2g_status p2g_slice_checksums(const uint8_t* src, uint64_t src_strid
     cudaStream_t s = c.st[0];
     P2G_CU(c.src.ensure((size_t)slice_size * count));
     P2G_CU(c.checks.ensure(sizeof(p2g_slice_checksum) * count));
-    P2G_CU(cudaMemcpy2DAsync(c.src.p, slice_size, src, src_stride, slice_size, count, cudaMemcpyHostToDevice, s));
+    P2G_TRY(upload_rows(c, c.src.as<uint8_t>(), slice_size, src, src_stride, slice_size, count, s));
     P2G_CU(launch_md5_slices(c.src.as<uint8_t>(), slice_size, count, slice_size, c.checks.as<p2g_slice_checksum>(), s));
     P2G_CU(launch_crc_slices(c.src.as<uint8_t>(), slice_size, count, slice_size, c.checks.as<p2g_slice_checksum>(), s));
     P2G_CU(cudaMemcpyAsync(out, c.checks.p, sizeof(p2g_slice_checksum) * count, cudaMemcpyDeviceToHost, s));
@@ -1322,26 +1411,30 @@ extern "C" p2g_status p2g_file_hashes(const uint8_t* const* data, const uint64_t
             hs[n + f] = {(uint64_t)(data[f] - base), lengths[f]};
         }
         P2G_CU(cudaMemcpyAsync(c.spans.p, hs, sizeof(FileSpan) * 2 * n, cudaMemcpyHostToDevice, s));
-        if (hash16k_out) P2G_CU(launch_md5_files(base, c.spans.as<FileSpan>(), n, hash16k_out, s));
-        if (hash_full_out) P2G_CU(launch_md5_files(base, c.spans.as<FileSpan>() + n, n, hash_full_out, s));
+        bool vec = (uintptr_t)base % 16 == 0;
+        for (uint32_t f = 0; f < n; ++f) vec = vec && (uintptr_t)data[f] % 16 == 0;
+        if (hash16k_out) P2G_CU(launch_md5_files(base, c.spans.as<FileSpan>(), n, hash16k_out, vec, s));
+        if (hash_full_out) P2G_CU(launch_md5_files(base, c.spans.as<FileSpan>() + n, n, hash_full_out, vec, s));
         P2G_CU(cudaStreamSynchronize(s));  // h_spans is reused by the next call
         return P2G_OK;
     }
     cudaStream_t s = c.st[0];
     P2G_CU(c.src.ensure(std::max<uint64_t>(total + 16 * n, 16)));
     uint64_t off = 0;
+    std::vector<UploadSeg> seg;
     for (uint32_t f = 0; f < n; ++f) {
         hs[f] = {off, std::min<uint64_t>(lengths[f], P2G_HASH16K_LEN)};
         hs[n + f] = {off, lengths[f]};
-        if (lengths[f]) P2G_CU(cudaMemcpyAsync(c.src.as<uint8_t>() + off, data[f], lengths[f], cudaMemcpyHostToDevice, s));
+        if (lengths[f]) seg.push_back({data[f], off, lengths[f]});
         off = round_up(off + lengths[f], 16);
     }
+    P2G_TRY(upload_host(c, c.src.as<uint8_t>(), seg, s));
     P2G_CU(c.hfull.ensure(32 * (size_t)n));
     uint8_t* d16 = c.hfull.as<uint8_t>();
     uint8_t* dfull = d16 + 16 * (size_t)n;
     P2G_CU(cudaMemcpyAsync(c.spans.p, hs, sizeof(FileSpan) * 2 * n, cudaMemcpyHostToDevice, s));
-    P2G_CU(launch_md5_files(c.src.as<uint8_t>(), c.spans.as<FileSpan>(), n, d16, s));
-    P2G_CU(launch_md5_files(c.src.as<uint8_t>(), c.spans.as<FileSpan>() + n, n, dfull, s));
+    // both hashes of every file in one launch: the 16 KiB chains beside the long ones
+    P2G_CU(launch_md5_files(c.src.as<uint8_t>(), c.spans.as<FileSpan>(), 2 * n, d16, true, s));
     if (hash16k_out) P2G_CU(cudaMemcpyAsync(hash16k_out, d16, 16 * (size_t)n, cudaMemcpyDeviceToHost, s));
     if (hash_full_out) P2G_CU(cudaMemcpyAsync(hash_full_out, dfull, 16 * (size_t)n, cudaMemcpyDeviceToHost, s));
     P2G_CU(cudaStreamSynchronize(s));
@@ -1369,7 +1462,7 @@ extern "C" p2g_status p2g_recovery_packet_md5(const uint8_t set_id[16], const ui
     cudaStream_t s = c.st[0];
     P2G_CU(c.rec.ensure((size_t)slice_size * count));
     P2G_CU(c.pkt.ensure(16 * (size_t)count));
-    P2G_CU(cudaMemcpy2DAsync(c.rec.p, slice_size, recovery, recovery_stride, slice_size, count, cudaMemcpyHostToDevice, s));
+    P2G_TRY(upload_rows(c, c.rec.as<uint8_t>(), slice_size, recovery, recovery_stride, slice_size, count, s));
     P2G_CU(launch_md5_recovery(c.rec.as<uint8_t>(), slice_size, count, slice_size, set_id, first_exponent,
                                c.pkt.as<uint8_t>(), s));
     P2G_CU(cudaMemcpyAsync(md5_out, c.pkt.p, 16 * (size_t)count, cudaMemcpyDeviceToHost, s));

@@ -74,8 +74,9 @@ cudaError_t launch_md5_slices(const uint8_t* src, uint64_t stride, uint32_t coun
                               uint64_t slice_size, p2g_slice_checksum* out, cudaStream_t st);
 cudaError_t launch_crc_slices(const uint8_t* src, uint64_t stride, uint32_t count,
                               uint64_t slice_size, p2g_slice_checksum* out, cudaStream_t st);
+// vec: every file starts 16-byte aligned (else 4-byte).
 cudaError_t launch_md5_files(const uint8_t* base, const FileSpan* spans, uint32_t n,
-                             uint8_t* out16, cudaStream_t st);
+                             uint8_t* out16, bool vec, cudaStream_t st);
 cudaError_t launch_md5_recovery(const uint8_t* rec, uint64_t stride, uint32_t count,
                                 uint64_t slice_size, const uint8_t set_id[16], uint32_t first_exp,
                                 uint8_t* out16, cudaStream_t st);

@@ -2256,14 +2256,18 @@ cudaError_t launch_crc_slices(const uint8_t* src, uint64_t stride, uint32_t coun
     return cudaGetLastError();
 }
 
-cudaError_t launch_md5_files(const uint8_t* base, const FileSpan* spans, uint32_t n, uint8_t* out16,
+cudaError_t launch_md5_files(const uint8_t* base, const FileSpan* spans, uint32_t n, uint8_t* out16, bool vec,
                              cudaStream_t st) {
     if (!n) return cudaSuccess;
     const HashGrid g = hash_grid(n);
-    cudaError_t e = allow_exclusive(md5_files_kernel<false>);
-    if (e != cudaSuccess) return e;
-    // file starts are only known to be 4-byte aligned
-    md5_files_kernel<false><<<g.blocks, g.threads, g.smem, st>>>(base, spans, n, out16);
+    cudaError_t e;
+    if (vec) {
+        if ((e = allow_exclusive(md5_files_kernel<true>)) != cudaSuccess) return e;
+        md5_files_kernel<true><<<g.blocks, g.threads, g.smem, st>>>(base, spans, n, out16);
+    } else {
+        if ((e = allow_exclusive(md5_files_kernel<false>)) != cudaSuccess) return e;
+        md5_files_kernel<false><<<g.blocks, g.threads, g.smem, st>>>(base, spans, n, out16);
+    }
     count_launch();
     return cudaGetLastError();
 }

@@ -104,3 +104,23 @@ def test_slice_crc_in_device_job(p2g, gpu):
         for i in range(slices):
             s = host[i * size:(i + 1) * size].tobytes()
             assert got[i].tobytes() == hashlib.md5(s).digest() + zlib.crc32(s).to_bytes(4, "little"), (size, i)
+
+
+def test_staged_host_uploads(p2g, gpu, oracle):
+    """Pageable inputs around the staging chunks (1 MiB): one run of bytes,
+    many pieces with gaps between them, and rows padded to another stride."""
+    import numpy as np
+
+    rng = np.random.default_rng(9)
+    for size, count in ((1 << 20, 1), ((1 << 20) + 4, 3), (262140, 21), (1028, 4097)):
+        src = rng.integers(0, 256, size * count, dtype=np.uint8)
+        got = p2g.slice_checksums(src, size)
+        assert [(c.md5, c.crc32) for c in got] == [
+            (hashlib.md5(s).digest(), zlib.crc32(s)) for s in (src[i * size:(i + 1) * size].tobytes() for i in range(count))]
+    lengths = [1, (1 << 20) - 1, 15, (1 << 20) + 1, 3 << 20, 0, 7, 700_001]
+    files = [rng.integers(0, 256, n, dtype=np.uint8).tobytes() for n in lengths]
+    assert p2g.file_hashes(files) == [(hashlib.md5(f).digest(), hashlib.md5(f[:16384]).digest()) for f in files]
+    assert p2g.file_hashes([bytearray(f) for f in files]) == p2g.file_hashes(files)
+    S, size, R = 130, 16388, 3  # 16,400-byte rows on the device
+    src = rng.integers(0, 256, S * size, dtype=np.uint8)
+    assert np.array_equal(p2g.encode(src, size, R), oracle.encode_fast(src, S, size, R))
