@@ -137,7 +137,7 @@ inline uint32_t slice_range(const PlanJob& j, uint32_t C) {
 // tile's row groups run together and share its source reads in L2, and last
 // the short CRC items, which fill the ragged final round of the encode.  A
 // folded item covers the last row group of `fold` adjacent tiles.
-Plan build_items(const std::vector<PlanJob>& jobs) {
+Plan build_items(const std::vector<PlanJob>& jobs, uint32_t ctas) {
     Plan p;
     p.band_items.resize(jobs.size());
     p.band_syms.assign(jobs.size(), 0);
@@ -173,9 +173,12 @@ Plan build_items(const std::vector<PlanJob>& jobs) {
         // A job alone whose chains last more than half as long as its encode
         // keeps one CTA on each row block's chains: left to the CTAs that
         // complete bands, the blocks' last bands ran one after the other (538
-        // MB, 200 rows: encode done at 4.3 ms, chains at 5.2).
-        if (j.lone && j.chains && nb > 1 && 2 * md5_ms(j.slice + 36) * kMaxCtas > encode_cost_ms(j.slice, j.S, j.R, j.mma))
-            for (uint32_t q = 0; q < (j.R + kChainRows - 1) / kChainRows; ++q)
+        // MB, 200 rows: encode done at 4.3 ms, chains at 5.2).  They wait for
+        // the other CTAs' encode items, so they take a quarter of the CTAs at most.
+        const uint32_t Q = (j.R + kChainRows - 1) / kChainRows;
+        if (j.lone && j.chains && nb > 1 && 4 * Q <= ctas &&
+            2 * md5_ms(j.slice + 36) * ctas > encode_cost_ms(j.slice, j.S, j.R, j.mma))
+            for (uint32_t q = 0; q < Q; ++q)
                 pre.push_back({9e29, {ji, kItemChain, q, 0, 0, 0}});
         const uint32_t F = j.mma ? 1u : tail_fold(j.R);
         p.band_syms[ji] = bt * j.ts;
@@ -325,7 +328,7 @@ Plan plan_batch(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
         for (uint32_t chunks : {2u, 4u, 8u}) {
             j.split_bands = std::min(bands, nb);
             j.split_chunks = chunks;
-            Plan p = build_items(jobs);
+            Plan p = build_items(jobs, ctas);
             p.makespan = simulate(jobs, p, ctas);
             if (p.makespan < best.makespan * kPlanMargin) {
                 best = std::move(p);
@@ -365,7 +368,7 @@ Plan plan_tiles(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
             j.tiles = tiles;
         }
     }
-    Plan best = build_items(jobs);
+    Plan best = build_items(jobs, ctas);
     best.makespan = simulate(jobs, best, ctas);
     if (flags & P2G_BATCH_NO_AUTOTUNE) return best;
     // lower bound at the widest tiles: all work spread evenly over the CTAs
@@ -391,7 +394,7 @@ Plan plan_tiles(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
             const uint32_t t = base * mult;
             if ((j.Np + t - 1) / t < 64) continue;  // tiles too small to pay for their table builds
             set_tiling(j, t);
-            Plan p = build_items(jobs);
+            Plan p = build_items(jobs, ctas);
             p.makespan = simulate(jobs, p, ctas);
             if (p.makespan < best.makespan * kPlanMargin) {
                 best = std::move(p);

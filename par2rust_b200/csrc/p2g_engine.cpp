@@ -26,6 +26,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -1218,15 +1219,21 @@ static p2g_status upload_rows(Context& c, uint8_t* dst, uint64_t dst_stride, con
         return P2G_OK;
     }
     std::vector<UploadSeg> seg;
-    if (src_stride == len && dst_stride == len) {
-        seg.push_back({src, 0, len * count});
-    } else {
-        seg.reserve(count);
-        for (uint32_t i = 0; i < count; ++i) seg.push_back({src + i * src_stride, i * dst_stride, len});
-    }
     cudaPointerAttributes a;
+    bool staged = true;
     if (cudaPointerGetAttributes(&a, src) != cudaSuccess) cudaGetLastError();
-    else if (a.type != cudaMemoryTypeUnregistered) {
+    else if (a.type != cudaMemoryTypeUnregistered) staged = false;
+    try {
+        if (staged && src_stride == len && dst_stride == len) {
+            seg.push_back({src, 0, len * count});
+        } else if (staged) {
+            seg.reserve(count);
+            for (uint32_t i = 0; i < count; ++i) seg.push_back({src + i * src_stride, i * dst_stride, len});
+        }
+    } catch (const std::bad_alloc&) {
+        staged = false;
+    }
+    if (!staged) {
         P2G_CU(cudaMemcpy2DAsync(dst, dst_stride, src, src_stride, len, count, cudaMemcpyHostToDevice, s));
         return P2G_OK;
     }
@@ -1422,10 +1429,19 @@ extern "C" p2g_status p2g_file_hashes(const uint8_t* const* data, const uint64_t
     P2G_CU(c.src.ensure(std::max<uint64_t>(total + 16 * n, 16)));
     uint64_t off = 0;
     std::vector<UploadSeg> seg;
+    bool listed = true;
+    try {
+        seg.reserve(n);
+    } catch (const std::bad_alloc&) {
+        listed = false;
+    }
     for (uint32_t f = 0; f < n; ++f) {
         hs[f] = {off, std::min<uint64_t>(lengths[f], P2G_HASH16K_LEN)};
         hs[n + f] = {off, lengths[f]};
-        if (lengths[f]) seg.push_back({data[f], off, lengths[f]});
+        if (lengths[f] && listed)
+            seg.push_back({data[f], off, lengths[f]});
+        else if (lengths[f])
+            P2G_CU(cudaMemcpyAsync(c.src.as<uint8_t>() + off, data[f], lengths[f], cudaMemcpyHostToDevice, s));
         off = round_up(off + lengths[f], 16);
     }
     P2G_TRY(upload_host(c, c.src.as<uint8_t>(), seg, s));

@@ -1363,8 +1363,7 @@ __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, c
     MmaSlot& cur = slots[P.tcount & 1u];
     MmaSlot& nxt = slots[(P.tcount & 1u) ^ 1u];
     P.next = &nxt.T;
-    if (threadIdx.x < 32) mma::tensormap_acquire(cur.T.src_map);  // written by the host's upload of the jobs
-    const bool ok = mma::run_tile<kBatchInStages>(P, cur.T, [&] {
+    const bool ok = mma::run_tile<kBatchInStages, true>(P, cur.T, [&] {
         if (threadIdx.x & 31) return;
         const BatchJob& J = jobs[cur.job];
         if (count_prev && jobs[nxt.job].n_bands) {
@@ -1391,7 +1390,6 @@ __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, c
             return;
         }
         const BatchJob& Jn = jobs[it.job];
-        mma::tensormap_acquire(&Jn.src_map);
         nxt.job = it.job;
         nxt.band = it.b >> 16;
         nxt.T = batch_mma_tile_of(Jn, it);

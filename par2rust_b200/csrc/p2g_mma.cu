@@ -157,7 +157,7 @@ __device__ __noinline__ bool encode_mma_tile(const EncodeArgs& A, uint32_t tile,
     Tile* const slot = reinterpret_cast<Tile*>(smem + kOffNext);
     P.next = slot;
     const Tile T = tile_of(A, tile);
-    const bool ok = run_tile<kInStages>(P, T, [&] {
+    const bool ok = run_tile<kInStages, false>(P, T, [&] {
         if ((threadIdx.x & 31) == 0) {
             if (next < A.row_tiles * A.sym_tiles)
                 *slot = tile_of(A, next);

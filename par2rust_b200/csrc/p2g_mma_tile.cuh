@@ -312,7 +312,9 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // whose wait gave up runs on to its end (every later wait returns at once; the
 // tile is dropped, its memory is the CTA's own and nothing is stored).
 constexpr uint32_t kHelperLead = 4;  // with 5 more in flight, about 8,000 cycles before the tile's end
-template <int IN, class Helper>
+// ACQUIRE: the tensor maps were written by ordinary stores or copies (the
+// batch job descriptors); the warp that issues the copies acquires each.
+template <int IN, bool ACQUIRE, class Helper>
 __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper) {
     const uint32_t warp = uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const Bars<IN> B(uni(P.bars));
@@ -357,14 +359,17 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
                 }
             }
         };
+        if (ACQUIRE && pre == 0) tensormap_acquire(T.src_map);
         issue(uni((uint64_t)(uintptr_t)T.src_map), uni((uint64_t)(uintptr_t)T.aimg), n0, s0, rows, pre, NI);
         if (ok) ok = warp_wait(B.next_full, tc & 1u, P.abort_flag);
         if (ok) {
             const uint32_t n_rows = uni(P.next->rows), nx = uni(P.next->n0), ns = uni(P.next->s0);
             const uint32_t ni = (uni(P.next->sn) + kInSlices - 1) / kInSlices;
-            if (n_rows && n_rows <= kMaxRows && !(nx & 7u) && !(ns % kInSlices))
+            if (n_rows && n_rows <= kMaxRows && !(nx & 7u) && !(ns % kInSlices)) {
+                if (ACQUIRE) tensormap_acquire(P.next->src_map);
                 issue(uni((uint64_t)(uintptr_t)P.next->src_map), uni((uint64_t)(uintptr_t)P.next->aimg), nx, ns, n_rows, 0,
                       ni < (uint32_t)IN ? ni : (uint32_t)IN);
+            }
         }
         if (!ok) {  // copies issued but maybe not consumed land before the stages are reused
             for (uint32_t q = gi > gi0 + IN ? gi - IN : gi0; q < gi; ++q)
