@@ -1363,7 +1363,7 @@ __device__ __noinline__ bool batch_mma_tile(const BatchJob* __restrict__ jobs, c
     MmaSlot& cur = slots[P.tcount & 1u];
     MmaSlot& nxt = slots[(P.tcount & 1u) ^ 1u];
     P.next = &nxt.T;
-    const bool ok = mma::run_tile<kBatchInStages, true>(P, cur.T, [&] {
+    const bool ok = mma::run_tile<kBatchInStages, true, false>(P, cur.T, [&] {
         if (threadIdx.x & 31) return;
         const BatchJob& J = jobs[cur.job];
         if (count_prev && jobs[nxt.job].n_bands) {

@@ -55,8 +55,8 @@ constexpr int kInStages = 6;  // 4 K-steps each: the MMAs of 20 in reserve, 4,20
 // shared memory layout (bytes): the ring, barriers, misc
 constexpr uint32_t kOffBars = kInStages * kInStageBytes;
 constexpr uint32_t kOffMisc = kOffBars + bar_bytes(kInStages);
-constexpr uint32_t kOffNext = kOffMisc + 32;  // the next tile
-constexpr uint32_t kSmemBytes = kOffNext + sizeof(Tile);
+constexpr uint32_t kOffNext = kOffMisc + 32;  // two tiles: the one at work and the next
+constexpr uint32_t kSmemBytes = kOffNext + 2 * sizeof(Tile);
 static_assert(kSmemBytes > 116 * 1024, "one CTA per SM: TMEM is allocated whole");
 static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
 static_assert(mma_image_steps(1027) == image_steps(1027) && mma_image_steps(32) == image_steps(32) &&
@@ -138,11 +138,18 @@ __device__ __forceinline__ Tile tile_of(const EncodeArgs& A, uint32_t at) {
     return T;
 }
 
-// One tile, out of line with its pipeline state in shared memory (misc[0]
-// TMEM base, [1] abort flag, [2..5] state), as in the batch kernel: inlined
-// into the tile loop the compiler keeps the MMA warp's operands out of uniform
-// registers, and a K-step takes 300 cycles.
-__device__ __noinline__ bool encode_mma_tile(const EncodeArgs& A, uint32_t tile, uint32_t next) {
+// One tile, out of line as in the batch kernel: inlined into the tile loop the
+// compiler keeps the MMA warp's operands out of uniform registers, and a
+// K-step takes 300 cycles.  The pipeline's state stays in registers from tile
+// to tile (shared memory and a second CTA barrier cost 1-2 % on short tiles).
+// The tile is in shared memory, worked out by one thread: its divisions by
+// every thread ahead of the roles cost 3 us of 56 at 64 slices.
+// misc: [0] TMEM base, [1] abort flag, [5] input stages issued.
+struct PipeState {
+    uint32_t gi, tcount, pre, ok;
+};
+__device__ __noinline__ PipeState encode_mma_tile(const EncodeArgs& A, uint32_t next, uint32_t gi, uint32_t tcount,
+                                                  uint32_t pre) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint32_t* misc = reinterpret_cast<uint32_t*>(smem + kOffMisc);
     mma::Pipe P;
@@ -150,14 +157,15 @@ __device__ __noinline__ bool encode_mma_tile(const EncodeArgs& A, uint32_t tile,
     P.bars = smem_addr(smem + kOffBars);
     P.tmem = misc[0];
     P.abort_flag = misc + 1;
-    P.gi = misc[2];
-    P.tcount = misc[3];
-    P.pre = misc[4];
+    P.gi = gi;
+    P.tcount = tcount;
+    P.pre = pre;
     P.issued = misc + 5;
-    Tile* const slot = reinterpret_cast<Tile*>(smem + kOffNext);
+    // the helper warp works out the next tile while this one runs
+    Tile* const slots = reinterpret_cast<Tile*>(smem + kOffNext);
+    Tile* const slot = slots + ((P.tcount & 1u) ^ 1u);
     P.next = slot;
-    const Tile T = tile_of(A, tile);
-    const bool ok = run_tile<kInStages, false>(P, T, [&] {
+    const bool ok = run_tile<kInStages, false, true>(P, slots[P.tcount & 1u], [&] {
         if ((threadIdx.x & 31) == 0) {
             if (next < A.row_tiles * A.sym_tiles)
                 *slot = tile_of(A, next);
@@ -165,13 +173,7 @@ __device__ __noinline__ bool encode_mma_tile(const EncodeArgs& A, uint32_t tile,
                 slot->rows = 0;
         }
     });  // ends with a CTA barrier
-    if (threadIdx.x == 0) {
-        misc[2] = P.gi;
-        misc[3] = P.tcount;
-        misc[4] = P.pre;
-    }
-    __syncthreads();
-    return ok;
+    return {P.gi, P.tcount, P.pre, ok};
 }
 
 __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_constant__ EncodeArgs A,
@@ -181,7 +183,8 @@ __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_co
     uint32_t* misc = reinterpret_cast<uint32_t*>(smem + kOffMisc);
     if (tid == 0) {
         init_bars<kInStages>(smem_addr(smem + kOffBars));
-        for (int i = 1; i < 6; ++i) misc[i] = 0;
+        misc[1] = misc[5] = 0;
+        *reinterpret_cast<Tile*>(smem + kOffNext) = tile_of(A, blockIdx.x);
     }
     if (warp == 1) tmem_alloc(smem_addr(misc));  // the whole of TMEM: two accumulators, A stages, scale factors
     tc_fence_before();
@@ -192,10 +195,10 @@ __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    bool ok = true;
-    for (uint32_t tile = blockIdx.x; ok && tile < A.row_tiles * A.sym_tiles; tile += gridDim.x)
-        ok = encode_mma_tile(A, tile, tile + gridDim.x);
-    if (tid == 0 && !ok) atomicOr(err, 1);
+    PipeState st = {0, 0, 0, 1};
+    for (uint32_t tile = blockIdx.x; st.ok && tile < A.row_tiles * A.sym_tiles; tile += gridDim.x)
+        st = encode_mma_tile(A, tile + gridDim.x, st.gi, st.tcount, st.pre);
+    if (tid == 0 && !st.ok) atomicOr(err, 1);
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
