@@ -211,6 +211,12 @@ void p2g_output_set_free(p2g_output_set *os);
  * completes, for at most `polls` tries (1..2^24), and the call returns
  * P2G_ERR_TIMEOUT when the bound fired (it always should). */
 p2g_status p2g_check_bounded_wait(uint32_t polls);
+/* The same for the tensor-core encode: `tiles` tiles of 13 rows x 256 symbols
+ * over `input_slices` slices (33..32768) run with the third 16-slice stage of
+ * each never copied, so that every role of the kernel gives up, its copies and
+ * MMAs in flight land and its tensor memory is freed.  Returns P2G_ERR_TIMEOUT
+ * (it always should). */
+p2g_status p2g_check_tile_wait(uint32_t input_slices, uint32_t tiles);
 
 /* ---- hot-path seams -------------------------------------------------- */
 

@@ -475,6 +475,12 @@ def check_bounded_wait(polls: int = 1 << 16) -> None:
     _check(lib().p2g_check_bounded_wait(int(polls)))
 
 
+def check_tile_wait(input_slices: int = 64, tiles: int = 1) -> None:
+    """The same in the tensor-core encode: ``tiles`` tiles over
+    ``input_slices`` slices, one 16-slice stage of each never copied."""
+    _check(lib().p2g_check_tile_wait(int(input_slices), int(tiles)))
+
+
 def gf_mul_xor(coeff: int, input: bytes, output: bytearray) -> None:
     """output ^= coeff * input over LE GF(2^16) symbols (gf_mul_xor_dispatch)."""
     import numpy as np

@@ -1150,6 +1150,30 @@ extern "C" p2g_status p2g_check_bounded_wait(uint32_t polls) {
     return P2G_OK;
 }
 
+extern "C" p2g_status p2g_check_tile_wait(uint32_t input_slices, uint32_t tiles) {
+    Context& c = ctx();
+    std::lock_guard<std::recursive_mutex> lk(c.mu);
+    clear_error();
+    if (input_slices < 33 || input_slices > P2G_MAX_INPUT_BLOCKS || !tiles || tiles > 4096)
+        return set_error(P2G_ERR_INVALID_ARGUMENT, "input_slices must be in [33, 32768], tiles in [1, 4096]");
+    P2G_TRY(ensure_ready(c));
+    cudaStream_t s = c.st[0];
+    if (c.scratch_pending) P2G_CU(cudaStreamWaitEvent(s, c.ev_scratch, 0));
+    const uint64_t slice = 2ull * kMmaTileSymbols * tiles;
+    if (slice * input_slices > 1ull << 30) return set_error(P2G_ERR_INVALID_ARGUMENT, "more than 1 GiB of slices");
+    P2G_CU(c.src.ensure(slice * input_slices));
+    P2G_CU(c.rec.ensure(slice * kMmaMaxRows));
+    P2G_CU(c.aimg.ensure(mma_aimg_bytes(input_slices, kMmaMaxRows)));
+    P2G_CU(cudaMemsetAsync(c.err.p, 0, sizeof(int), s));
+    P2G_CU(cudaMemsetAsync(c.src.p, 0, slice * input_slices, s));
+    P2G_CU(launch_encode_mma(c.src.as<uint8_t>(), slice, input_slices, slice, kMmaMaxRows, 0, c.aimg.as<uint8_t>(),
+                             c.rec.as<uint8_t>(), slice, c.err.as<int>(), s, true));
+    P2G_CU(cudaMemcpyAsync(c.h_err.p, c.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    P2G_CU(cudaStreamSynchronize(s));
+    c.scratch_pending = false;
+    return check_device_error(c);
+}
+
 // ---- seams ----------------------------------------------------------------
 // Uploads of the calls on host buffers.  The driver copies pageable memory at
 // ~11 GB/s on one thread, and ~8 us a piece; here up to four threads copy 1 MiB

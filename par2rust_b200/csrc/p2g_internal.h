@@ -166,7 +166,7 @@ constexpr uint32_t mma_image_steps(uint32_t S) { return (S + 15) / 16 * 4; }
 cudaError_t make_src_map(CUtensorMap* map, const void* src, uint64_t stride, uint32_t S, uint32_t Np);
 cudaError_t launch_encode_mma(const uint8_t* src, uint64_t src_stride, uint32_t S, uint64_t slice_size, uint32_t R,
                               uint32_t first_exp, uint8_t* aimg, uint8_t* rec, uint64_t rec_stride, int* err,
-                              cudaStream_t st);
+                              cudaStream_t st, bool give_up = false);  // give_up: a stage's copies are left out
 
 // Size in bytes of the coefficient-basis scratch for S slices and RG groups.
 inline size_t basis_bytes(uint32_t S, uint32_t RG) { return (size_t)S * RG * 512 * sizeof(uint16_t); }

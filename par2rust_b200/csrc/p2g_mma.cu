@@ -148,6 +148,7 @@ __device__ __forceinline__ Tile tile_of(const EncodeArgs& A, uint32_t at) {
 struct PipeState {
     uint32_t gi, tcount, pre, ok;
 };
+template <uint32_t POLLS, uint32_t DROP>
 __device__ __noinline__ PipeState encode_mma_tile(const EncodeArgs& A, uint32_t next, uint32_t gi, uint32_t tcount,
                                                   uint32_t pre) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -165,7 +166,7 @@ __device__ __noinline__ PipeState encode_mma_tile(const EncodeArgs& A, uint32_t 
     Tile* const slots = reinterpret_cast<Tile*>(smem + kOffNext);
     Tile* const slot = slots + ((P.tcount & 1u) ^ 1u);
     P.next = slot;
-    const bool ok = run_tile<kInStages, false, true>(P, slots[P.tcount & 1u], [&] {
+    const bool ok = run_tile<kInStages, false, true, POLLS, DROP>(P, slots[P.tcount & 1u], [&] {
         if ((threadIdx.x & 31) == 0) {
             if (next < A.row_tiles * A.sym_tiles)
                 *slot = tile_of(A, next);
@@ -176,6 +177,7 @@ __device__ __noinline__ PipeState encode_mma_tile(const EncodeArgs& A, uint32_t 
     return {P.gi, P.tcount, P.pre, ok};
 }
 
+template <uint32_t POLLS, uint32_t DROP>
 __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_constant__ EncodeArgs A,
                                                                  int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_co
     tc_fence_after();
     PipeState st = {0, 0, 0, 1};
     for (uint32_t tile = blockIdx.x; st.ok && tile < A.row_tiles * A.sym_tiles; tile += gridDim.x)
-        st = encode_mma_tile(A, tile + gridDim.x, st.gi, st.tcount, st.pre);
+        st = encode_mma_tile<POLLS, DROP>(A, tile + gridDim.x, st.gi, st.tcount, st.pre);
     if (tid == 0 && !st.ok) atomicOr(err, 1);
     tc_fence_before();
     __syncthreads();
@@ -212,6 +214,10 @@ __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_co
 // Host side
 // ---------------------------------------------------------------------------
 namespace {
+// The kernel of every encode, and the one that checks the give-up path: a tile's
+// third stage never arrives and a wait is 4,096 polls.
+constexpr auto encode_kernel = encode_mma_kernel<kTilePolls, kDropNone>;
+constexpr auto giveup_kernel = encode_mma_kernel<4096, 2>;
 // The trace sequence and the dual basis from the field itself (polynomial
 // 0x1100B, generator 2).  Returns false if the trace form were singular (it
 // never is).
@@ -274,9 +280,9 @@ cudaError_t mma_prepare() {
     if (!build_trace_tables(bits, dual)) return cudaErrorInvalidValue;
     if ((e = cudaMemcpyToSymbol(d_trace_bits, bits.data(), 2 * bits.size())) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(d_dual_log, dual, sizeof dual)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(encode_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)) !=
-        cudaSuccess)
-        return e;
+    for (auto k : {encode_kernel, giveup_kernel})
+        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)) != cudaSuccess)
+            return e;
     if (dev >= 0 && dev < 256) done[dev] = true;
     return cudaSuccess;
 }
@@ -337,7 +343,7 @@ cudaError_t make_src_map(CUtensorMap* map, const void* src, uint64_t stride, uin
 
 cudaError_t launch_encode_mma(const uint8_t* src, uint64_t src_stride, uint32_t S, uint64_t slice_size, uint32_t R,
                               uint32_t first_exp, uint8_t* aimg, uint8_t* rec, uint64_t rec_stride, int* err,
-                              cudaStream_t st) {
+                              cudaStream_t st, bool give_up) {
     if (!S || !R) return cudaSuccess;
     cudaError_t e = mma_prepare();
     if (e != cudaSuccess) return e;
@@ -360,7 +366,7 @@ cudaError_t launch_encode_mma(const uint8_t* src, uint64_t src_stride, uint32_t 
     a_image_kernel<<<cb, kImageThreads, 0, st>>>(aimg, logbase, S, R, first_exp);
     add_launches(1);
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)A.row_tiles * A.sym_tiles, (uint64_t)sms);
-    encode_mma_kernel<<<grid, kThreads, kSmemBytes, st>>>(A, err);
+    (give_up ? giveup_kernel : encode_kernel)<<<grid, kThreads, kSmemBytes, st>>>(A, err);
     add_launches(1);
     return cudaGetLastError();
 }

@@ -93,10 +93,12 @@ __device__ __forceinline__ bool bar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// Polls of one wait before it gives up.
+constexpr uint32_t kTilePolls = 1u << 22;
 // Waits (bounded) for a phase without looking at the abort flag: for
 // copies and MMAs in flight, which land whatever happened elsewhere.
-__device__ __forceinline__ void bar_drain(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < (1u << 22) && !bar_try_wait(bar, parity); ++it) {
+__device__ __forceinline__ void bar_drain(uint32_t bar, uint32_t parity, uint32_t polls = kTilePolls) {
+    for (uint32_t it = 0; it < polls && !bar_try_wait(bar, parity); ++it) {
     }
 }
 __device__ __forceinline__ void tma_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -292,12 +294,14 @@ __device__ __forceinline__ uint64_t uni(uint64_t v) { return __shfl_sync(0xFFFFF
 // Bounded wait by a whole warp: false when it gave up (it then sets the abort
 // flag) or when another role has given up.  The lanes vote on every poll, so
 // that the loop's branch is one for the warp.
+template <uint32_t POLLS>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-    for (uint32_t it = 0; it < (1u << 22); ++it) {
+    for (uint32_t it = 0; it < POLLS; ++it) {
         if (__all_sync(0xFFFFFFFFu, bar_try_wait(bar, parity))) return true;
         if ((it & 255u) == 255u && __any_sync(0xFFFFFFFFu, *abort_flag != 0)) return false;
     }
     *abort_flag = 1u;
+    __threadfence_block();  // before anything this role still commits or arrives at
     return false;
 }
 
@@ -311,8 +315,8 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // that tile's first input stages while this tile's last K-steps and epilogue
 // run, so the next tile starts without a copy round trip.  Only warp 0's P.pre
 // counts (the stages it issued ahead); the next call must be for that same
-// tile.  When any role's wait gives up, warp 0 waits for every copy it issued,
-// the next tile's included, before this returns.
+// tile.  When any role's wait gives up, warp 0 issues nothing more and waits for
+// every copy it issued, the next tile's included, before this returns.
 //
 // Every role runs whole warps on values the compiler knows to be the same in
 // every lane (uni), with only the asynchronous instructions under the elected
@@ -323,8 +327,8 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // this way the warp keeps up with the MMAs.  For
 // the same reason the MMA and builder loops have no branch beside the waits'
 // own: K-steps past the tile's last multiply the builders' zeros, and a role
-// whose wait gave up runs on to its end (every later wait returns at once; the
-// tile is dropped, its memory is the CTA's own and nothing is stored).
+// whose wait gave up runs on to its end (the tile is dropped, its memory is the
+// CTA's own and nothing is stored).
 constexpr uint32_t kHelperLead = 4;  // with 5 more in flight, about 8,000 cycles before the tile's end
 // ACQUIRE: the tensor maps were written by ordinary stores or copies (the
 // batch job descriptors); the warp that issues the copies acquires each.
@@ -335,7 +339,11 @@ constexpr uint32_t kHelperLead = 4;  // with 5 more in flight, about 8,000 cycle
 // large ones, which the board's power limit holds, stay within 0.6 %.  In the
 // batch kernel the registers spill in its other items, and a 16 MiB job took
 // 682 us instead of 672.
-template <int IN, bool ACQUIRE, bool LOAD_AHEAD, class Helper>
+// POLLS, DROP: for the check of the give-up path alone (encode_mma_kernel's
+// other form); it waits POLLS polls and leaves out the copies of a tile's stage
+// DROP, so that every wait behind them runs out.
+constexpr uint32_t kDropNone = 0xFFFFFFFFu;
+template <int IN, bool ACQUIRE, bool LOAD_AHEAD, uint32_t POLLS = kTilePolls, uint32_t DROP = kDropNone, class Helper>
 __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper) {
     const uint32_t warp = uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const Bars<IN> B(uni(P.bars));
@@ -365,10 +373,15 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
             const uint8_t* a = reinterpret_cast<const uint8_t*>(aimg) + (uint64_t)(first / kInSlices + k0) * bytes;
             uint32_t sa = first + k0 * kInSlices;
             for (uint32_t k = k0; k < k1; ++k, ++gi, sa += kInSlices, a += bytes) {
-                ok = warp_wait(B.in_empty + 8 * st, par, P.abort_flag);
+                // A role that gave up on a stage runs on and gives the stage
+                // back with its copies perhaps in flight: none may follow them
+                // into it, nor its barrier be armed a second time.  The flag
+                // was set before the stage was given back.
+                ok = warp_wait<POLLS>(B.in_empty + 8 * st, par, P.abort_flag) &&
+                     !__any_sync(0xFFFFFFFFu, *P.abort_flag != 0);
                 if (!ok) return;
                 const uint32_t dst = in0 + st * kInStageBytes, full = B.in_full + 8 * st;
-                if (lead) {
+                if (lead && k != DROP) {
                     bar_expect_tx(full, bytes + kInSrcBytes);
                     tma_1d(dst, a, bytes, full);
                     tma_2d(dst + kInBBytes, reinterpret_cast<const void*>(map), (int32_t)x, (int32_t)sa, full);
@@ -382,7 +395,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
         };
         if (ACQUIRE && pre == 0) tensormap_acquire(T.src_map);
         issue(uni((uint64_t)(uintptr_t)T.src_map), uni((uint64_t)(uintptr_t)T.aimg), n0, s0, rows, pre, NI);
-        if (ok) ok = warp_wait(B.next_full, tc & 1u, P.abort_flag);
+        if (ok) ok = warp_wait<POLLS>(B.next_full, tc & 1u, P.abort_flag);
         if (ok) {
             const uint32_t n_rows = uni(P.next->rows), nx = uni(P.next->n0), ns = uni(P.next->s0);
             const uint32_t ni = (uni(P.next->sn) + kInSlices - 1) / kInSlices;
@@ -394,7 +407,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
         }
         if (!ok) {  // copies issued but maybe not consumed land before the stages are reused
             for (uint32_t q = gi > gi0 + IN ? gi - IN : gi0; q < gi; ++q)
-                bar_drain(B.in_full + 8 * (q % IN), (q / IN) & 1u);
+                bar_drain(B.in_full + 8 * (q % IN), (q / IN) & 1u, POLLS);
         } else {
             issued_end = gi;  // >= gi0 + NI: this tile's stages all went out
         }
@@ -402,15 +415,15 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
         uint32_t leader;
         const bool lead = elect_one(leader);
         const uint32_t id = idesc(16 * rows), step = rows * kRowStepBytes, sf = tmem + kSfCol;
-        ok = warp_wait(B.acc_empty, (tc & 1u) ^ 1u, P.abort_flag);
+        ok = warp_wait<POLLS>(B.acc_empty, (tc & 1u) ^ 1u, P.abort_flag);
         tc_fence_after();
         uint32_t si = gi0 % IN, pi = (gi0 / IN) & 1u, pa = gi0 & 1u;
         for (uint32_t k = 0; k < NI; ++k) {
-            ok &= warp_wait(B.in_full + 8 * si, pi, P.abort_flag);
+            ok &= warp_wait<POLLS>(B.in_full + 8 * si, pi, P.abort_flag);
             const uint32_t b0 = in0 + si * kInStageBytes;
 #pragma unroll
             for (uint32_t u = 0; u < kAStages; ++u) {
-                ok &= warp_wait(B.a_full + 8 * u, pa, P.abort_flag);
+                ok &= warp_wait<POLLS>(B.a_full + 8 * u, pa, P.abort_flag);
                 tc_fence_after();
                 if (lead) {
 #pragma unroll
@@ -432,7 +445,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
         }
         if (lead) mma_commit(B.acc_full);
         // every MMA issued completes before its stages or TMEM are reused
-        if (!ok) bar_drain(B.acc_full, tc & 1u);
+        if (!ok) bar_drain(B.acc_full, tc & 1u, POLLS);
     } else if (warp == 2) {
         const uint32_t at = NI > kHelperLead ? gi0 + NI - kHelperLead : gi0;
         for (uint32_t it = 0; it < (1u << 20) && (int32_t)(*P.issued - at) < 0 && !*P.abort_flag; ++it) __nanosleep(64);
@@ -445,7 +458,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
         if (j < 2) {  // builders: K-steps j and j + 2 of every input stage
             uint32_t si = gi0 % IN, pi = (gi0 / IN) & 1u, pa = (gi0 & 1u) ^ 1u, left = sn;
             for (uint32_t k = 0; k < NI; ++k, left -= kInSlices) {
-                ok &= warp_wait(B.in_full + 8 * si, pi, P.abort_flag);
+                ok &= warp_wait<POLLS>(B.in_full + 8 * si, pi, P.abort_flag);
                 // one word: symbols 2m (low) and 2m+1 of a slice; past the range 0
                 const uint32_t a = in0 + kInBBytes + (32 * q + lane) * 4 + si * kInStageBytes;
                 uint32_t x[2 * kKSlices];
@@ -458,7 +471,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
 // the second K-step is spread while the first is stored
                 uint32_t v[16], w[16];
                 spread4(x, v);
-                ok &= warp_wait(B.a_empty + 8 * 0, pa, P.abort_flag);
+                ok &= warp_wait<POLLS>(B.a_empty + 8 * 0, pa, P.abort_flag);
                 tc_fence_after();
                 tmem_st16(lanes + kACol + 16 * j, v);
                 spread4(x + kKSlices, w);
@@ -466,7 +479,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) bar_arrive(B.a_full + 8 * 0);
-                ok &= warp_wait(B.a_empty + 8 * 1, pa, P.abort_flag);
+                ok &= warp_wait<POLLS>(B.a_empty + 8 * 1, pa, P.abort_flag);
                 tc_fence_after();
                 tmem_st16(lanes + kACol + 16 * (j + 2), w);
                 tmem_st_wait();
@@ -480,7 +493,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
                 }
             }
         }
-        ok &= warp_wait(B.acc_full, tc & 1u, P.abort_flag);
+        ok &= warp_wait<POLLS>(B.acc_full, tc & 1u, P.abort_flag);
         tc_fence_after();
         const uint32_t m = 2 * (32 * q + lane);  // this lane's symbols m, m+1
         const uint32_t r0 = uni(T.r0), left = uni(T.R) - r0, live = left < rows ? left : rows;
@@ -539,7 +552,7 @@ __device__ __forceinline__ bool run_tile(Pipe& P, const Tile& T, Helper&& helper
         // last stages, the next tile's first) land before the stages are
         // reused or the CTA exits
         for (uint32_t q = issued_end > gi0 + IN ? issued_end - IN : gi0; q < issued_end; ++q)
-            bar_drain(B.in_full + 8 * (q % IN), (q / IN) & 1u);
+            bar_drain(B.in_full + 8 * (q % IN), (q / IN) & 1u, POLLS);
     }
     P.gi += NI;
     P.pre = bad || !issued_end ? 0u : issued_end - gi0 - NI;

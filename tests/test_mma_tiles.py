@@ -24,6 +24,20 @@ def test_tensor_tile_edges(p2g, gpu, oracle, S, slice_, R, fe):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("slices,tiles", [(33, 1), (48, 1), (400, 300)])
+def test_tile_that_gives_up(p2g, gpu, oracle, slices, tiles):
+    """A stage that never arrives (the last one; one after which the input
+    ring wraps, with a next tile's stages asked for): every role gives up, the
+    call reports it, and the next encode is right."""
+    from par2rust_b200.workloads import file_bytes
+
+    with pytest.raises(p2g.DeviceTimeout):
+        p2g.check_tile_wait(slices, tiles)
+    src = file_bytes(slices, 40 * 1024)
+    assert np.array_equal(p2g.encode(src, 1024, 15, variant=p2g.ENCODE_TENSOR), oracle.encode_fast(src, 40, 1024, 15))
+
+
 def test_rows_of_the_multiplication_matrix_are_trace_runs():
     """Bit i of c * 2^j is Tr(2^(log c + log d_i + j)), d_i the basis dual to 1, 2, .., 2^15."""
     al = np.zeros(65535, np.int64)
