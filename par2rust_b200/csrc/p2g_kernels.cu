@@ -1909,12 +1909,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
                 mma::bar_drain(B.in_full + 8 * (q % kBatchInStages), (q / kBatchInStages) & 1u);
         }
         if ((tid >> 5) == 1) {
-            if ((tid & 31) == 0) {
-                const mma::Bars<kBatchInStages> B(mma_bars);
-                mma::mma_commit(B.drain);
-                mma::bar_drain(B.drain, 0);
-            }
-            __syncwarp();
+            mma::mma_drain(mma::Bars<kBatchInStages>(mma_bars).drain);
             mma::tc_fence_after();
             mma::tmem_free(mma_misc[0]);
         }

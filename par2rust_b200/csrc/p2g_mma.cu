@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1) encode_mma_kernel(const __grid_co
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
+        if (!st.ok) mma_drain(Bars<kInStages>(smem_addr(smem + kOffBars)).drain);
         __syncwarp();
         tc_fence_after();
         tmem_free(tmem);

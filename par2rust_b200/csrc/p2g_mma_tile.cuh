@@ -248,6 +248,20 @@ __device__ __forceinline__ void tmem_alloc(uint32_t slot) {
 __device__ __forceinline__ void tmem_free(uint32_t tmem) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
+// The lane that issues a warp's asynchronous instructions.
+__device__ __forceinline__ bool elect_one(uint32_t& leader) {
+    uint32_t p;
+    asm volatile("{\n .reg .pred P;\n elect.sync %0|P, 0xFFFFFFFF;\n selp.u32 %1, 1, 0, P;\n}" : "=r"(leader), "=r"(p));
+    return p != 0;
+}
+// Every MMA that this warp issued has completed (all lanes of the MMA warp, once
+// per launch: the barrier's first phase).
+__device__ __forceinline__ void mma_drain(uint32_t drain) {
+    uint32_t leader;
+    if (elect_one(leader)) mma_commit(drain);
+    bar_drain(drain, 0);
+    __syncwarp();
+}
 // Scale factors 1.0 (UE8M0 127) over the 32 lanes of warp quadrant q
 // (called by four warps with distinct quadrants).
 __device__ __forceinline__ void sf_fill(uint32_t tmem, uint32_t q) {
@@ -283,12 +297,6 @@ struct Pipe {
     const Tile* next;           // shared: the tile that follows, written by the helper warp (rows 0: none)
 };
 
-// The lane that issues a warp's asynchronous instructions.
-__device__ __forceinline__ bool elect_one(uint32_t& leader) {
-    uint32_t p;
-    asm volatile("{\n .reg .pred P;\n elect.sync %0|P, 0xFFFFFFFF;\n selp.u32 %1, 1, 0, P;\n}" : "=r"(leader), "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ uint32_t uni(uint32_t v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
 __device__ __forceinline__ uint64_t uni(uint64_t v) { return __shfl_sync(0xFFFFFFFFu, (unsigned long long)v, 0); }
 // Bounded wait by a whole warp: false when it gave up (it then sets the abort
@@ -309,14 +317,16 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
 // warp 1 issues the MMAs, warp 2 finds the next tile, warps 4..11 build A (warp w its lane quadrant w % 4
 // of every other K-step), and warps 4..15 run the epilogue (every third row of
 // their quadrant).  Returns false (uniformly, after a CTA barrier) when a
-// bounded wait gave up; copies and MMAs in flight have then landed.
+// bounded wait gave up; copies in flight have then landed.
 // helper: run by warp 2 when warp 0 has kHelperLead stages of this tile left to
 // issue; it writes the tile this CTA runs next to *P.next.  Warp 0 then issues
 // that tile's first input stages while this tile's last K-steps and epilogue
 // run, so the next tile starts without a copy round trip.  Only warp 0's P.pre
 // counts (the stages it issued ahead); the next call must be for that same
 // tile.  When any role's wait gives up, warp 0 issues nothing more and waits for
-// every copy it issued, the next tile's included, before this returns.
+// every copy it issued, the next tile's included, before this returns.  MMAs may
+// then still run where only another role gave up: mma_drain stands before TMEM
+// is freed (a wait for them here, after the roles, made the 538 MB job 2 % slower).
 //
 // Every role runs whole warps on values the compiler knows to be the same in
 // every lane (uni), with only the asynchronous instructions under the elected
