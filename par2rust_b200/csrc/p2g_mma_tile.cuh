@@ -301,12 +301,17 @@ __device__ __forceinline__ uint32_t uni(uint32_t v) { return __shfl_sync(0xFFFFF
 __device__ __forceinline__ uint64_t uni(uint64_t v) { return __shfl_sync(0xFFFFFFFFu, (unsigned long long)v, 0); }
 // Bounded wait by a whole warp: false when it gave up (it then sets the abort
 // flag) or when another role has given up.  The lanes vote on every poll, so
-// that the loop's branch is one for the warp.
+// that the loop's branch is one for the warp.  A failed poll takes ~8 us (the
+// instruction waits by itself), a pipeline without faults sees one or two in a
+// row: the flag is looked at after the 16th, so that a role which runs on after
+// giving up is through an unsatisfied wait in 0.13 ms instead of the 2 ms of 256
+// (a tile of 32,768 slices has 6,000 waits), and never before (after the first,
+// the 538 MB job took 1.2 % longer).
 template <uint32_t POLLS>
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
     for (uint32_t it = 0; it < POLLS; ++it) {
         if (__all_sync(0xFFFFFFFFu, bar_try_wait(bar, parity))) return true;
-        if ((it & 255u) == 255u && __any_sync(0xFFFFFFFFu, *abort_flag != 0)) return false;
+        if ((it & 255u) == 15u && __any_sync(0xFFFFFFFFu, *abort_flag != 0)) return false;
     }
     *abort_flag = 1u;
     __threadfence_block();  // before anything this role still commits or arrives at

@@ -25,15 +25,19 @@ def test_tensor_tile_edges(p2g, gpu, oracle, S, slice_, R, fe):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("slices,tiles", [(33, 1), (48, 1), (400, 300)])
+@pytest.mark.parametrize("slices,tiles", [(33, 1), (48, 1), (400, 300), (32768, 40)])
 def test_tile_that_gives_up(p2g, gpu, oracle, slices, tiles):
     """A stage that never arrives (the last one; one after which the input
-    ring wraps, with a next tile's stages asked for): every role gives up, the
-    call reports it, and the next encode is right."""
+    ring wraps, with a next tile's stages asked for; one with 2,045 behind it):
+    every role gives up, the call reports it soon, and the next encode is right."""
+    import time
+
     from par2rust_b200.workloads import file_bytes
 
+    t0 = time.time()
     with pytest.raises(p2g.DeviceTimeout):
         p2g.check_tile_wait(slices, tiles)
+    assert time.time() - t0 < 5
     src = file_bytes(slices, 40 * 1024)
     assert np.array_equal(p2g.encode(src, 1024, 15, variant=p2g.ENCODE_TENSOR), oracle.encode_fast(src, 40, 1024, 15))
 
