@@ -67,6 +67,7 @@ struct DevBuf {
         if (e == cudaSuccess) cap = want;
         return e;
     }
+    bool holds(size_t n) const { return p && n <= cap; }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
 };
@@ -148,6 +149,7 @@ static p2g_status ensure_ready(Context& c) {
         for (auto& ev : c.ev_band) P2G_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         for (auto& ev : c.ev_up) P2G_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         P2G_CU(upload_tables());
+        P2G_CU(mma_prepare());  // now, not by the first tensor-core call: that may be inside a stream capture
         P2G_CU(c.err.ensure(64));
         P2G_CU(c.h_err.ensure(64));
         c.device = dev;
@@ -222,6 +224,10 @@ static p2g_status join_into(Context& c, cudaStream_t caller) {
 // P2G_ENCODE_BASIS=derive has the encode kernel derive it (no scratch, ~6%
 // more encode time on B200: 512 extra lookups per slice in a loop that is
 // close to its issue limit).
+static bool generate_basis() {
+    const char* e = getenv("P2G_ENCODE_BASIS");
+    return e && !strcmp(e, "derive");
+}
 // Which encode kernel runs a job: the shared-memory lookup kernel or the
 // tensor-core bit-sliced one.  P2G_ENCODE_LUT / P2G_ENCODE_TENSOR (or
 // P2G_ENCODE_VARIANT=lut|tensor) force one; otherwise the planner's cost
@@ -240,9 +246,17 @@ static bool use_tensor_encode(uint32_t flags, uint32_t S, uint32_t R, uint64_t s
 // *use_tensor's case.  Where the rule alone picked the tensor cores and the
 // image does not fit the device, the lookup kernel (whose bases are a quarter
 // of it) runs instead.
+// Nothing can be allocated while a stream is captured: there a call whose
+// kernel's scratch is not in place takes the other one where that one's is (a
+// program that warmed the library up on one shape may capture another).
 static p2g_status choose_encode(Context& c, uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size,
-                                bool* use_tensor) {
+                                bool capturing, bool* use_tensor) {
     *use_tensor = use_tensor_encode(flags, S, R, slice_size, true);
+    if (capturing && !(flags & (P2G_ENCODE_TENSOR | P2G_ENCODE_LUT))) {
+        const bool image = c.aimg.holds(mma_aimg_bytes(S, R));
+        const bool bases = generate_basis() || c.basis.holds(basis_bytes(S, (R + kRowsPerGroup - 1) / kRowsPerGroup));
+        if (image != bases) *use_tensor = image;
+    }
     if (!*use_tensor) return P2G_OK;
     const cudaError_t e = c.aimg.ensure(mma_aimg_bytes(S, R));
     if (e == cudaSuccess) return P2G_OK;
@@ -254,10 +268,6 @@ static p2g_status choose_encode(Context& c, uint32_t flags, uint32_t S, uint32_t
     return cuda_fail(e, "coefficient image");
 }
 
-static bool generate_basis() {
-    const char* e = getenv("P2G_ENCODE_BASIS");
-    return e && !strcmp(e, "derive");
-}
 
 enum class FileHashMode { Device, Host };
 static double env_double(const char* name, double dflt) {
@@ -1326,7 +1336,7 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
         if (order && c.scratch_pending) P2G_CU(cudaStreamWaitEvent(s, c.ev_scratch, 0));
         P2G_CU(cudaMemsetAsync(c.err.p, 0, sizeof(int), s));
         bool tensor = false;
-        P2G_TRY(choose_encode(c, jb.flags, S, R, jb.slice_size, &tensor));
+        P2G_TRY(choose_encode(c, jb.flags, S, R, jb.slice_size, !order, &tensor));
         if (tensor) {
             P2G_CU(launch_encode_mma(jb.src, jb.src_stride, S, jb.slice_size, R, jb.first_exponent,
                                      c.aimg.as<uint8_t>(), jb.recovery, jb.recovery_stride, c.err.as<int>(), s));
@@ -1363,7 +1373,7 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
         if (stride != jb.slice_size)  // the 16-byte padding of each row is read: zero it
             P2G_CU(cudaMemset2DAsync(c.src.as<uint8_t>() + jb.slice_size, stride, 0, stride - jb.slice_size, S, s));
         bool tensor = false;
-        P2G_TRY(choose_encode(c, jb.flags, S, R, jb.slice_size, &tensor));
+        P2G_TRY(choose_encode(c, jb.flags, S, R, jb.slice_size, false, &tensor));
         if (tensor) {
             P2G_CU(launch_encode_mma(c.src.as<uint8_t>(), stride, S, jb.slice_size, R, jb.first_exponent,
                                      c.aimg.as<uint8_t>(), c.rec.as<uint8_t>(), stride, c.err.as<int>(), s));

@@ -1,0 +1,56 @@
+"""Which kernel an encode call runs on, where its first choice cannot run: inside
+a stream capture.  Each test is a process of its own, since the library keeps
+its scratch."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _run(code, **env):
+    head = """
+        import sys
+        sys.path.insert(0, %r)
+        import numpy as np, torch
+        import par2rust_b200 as p2g
+        from oracle import oracle
+        from par2rust_b200.workloads import file_bytes
+
+        def encode(src, S, size, rows, **kw):
+            rec = torch.zeros((rows, size), dtype=torch.uint8, device="cuda")
+            p2g.encode_device(src.data_ptr(), size, S, size, rows, rec.data_ptr(), size,
+                              torch.cuda.current_stream().cuda_stream, **kw)
+            return rec
+    """ % ROOT
+    r = subprocess.run([sys.executable, "-c", textwrap.dedent(head) + textwrap.dedent(code)], cwd=ROOT,
+                       env=dict(os.environ, **env), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("warm,S,size,rows", [("LUT", 64, 16384, 20), ("TENSOR", 4, 1024, 3), ("LUT", 4, 1024, 3),
+                                              ("TENSOR", 64, 16384, 20)])
+def test_capture_after_one_kernel_ran(p2g, gpu, warm, S, size, rows):
+    """A program that has only run one of the kernels captures a call of a
+    smaller shape, whichever kernel the rule would give it."""
+    _run("""
+        S, size, rows = %d, %d, %d
+        big = torch.from_numpy(file_bytes(1, 256 * 1024).copy()).cuda()
+        encode(big, 256, 1024, 200, variant=p2g.ENCODE_%s)
+        data = file_bytes(2, S * size)
+        src = torch.from_numpy(data.copy()).cuda()
+        g = torch.cuda.CUDAGraph()
+        rec = torch.zeros((rows, size), dtype=torch.uint8, device="cuda")
+        with torch.cuda.graph(g):
+            p2g.encode_device(src.data_ptr(), size, S, size, rows, rec.data_ptr(), size,
+                              torch.cuda.current_stream().cuda_stream)
+        for _ in range(2):
+            rec.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(rec.cpu().numpy().ravel(), oracle.encode_fast(data, S, size, rows))
+    """ % (S, size, rows, warm))
