@@ -750,7 +750,7 @@ extern "C" p2g_status p2g_batch_create(const p2g_batch_job* jobs, uint32_t n, ui
     // 256-job mixed launch still ran into a bounded wait (each kind alone is
     // bit-exact).
     const char* ev = getenv("P2G_ENCODE_VARIANT");
-    bool use_mma;
+    bool use_mma, by_cost = false;
     if (flags & P2G_BATCH_TENSOR) {
         use_mma = true;
     } else if (flags & P2G_BATCH_LUT) {
@@ -763,7 +763,7 @@ extern "C" p2g_status p2g_batch_create(const p2g_batch_job* jobs, uint32_t n, ui
             lut += encode_cost_ms(shape[i].slice, shape[i].S, shape[i].R, false);
             mma += encode_cost_ms(shape[i].slice, shape[i].S, shape[i].R, true);
         }
-        use_mma = mma < lut;
+        use_mma = by_cost = mma < lut;
     }
     for (uint32_t i = 0; i < n; ++i) shape[i].mma = use_mma && shape[i].R;
     P2G_TRY(ensure_device_ready());
@@ -823,6 +823,12 @@ extern "C" p2g_status p2g_batch_create(const p2g_batch_job* jobs, uint32_t n, ui
     cudaError_t e = cudaMalloc(&b->arena, off);
     if (e != cudaSuccess) {
         release(b);
+        if (e == cudaErrorMemoryAllocation && by_cost) {
+            // the coefficient images (R x S x 128 B a job) do not fit: the
+            // lookup kernel's bases take a quarter, or are derived
+            cudaGetLastError();
+            return p2g_batch_create(jobs, n, flags | P2G_BATCH_LUT, out);
+        }
         return cuda_fail(e, "batch arena");
     }
     uint8_t* A = static_cast<uint8_t*>(b->arena);

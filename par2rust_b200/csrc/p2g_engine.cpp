@@ -232,40 +232,55 @@ static bool generate_basis() {
 // tensor-core bit-sliced one.  P2G_ENCODE_LUT / P2G_ENCODE_TENSOR (or
 // P2G_ENCODE_VARIANT=lut|tensor) force one; otherwise the planner's cost
 // model picks by shape (prefer_mma, or prefer_mma_alone for an encode call).
-static bool use_tensor_encode(uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size, bool alone = false) {
-    if (flags & P2G_ENCODE_TENSOR) return true;
-    if (flags & P2G_ENCODE_LUT) return false;
+enum class Forced { No, Lut, Tensor };
+static Forced forced_encode(uint32_t flags) {
+    if (flags & P2G_ENCODE_TENSOR) return Forced::Tensor;
+    if (flags & P2G_ENCODE_LUT) return Forced::Lut;
     if (const char* e = getenv("P2G_ENCODE_VARIANT")) {
-        if (!strcmp(e, "tensor")) return true;
-        if (!strcmp(e, "lut")) return false;
+        if (!strcmp(e, "tensor")) return Forced::Tensor;
+        if (!strcmp(e, "lut")) return Forced::Lut;
     }
-    return alone ? prefer_mma_alone(slice_size, S, R) : prefer_mma(slice_size, S, R);
+    return Forced::No;
+}
+
+// Room for a coefficient image of `bytes`.  Where the rule alone picked the
+// tensor cores and the image does not fit the device (R x S x 128 B, up to four
+// times the lookup kernel's bases), `*other` is set and the lookup kernel runs
+// instead; the image held so far is kept then.
+static p2g_status ensure_image(Context& c, size_t bytes, Forced forced, bool* other) {
+    *other = false;
+    if (c.aimg.holds(bytes)) return P2G_OK;
+    size_t left = 0, total = 0;
+    P2G_CU(cudaMemGetInfo(&left, &total));
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (forced != Forced::No || left + c.aimg.cap >= bytes) e = c.aimg.ensure(bytes);
+    if (e == cudaErrorMemoryAllocation && forced == Forced::No) {
+        cudaGetLastError();
+        *other = true;
+        return P2G_OK;
+    }
+    return e == cudaSuccess ? P2G_OK : cuda_fail(e, "coefficient image");
 }
 
 // The kernel of one encode call, with room for its coefficient image in
-// *use_tensor's case.  Where the rule alone picked the tensor cores and the
-// image does not fit the device, the lookup kernel (whose bases are a quarter
-// of it) runs instead.
+// *use_tensor's case (ensure_image).
 // Nothing can be allocated while a stream is captured: there a call whose
 // kernel's scratch is not in place takes the other one where that one's is (a
 // program that warmed the library up on one shape may capture another).
 static p2g_status choose_encode(Context& c, uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size,
                                 bool capturing, bool* use_tensor) {
-    *use_tensor = use_tensor_encode(flags, S, R, slice_size, true);
-    if (capturing && !(flags & (P2G_ENCODE_TENSOR | P2G_ENCODE_LUT))) {
+    const Forced forced = forced_encode(flags);
+    *use_tensor = forced == Forced::No ? prefer_mma_alone(slice_size, S, R) : forced == Forced::Tensor;
+    if (capturing && forced == Forced::No) {
         const bool image = c.aimg.holds(mma_aimg_bytes(S, R));
         const bool bases = generate_basis() || c.basis.holds(basis_bytes(S, (R + kRowsPerGroup - 1) / kRowsPerGroup));
         if (image != bases) *use_tensor = image;
     }
     if (!*use_tensor) return P2G_OK;
-    const cudaError_t e = c.aimg.ensure(mma_aimg_bytes(S, R));
-    if (e == cudaSuccess) return P2G_OK;
-    if (e == cudaErrorMemoryAllocation && !(flags & P2G_ENCODE_TENSOR) && !prefer_mma(slice_size, S, R)) {
-        cudaGetLastError();
-        *use_tensor = false;
-        return P2G_OK;
-    }
-    return cuda_fail(e, "coefficient image");
+    bool other = false;
+    P2G_TRY(ensure_image(c, mma_aimg_bytes(S, R), forced, &other));
+    if (other) *use_tensor = false;
+    return P2G_OK;
 }
 
 
@@ -443,7 +458,9 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
         const char* e = getenv("P2G_TAIL_SPLIT");
         return !(e && !strcmp(e, "0"));
     }();
-    const bool mma = j.R && j.S && use_tensor_encode(j.variant, j.S, j.R, j.slice);
+    const Forced forced = forced_encode(j.variant);
+    const bool mma = j.R && j.S &&
+                     (forced == Forced::No ? prefer_mma(j.slice, j.S, j.R) : forced == Forced::Tensor);
     const SingleJobPlan pl = plan_single_job(j.slice, j.S, j.R && j.S ? j.R : 0, n, j.d_checks != nullptr, sid_item,
                                              chains, (uint32_t)device_sm_count(), j.d_hfull ? max_len : 0,
                                              split_tail, mma);
@@ -474,7 +491,14 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     // basis (precomputed unless P2G_ENCODE_BASIS=derive) and 16-byte aligned slices
     const bool gen = generate_basis() || mma;  // the tensor-core items read their coefficient image instead
     if (j.R && j.S && !gen) P2G_CU(c.basis.ensure(basis_bytes(j.S, RG)));
-    if (mma) P2G_CU(c.aimg.ensure(mma_aimg_bytes(j.S, j.R)));
+    if (mma) {
+        bool other = false;
+        P2G_TRY(ensure_image(c, mma_aimg_bytes(j.S, j.R), forced, &other));
+        if (other) {
+            j.variant = P2G_ENCODE_LUT;
+            return run_device_job_persistent(c, j, st);
+        }
+    }
     const uint8_t* esrc = j.d_src;
     uint64_t estride = j.slice;
     if (j.R && j.S && j.slice % 16) {

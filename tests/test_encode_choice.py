@@ -1,5 +1,5 @@
 """Which kernel an encode call runs on, where its first choice cannot run: inside
-a stream capture.  Each test is a process of its own, since the library keeps
+a stream capture, or with the device too full for the coefficient image.  Each test is a process of its own, since the library keeps
 its scratch."""
 import os
 import subprocess
@@ -54,3 +54,62 @@ def test_capture_after_one_kernel_ran(p2g, gpu, warm, S, size, rows):
             torch.cuda.synchronize()
             assert np.array_equal(rec.cpu().numpy().ravel(), oracle.encode_fast(data, S, size, rows))
     """ % (S, size, rows, warm))
+
+
+FULL = """
+    S, size, rows = 32768, 64, 512  # image 2.2 GB, bases 0.5 GB
+    data = file_bytes(2, S * size)
+    src = torch.from_numpy(np.concatenate([data, np.zeros(16, np.uint8)])).cuda()
+    bufs = p2g.DeviceJobBuffers(S, 1, size, rows, src.device)
+    want = oracle.encode_rows(data, S, size, [0, 1, 300, 511])
+    small = encode(src, 64, size, 20, variant=p2g.ENCODE_TENSOR)  # the library is up, a small image is held
+    torch.cuda.synchronize()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (1500 << 20), dtype=torch.uint8, device="cuda")
+
+    def check(rec):
+        torch.cuda.synchronize()
+        assert np.array_equal(rec.view(rows, -1)[[0, 1, 300, 511], :size].cpu().numpy(), want)
+
+    def refused(call):
+        try:
+            call()
+        except p2g.OutOfMemory:
+            return
+        raise AssertionError("accepted")
+
+    def job(**kw):
+        bufs.recovery.zero_()
+        return p2g.run_device_job(src, [S * size], [b"f"], size, rows, bufs, skip_hash_full=True, **kw).recovery
+
+    def batch(flags=0):
+        bufs.recovery.zero_()
+        b = p2g.Batch([p2g.BatchJobSpec(src, [S * size], [b"f"], size, rows, bufs)], flags)
+        b.launch()
+        torch.cuda.synchronize()
+        b.check()
+        b.close()
+        return bufs.recovery
+"""
+
+
+@pytest.mark.gpu
+def test_image_that_does_not_fit(p2g, gpu):
+    """Left to the rule, an encode, a job and a batch run on the lookup kernel
+    then; the forced tensor kernel reports that memory is short."""
+    _run(FULL + """
+    check(encode(src, S, size, rows))
+    check(job())
+    check(batch())
+    refused(lambda: encode(src, S, size, rows, variant=p2g.ENCODE_TENSOR))
+    refused(lambda: job(variant=p2g.ENCODE_TENSOR))
+    refused(lambda: batch(p2g.BATCH_TENSOR))
+    """)
+
+
+@pytest.mark.gpu
+def test_image_that_does_not_fit_forced_by_the_environment(p2g, gpu):
+    _run(FULL + """
+    refused(lambda: encode(src, S, size, rows))
+    refused(job)
+    refused(batch)
+    """, P2G_ENCODE_VARIANT="tensor")
