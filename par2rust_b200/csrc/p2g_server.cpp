@@ -598,13 +598,17 @@ extern "C" p2g_status p2g_server_submit(p2g_server* s, const p2g_server_job* rq,
     j->RG = (j->R + kRowsPerGroup - 1) / kRowsPerGroup;
     j->Np = (uint32_t)(round_up(j->slice, 16) / 2);
     j->footprint = S * j->slice + (uint64_t)j->R * round_up(j->slice, 16);
-    // tensor-core encode when the cost model prefers it and the coefficient image
-    // (R x S x 128 B) stays within a quarter of the source bytes
+    // tensor-core encode when the cost model prefers it, the coefficient image
+    // (R x S x 128 B) stays within a quarter of the source bytes, and the job
+    // with it within the budget (a job that fits it without runs on the lookup
+    // kernel, whose bases take no memory here)
     const char* ev = getenv("P2G_ENCODE_VARIANT");  // "lut" / "tensor" force a kind (tensor: if the image fits)
+    const bool forced = ev && !strcmp(ev, "tensor");
     const bool want_mma = ev && !strcmp(ev, "lut") ? false
-                          : ev && !strcmp(ev, "tensor") ? true
-                                                        : prefer_mma(j->slice, j->S, j->R);
-    if (j->R && want_mma && 4 * mma_aimg_bytes(j->S, j->R) <= S * j->slice) {
+                          : forced                 ? true
+                                                   : prefer_mma(j->slice, j->S, j->R);
+    if (j->R && want_mma && 4 * mma_aimg_bytes(j->S, j->R) <= S * j->slice &&
+        (forced || j->footprint + mma_aimg_bytes(j->S, j->R) <= s->budget)) {
         j->mma = true;
         j->aimg_bytes = mma_aimg_bytes(j->S, j->R);
         j->footprint += j->aimg_bytes;

@@ -150,3 +150,13 @@ def test_serve_rejects_bad_requests(p2g, gpu):
         srv.submit_seeded([100], [1], [b"x"], 4098, 8)
     assert srv.stats()["submitted"] == 0
     srv.close()
+
+
+def test_serve_job_that_fits_only_without_its_image(p2g, oracle, gpu):
+    """64 slices of 16 KiB, 12 rows: 1,245,184 bytes, and a coefficient image of
+    98,304 more on the tensor cores.  A budget between the two takes the job."""
+    job = (11, ([64 * 16384 - 9], 16384, 12))
+    assert _footprint(*job[1]) == 1_245_184
+    outs, _, stats = _serve(p2g, [job], 1_300_000)
+    assert stats["peak_resident_bytes"] <= 1_300_000
+    assert outs[11] == _expected(oracle, *((11,) + job[1]))
