@@ -269,6 +269,10 @@ typedef struct p2g_encode_job {
     void *stream;
 } p2g_encode_job;
 p2g_status p2g_encode(const p2g_encode_job *job);
+/* The kernel that p2g_encode picks by shape on a GPU of `ctas` SMs (host
+ * only): P2G_ENCODE_LUT or P2G_ENCODE_TENSOR in *variant. */
+p2g_status p2g_plan_encode(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count, uint32_t ctas,
+                           uint32_t *variant);
 
 /* p2g_encode without any allocation by the library.  No counterpart in the
  * reference: it exists for callers that must own all device memory (a

@@ -756,6 +756,14 @@ def plan_device_job(slice_size: int, input_slices: int, recovery_count: int, fil
     return items, z.value, nb.value
 
 
+def plan_encode(slice_size: int, input_slices: int, recovery_count: int, ctas: int = 148) -> int:
+    """ENCODE_LUT or ENCODE_TENSOR: the kernel that encode and encode_device
+    pick for a shape on a GPU of ``ctas`` SMs (host only)."""
+    v = C.c_uint32()
+    _check(lib().p2g_plan_encode(slice_size, input_slices, recovery_count, ctas, C.byref(v)))
+    return v.value
+
+
 class StagedBatch:
     """Batched create for jobs whose sources sit in pinned host memory.
 

@@ -280,6 +280,7 @@ SIGNATURES = [
     ("p2g_encode_noalloc", C.c_int, [C.POINTER(p2g_encode_job)]),
     ("p2g_check_bounded_wait", C.c_int, [C.c_uint32]),
     ("p2g_check_tile_wait", C.c_int, [C.c_uint32, C.c_uint32]),
+    ("p2g_plan_encode", C.c_int, [C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p]),
     ("p2g_plan_device_job", C.c_int,
      [C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p, C.c_uint32,
       C.POINTER(C.c_uint32), C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),

@@ -103,7 +103,6 @@ struct Plan {
 constexpr uint32_t kMaxBands = 64;  // packet-MD5 chain segments per job (64: 10.27 ms vs 10.59 at 16 for 538 MB / R 200)
 
 constexpr uint32_t kMaxMmaBands = 72;
-constexpr double kMaxCtas = 148;  // SMs of a B200
 
 // Bands of job j: runs of band_tiles consecutive tiles, a multiple of the
 // tail fold so that no folded item straddles two bands.  Tensor-core bands are
@@ -441,9 +440,9 @@ bool prefer_mma(uint64_t slice, uint32_t S, uint32_t R) {
 // for two within 14 %: 4 KiB x 1,024 x 1 takes 773 us on the lookup kernel and
 // 39 on the tensor cores, 256 KiB x 64 x 32 72 and 54, 1 MiB x 16 x 100 179
 // and 303.
-bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R) {
+bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R, uint32_t sms) {
     if (!R || S <= 6) return false;  // a few slices: the lookup kernel, or a tie
-    const uint32_t Np = (uint32_t)(round_up(slice, 16) / 2), sms = (uint32_t)kMaxCtas;
+    const uint32_t Np = (uint32_t)(round_up(slice, 16) / 2);
     const uint32_t rows = mma_rows(R), RT = mma_row_tiles(R);
     const uint64_t tiles = (uint64_t)((Np + kMmaTileSymbols - 1) / kMmaTileSymbols) * RT;
     const double mma = 8.0 + (double)((tiles + sms - 1) / sms) *
@@ -668,6 +667,16 @@ extern "C" p2g_status p2g_plan_device_job(uint64_t slice_size, uint32_t input_sl
     if (n_items) *n_items = n;
     if (zero_from_symbol) *zero_from_symbol = pl.zero_from_sym;
     if (band_count) *band_count = (uint32_t)pl.band_items.size();
+    return P2G_OK;
+}
+
+extern "C" p2g_status p2g_plan_encode(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count,
+                                      uint32_t ctas, uint32_t* variant) {
+    clear_error();
+    if (!ctas || !variant || input_slices > P2G_MAX_INPUT_BLOCKS)
+        return set_error(P2G_ERR_INVALID_ARGUMENT, "plan needs ctas > 0, up to 32768 input slices and a result");
+    P2G_TRY(check_common(1, recovery_count, slice_size));
+    *variant = prefer_mma_alone(slice_size, input_slices, recovery_count, ctas) ? P2G_ENCODE_TENSOR : P2G_ENCODE_LUT;
     return P2G_OK;
 }
 

@@ -270,7 +270,7 @@ static p2g_status ensure_image(Context& c, size_t bytes, Forced forced, bool* ot
 static p2g_status choose_encode(Context& c, uint32_t flags, uint32_t S, uint32_t R, uint64_t slice_size,
                                 bool capturing, bool* use_tensor) {
     const Forced forced = forced_encode(flags);
-    *use_tensor = forced == Forced::No ? prefer_mma_alone(slice_size, S, R) : forced == Forced::Tensor;
+    *use_tensor = forced == Forced::No ? prefer_mma_alone(slice_size, S, R, (uint32_t)device_sm_count()) : forced == Forced::Tensor;
     if (capturing && forced == Forced::No) {
         const bool image = c.aimg.holds(mma_aimg_bytes(S, R));
         const bool bases = generate_basis() || c.basis.holds(basis_bytes(S, (R + kRowsPerGroup - 1) / kRowsPerGroup));

@@ -294,8 +294,8 @@ double est_mma_item_ms(uint32_t slices, uint32_t rows);
 // (cost model), and whether the tensor cores are the cheaper.
 double encode_cost_ms(uint64_t slice, uint32_t S, uint32_t R, bool mma);
 bool prefer_mma(uint64_t slice, uint32_t S, uint32_t R);
-// The same for an encode with the GPU to itself (p2g_encode).
-bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R);
+// The same for an encode with the GPU, of `sms` SMs, to itself (p2g_encode).
+bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R, uint32_t sms);
 double est_scan_item_ms(uint64_t slice, uint32_t count);
 double est_crc_item_ms(uint64_t slice, uint32_t count);
 // slices per CRC item: ~kCrcItemBytes, at least 1, at most kCrcMaxSlices

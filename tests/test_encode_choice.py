@@ -1,6 +1,7 @@
-"""Which kernel an encode call runs on, where its first choice cannot run: inside
-a stream capture, or with the device too full for the coefficient image.  Each test is a process of its own, since the library keeps
-its scratch."""
+"""Which kernel an encode call runs on: the rule by shape (CPU), and where its
+first choice cannot run (GPU): inside a stream capture, or with the device too
+full for the coefficient image.  Each GPU test is a process of its own, since
+the library keeps its scratch."""
 import os
 import subprocess
 import sys
@@ -29,6 +30,13 @@ def _run(code, **env):
     r = subprocess.run([sys.executable, "-c", textwrap.dedent(head) + textwrap.dedent(code)], cwd=ROOT,
                        env=dict(os.environ, **env), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_rule_counts_the_waves_of_the_given_gpu(p2g):
+    """16 slices of 64 KiB, 32 rows: 384 tensor tiles, 3 waves of 148 SMs and 6
+    of 64, against one wave of lookup tiles."""
+    assert p2g.plan_encode(65536, 16, 32, ctas=148) == p2g.ENCODE_TENSOR
+    assert p2g.plan_encode(65536, 16, 32, ctas=64) == p2g.ENCODE_LUT
 
 
 @pytest.mark.gpu
