@@ -449,10 +449,13 @@ bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R, uint32_t sms) {
                                  (mma_image_steps(S) * std::max(212.0, 17.6 * rows) + 3600.0) / 1900.0 +
                        (double)RT * rows * S * 128.0 / 3.0e6;
     const uint32_t RG = (R + kRowsPerGroup - 1) / kRowsPerGroup, fold = tail_fold(R);
-    uint32_t ts = 0, n = 0;
-    choose_tiles(Np, RG, sms, &ts, &n, fold);
-    const uint64_t ctas = (uint64_t)n * (RG - 1) + (n + fold - 1) / fold;
-    const double lut = 6.0 + (double)((ctas + sms - 1) / sms) * S * (ts + kBuildCost) / (kEncRate / 1000.0);
+    // the lookup kernel's fewest waves, cut into as many tiles as fill them, up
+    // to choose_tiles' most; its loop over tile counts cost 8 us a call at 1 MiB
+    // slices (1 MiB x 8 x 1: 27.8 us instead of 19.5), 450 at 64 MiB
+    const uint64_t tmin = (Np + kEncTileSymbols - 1) / kEncTileSymbols;
+    const uint64_t waves = (tmin * (RG - 1) + (tmin + fold - 1) / fold + sms - 1) / sms;
+    const uint64_t fill = std::min(4 * tmin + 8, std::max(tmin, waves * sms * fold / ((RG - 1) * fold + 1)));
+    const double lut = 6.0 + (double)waves * S * ((Np + fill - 1) / fill + kBuildCost) / (kEncRate / 1000.0);
     return mma < lut;
 }
 double est_encode_item_ms(uint32_t slices, uint32_t syms) {

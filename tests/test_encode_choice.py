@@ -6,6 +6,7 @@ import os
 import subprocess
 import sys
 import textwrap
+import time
 
 import pytest
 
@@ -37,6 +38,15 @@ def test_rule_counts_the_waves_of_the_given_gpu(p2g):
     of 64, against one wave of lookup tiles."""
     assert p2g.plan_encode(65536, 16, 32, ctas=148) == p2g.ENCODE_TENSOR
     assert p2g.plan_encode(65536, 16, 32, ctas=64) == p2g.ENCODE_LUT
+
+
+def test_rule_costs_little_for_long_slices(p2g):
+    """It runs on every encode call, whose launches take ~15 us."""
+    p2g.plan_encode(64 << 20, 8, 4)
+    t = time.perf_counter()
+    for _ in range(200):
+        p2g.plan_encode(64 << 20, 8, 4)
+    assert (time.perf_counter() - t) / 200 < 20e-6
 
 
 @pytest.mark.gpu
