@@ -435,18 +435,19 @@ bool prefer_mma(uint64_t slice, uint32_t S, uint32_t R) {
 // An encode alone on the GPU ends with its last wave, not with its work: the
 // tiles of either kernel in whole waves of SMs, each tile's steps and fixed
 // part, the launches and, on the tensor cores, the coefficient image at ~3
-// TB/s.  Against the two kernels timed over 266 shapes (slices 4 KiB..1 MiB, 4
-// to 1,024 of them, 1 to 200 rows) this picks the faster or one within 1 %, but
-// for two within 14 %: 4 KiB x 1,024 x 1 takes 773 us on the lookup kernel and
-// 39 on the tensor cores, 256 KiB x 64 x 32 72 and 54, 1 MiB x 16 x 100 179
-// and 303.
+// TB/s.  Against the two kernels timed over 885 shapes (slices 256 B..1 MiB, 1 to
+// 1,024 of them, 1 to 200 rows) it picks one more than 3 % slower 14 times, by
+// 10 % at most; over 415 drawn ones, which the constants were not fitted to, 3
+// times (two within 5 %, one of 12 us by 20 %).  4 KiB x 1,024 x 1 takes 771 us
+// on the lookup kernel and 39 on the tensor cores, 256 KiB x 32 x 32 43 and 37,
+// 1 MiB x 16 x 100 179 and 258.
 bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R, uint32_t sms) {
-    if (!R || S <= 6) return false;  // a few slices: the lookup kernel, or a tie
+    if (!R || S <= 3) return false;  // a tie: the lookup kernel
     const uint32_t Np = (uint32_t)(round_up(slice, 16) / 2);
     const uint32_t rows = mma_rows(R), RT = mma_row_tiles(R);
     const uint64_t tiles = (uint64_t)((Np + kMmaTileSymbols - 1) / kMmaTileSymbols) * RT;
-    const double mma = 8.0 + (double)((tiles + sms - 1) / sms) *
-                                 (mma_image_steps(S) * std::max(212.0, 17.6 * rows) + 3600.0) / 1900.0 +
+    const double mma = 6.0 + (double)((tiles + sms - 1) / sms) *
+                                 (mma_image_steps(S) * std::max(212.0, 17.6 * rows) + 2500.0) / 1900.0 +
                        (double)RT * rows * S * 128.0 / 3.0e6;
     const uint32_t RG = (R + kRowsPerGroup - 1) / kRowsPerGroup, fold = tail_fold(R);
     // the lookup kernel's fewest waves, cut into as many tiles as fill them, up
@@ -455,7 +456,7 @@ bool prefer_mma_alone(uint64_t slice, uint32_t S, uint32_t R, uint32_t sms) {
     const uint64_t tmin = (Np + kEncTileSymbols - 1) / kEncTileSymbols;
     const uint64_t waves = (tmin * (RG - 1) + (tmin + fold - 1) / fold + sms - 1) / sms;
     const uint64_t fill = std::min(4 * tmin + 8, std::max(tmin, waves * sms * fold / ((RG - 1) * fold + 1)));
-    const double lut = 6.0 + (double)waves * S * ((Np + fill - 1) / fill + kBuildCost) / (kEncRate / 1000.0);
+    const double lut = 5.0 + (double)waves * S * ((Np + fill - 1) / fill + kBuildCost) / (kEncRate / 1000.0);
     return mma < lut;
 }
 double est_encode_item_ms(uint32_t slices, uint32_t syms) {

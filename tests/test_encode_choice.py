@@ -34,10 +34,25 @@ def _run(code, **env):
 
 
 def test_rule_counts_the_waves_of_the_given_gpu(p2g):
-    """16 slices of 64 KiB, 32 rows: 384 tensor tiles, 3 waves of 148 SMs and 6
+    """32 slices of 1 MiB, 4 rows: 2,048 tensor tiles, 14 waves of 148 SMs and 32
     of 64, against one wave of lookup tiles."""
-    assert p2g.plan_encode(65536, 16, 32, ctas=148) == p2g.ENCODE_TENSOR
-    assert p2g.plan_encode(65536, 16, 32, ctas=64) == p2g.ENCODE_LUT
+    assert p2g.plan_encode(1 << 20, 32, 4, ctas=148) == p2g.ENCODE_TENSOR
+    assert p2g.plan_encode(1 << 20, 32, 4, ctas=64) == p2g.ENCODE_LUT
+
+
+# (slice, slices, rows, us on the lookup kernel, us on the tensor cores), one B200
+MEASURED = [
+    (100016, 8, 2, 16.3, 11.4), (1048576, 32, 2, 42.6, 34.5), (262144, 32, 32, 42.6, 36.9),
+    (1048576, 16, 100, 179.2, 258.0), (4096, 1024, 1, 771.2, 38.6), (1048576, 7, 2, 18.2, 28.3),
+    (65536, 8, 20, 16.3, 14.3), (1048576, 8, 8, 20.3, 34.8), (262144, 64, 32, 72.8, 49.4),
+    (262144, 32, 100, 95.6, 86.3), (65536, 64, 8, 60.9, 14.6), (1048576, 8, 50, 65.3, 133.1),
+    (16384, 8, 100, 16.4, 14.6),
+]
+
+
+@pytest.mark.parametrize("size,S,rows,lut,mma", MEASURED)
+def test_rule_picks_the_kernel_that_is_faster(p2g, size, S, rows, lut, mma):
+    assert p2g.plan_encode(size, S, rows) == (p2g.ENCODE_LUT if lut < mma else p2g.ENCODE_TENSOR)
 
 
 def test_rule_costs_little_for_long_slices(p2g):
