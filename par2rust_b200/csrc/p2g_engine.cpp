@@ -1216,12 +1216,15 @@ extern "C" p2g_status p2g_check_tile_wait(uint32_t input_slices, uint32_t tiles)
 // Page-locked sources and small ones go by cudaMemcpyAsync.  The segments are
 // in ascending order of dst; bytes between them are left undefined.  The call
 // ends with its stream synchronised, so the slots are free for the next one.
+// A NULL source is refused as the driver's copy refuses it.
 struct UploadSeg {
     const uint8_t* src;
     uint64_t dst, len;
 };
 static p2g_status upload_host(Context& c, uint8_t* dst, const std::vector<UploadSeg>& seg, cudaStream_t s) {
     if (seg.empty()) return P2G_OK;
+    for (const UploadSeg& g : seg)
+        if (!g.src) return cuda_fail(cudaErrorInvalidValue, "NULL source");
     const uint64_t total = seg.back().dst + seg.back().len;
     bool staged = seg.size() > 1 ? total >= kUploadMin / 4 : total >= kUploadMin;
     for (size_t i = 0; staged && i < seg.size(); ++i) {
@@ -1272,6 +1275,7 @@ static p2g_status upload_host(Context& c, uint8_t* dst, const std::vector<Upload
 // `count` rows of `len` bytes, src_stride apart, to rows dst_stride apart.
 static p2g_status upload_rows(Context& c, uint8_t* dst, uint64_t dst_stride, const uint8_t* src, uint64_t src_stride,
                               uint64_t len, uint32_t count, cudaStream_t s) {
+    if (!src) return cuda_fail(cudaErrorInvalidValue, "NULL source");
     if (len * count < kUploadMin) {
         P2G_CU(cudaMemcpy2DAsync(dst, dst_stride, src, src_stride, len, count, cudaMemcpyHostToDevice, s));
         return P2G_OK;

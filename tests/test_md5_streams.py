@@ -124,3 +124,20 @@ def test_staged_host_uploads(p2g, gpu, oracle):
     S, size, R = 130, 16388, 3  # 16,400-byte rows on the device
     src = rng.integers(0, 256, S * size, dtype=np.uint8)
     assert np.array_equal(p2g.encode(src, size, R), oracle.encode_fast(src, S, size, R))
+
+
+@pytest.mark.parametrize("size", [4096, 1 << 20])  # the driver's copy, the staged one
+def test_null_host_buffers_are_refused(p2g, gpu, size):
+    out, one = (C.c_uint8 * 4096)(), C.create_string_buffer(size)
+    lib, lens = p2g.lib(), (C.c_uint64 * 2)(size, size)
+    files = (C.c_void_p * 2)(C.addressof(one), None)
+    job = p2g._ffi.p2g_encode_job(src=None, src_stride=size, input_count=2, slice_size=size, recovery_count=1,
+                                  first_exponent=0, recovery=C.addressof(one), recovery_stride=size,
+                                  flags=p2g.HOST_POINTERS, stream=None)
+    calls = [lambda: lib.p2g_slice_checksums(None, size, 2, size, out, p2g.HOST_POINTERS, None),
+             lambda: lib.p2g_recovery_packet_md5(bytes(16), None, size, 2, size, 0, out, p2g.HOST_POINTERS, None),
+             lambda: lib.p2g_file_hashes(files, lens, 2, out, out, p2g.HOST_POINTERS, None),
+             lambda: lib.p2g_encode(C.byref(job))]
+    for call in calls:
+        with pytest.raises(p2g.CudaError):
+            p2g._check(call())
