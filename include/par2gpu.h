@@ -436,10 +436,10 @@ p2g_status p2g_batch_plan(const p2g_batch_shape *shapes, uint32_t n, uint32_t ct
  * turns the tail split off here as it does for the job, and the encode
  * kernel is chosen as for the job (P2G_ENCODE_VARIANT, else by shape).  Lookup
  * kernel items cover 32-row groups (fold 1, 2 or 4 for a short last group);
- * tensor-core plans are reported in the planner's units of 16 rows by at
- * most 240 symbols, with fold 0 (the kernel's tiles, of up to 13 rows by 256
- * symbols, cover the units of one band and slice range).  It returns up to `cap` encode items as (row group, fold,
- * first symbol, symbols, band, first slice, slice count, accumulate), the
+ * the tiles of tensor-core plans are reported as the units of 16 rows by at
+ * most 240 symbols of a band and slice range that they cover, with fold 0
+ * (p2g_plan_device_queue lists the tiles themselves, of up to 13 rows by 256
+ * symbols).  It returns up to `cap` encode items as (row group, fold, first symbol, symbols, band, first slice, slice count, accumulate), the
  * number of encode items, and the first symbol of the columns that are
  * zeroed for accumulating items (the padded row width when there are none).
  * `with_chains` plans packet-MD5 chains as the job with packet MD5s does. */
@@ -450,6 +450,28 @@ p2g_status p2g_plan_device_job(uint64_t slice_size, uint32_t input_slices, uint3
                                uint32_t file_count, uint32_t with_chains, uint32_t ctas,
                                p2g_plan_item *items, uint32_t cap, uint32_t *n_items,
                                uint32_t *zero_from_symbol, uint32_t *band_count);
+/* The same plan as it is queued: up to `cap` items in the order in which the
+ * GPU's CTAs take them, their number, the encode items that each of up to
+ * `band_cap` bands counts, the number of bands, and the time the planner expects. */
+enum {
+    P2G_ITEM_SCAN = 0,          /* slice MD5 */
+    P2G_ITEM_ENCODE = 1,        /* lookup kernel tile */
+    P2G_ITEM_SET_ID = 3,
+    P2G_ITEM_CRC = 5,
+    P2G_ITEM_ENCODE_TENSOR = 7, /* tensor-core tile */
+    P2G_ITEM_CHAIN = 8          /* packet-MD5 chains of a block of rows, held by one CTA */
+};
+typedef struct p2g_queue_item {
+    uint32_t kind;
+    uint32_t row, rows;    /* encode and chain items */
+    uint32_t first, count; /* encode: symbols; scan and CRC32: slices */
+    uint32_t band, first_slice, slices, accumulate; /* encode */
+} p2g_queue_item;
+p2g_status p2g_plan_device_queue(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count,
+                                 uint32_t file_count, uint32_t with_chains, uint32_t ctas,
+                                 p2g_queue_item *items, uint32_t cap, uint32_t *n_items,
+                                 uint32_t *band_items, uint32_t band_cap, uint32_t *n_bands,
+                                 double *predicted_ms);
 
 /* ---- serving loop (no counterpart in par2rust, which runs one create at
  * a time) ------------------------------------------------------------------

@@ -740,10 +740,11 @@ def staged_groups(sizes: Sequence[int], groups: int) -> List[Tuple[int, int]]:
 
 def plan_device_job(slice_size: int, input_slices: int, recovery_count: int, file_count: int = 1,
                     with_chains: bool = True, ctas: int = 148):
-    """The encode items p2g_run_device_job would run (host-only planner):
-    returns (items, zero_from_symbol, bands); each item is a dict with
+    """The encode work of the queue p2g_run_device_job would run (host-only
+    planner): returns (items, zero_from_symbol, bands); each item is a dict with
     row_group, fold, first_symbol, symbols, band, first_slice, slices and
-    accumulate."""
+    accumulate.  Lookup items are those of the queue; tensor-core tiles are
+    given as the units of 16 rows x 240 symbols that they cover (fold 0)."""
     n = C.c_uint32()
     z = C.c_uint32()
     nb = C.c_uint32()
@@ -754,6 +755,26 @@ def plan_device_job(slice_size: int, input_slices: int, recovery_count: int, fil
                                      C.cast(arr, C.c_void_p), n.value, C.byref(n), C.byref(z), C.byref(nb)))
     items = [{f: getattr(arr[i], f) for f, _ in _ffi.p2g_plan_item._fields_} for i in range(n.value)]
     return items, z.value, nb.value
+
+
+ITEM_SCAN, ITEM_ENCODE, ITEM_SET_ID, ITEM_CRC, ITEM_ENCODE_TENSOR, ITEM_CHAIN = 0, 1, 3, 5, 7, 8
+
+
+def plan_device_queue(slice_size: int, input_slices: int, recovery_count: int, file_count: int = 1,
+                      with_chains: bool = True, ctas: int = 148):
+    """The queue of the same plan, item by item: returns (items, band_items,
+    predicted_ms).  Each item is a dict with kind (ITEM_*), row and rows, first
+    and count (symbols, or slices of a scan or CRC32 item), band, first_slice,
+    slices and accumulate; band_items are the encode items each band counts."""
+    n, nb, ms = C.c_uint32(), C.c_uint32(), C.c_double()
+    args = (slice_size, input_slices, recovery_count, file_count, int(with_chains), ctas)
+    _check(lib().p2g_plan_device_queue(*args, None, 0, C.byref(n), None, 0, C.byref(nb), C.byref(ms)))
+    arr = (_ffi.p2g_queue_item * max(n.value, 1))()
+    bands = (C.c_uint32 * max(nb.value, 1))()
+    _check(lib().p2g_plan_device_queue(*args, C.addressof(arr), n.value, C.byref(n), C.addressof(bands), nb.value,
+                                       C.byref(nb), C.byref(ms)))
+    items = [{f: getattr(arr[i], f) for f, _ in _ffi.p2g_queue_item._fields_} for i in range(n.value)]
+    return items, list(bands[:nb.value]), ms.value
 
 
 def plan_encode(slice_size: int, input_slices: int, recovery_count: int, ctas: int = 148) -> int:

@@ -99,6 +99,12 @@ class p2g_plan_item(C.Structure):
                 ("band", C.c_uint32), ("first_slice", C.c_uint32), ("slices", C.c_uint32), ("accumulate", C.c_uint32)]
 
 
+class p2g_queue_item(C.Structure):
+    _fields_ = [("kind", C.c_uint32), ("row", C.c_uint32), ("rows", C.c_uint32), ("first", C.c_uint32),
+                ("count", C.c_uint32), ("band", C.c_uint32), ("first_slice", C.c_uint32), ("slices", C.c_uint32),
+                ("accumulate", C.c_uint32)]
+
+
 class p2g_output_file(C.Structure):
     _fields_ = [("name", C.c_char_p), ("data", C.POINTER(C.c_uint8)), ("length", C.c_uint64)]
 
@@ -284,6 +290,9 @@ SIGNATURES = [
     ("p2g_plan_device_job", C.c_int,
      [C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p, C.c_uint32,
       C.POINTER(C.c_uint32), C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),
+    ("p2g_plan_device_queue", C.c_int,
+     [C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_void_p, C.c_uint32,
+      C.POINTER(C.c_uint32), C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32), C.POINTER(C.c_double)]),
     ("p2g_slice_checksums", C.c_int,
      [C.c_void_p, C.c_uint64, C.c_uint32, C.c_uint64, C.c_void_p, C.c_uint32, C.c_void_p]),
     ("p2g_file_hashes", C.c_int,

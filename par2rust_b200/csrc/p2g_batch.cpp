@@ -70,10 +70,10 @@ struct PlanJob {
     // into split_chunks slice ranges that XOR-accumulate into the rows.
     // split_chunks 0: the caller does not zero, never split.
     uint32_t split_bands = 0, split_chunks = 0;
-    // Encode on the tensor cores (kItemEncodeMma).  Bands and slice ranges are
-    // cut in units of 240 symbols (ts) x 16 rows (RG counts them), which
-    // p2g_plan_device_job reports; the items are the kernel's tiles of
-    // mma_rows(R) rows x 256 symbols of a band.
+    // Encode on the tensor cores (kItemEncodeMma).  Bands are cut in units of 240
+    // symbols (ts; RG counts 16-row units), which p2g_plan_device_job reports;
+    // the items are the kernel's tiles of mma_rows(R) rows x 256 symbols of a
+    // band (p2g_plan_device_queue).
     bool mma = false;
     uint32_t scan_slices = kScanSlices;  // slices per scan item
     bool lone = false;                   // the launch's only job: may have chain items
@@ -540,9 +540,7 @@ SingleJobPlan plan_single_job_uncached(uint64_t slice, uint32_t S, uint32_t R, u
     if (jobs[0].split_chunks > 1 && jobs[0].split_bands) {
         const uint32_t nb = (uint32_t)p.band_items[0].size();
         out.zero_from_sym = (nb - std::min(nb, jobs[0].split_bands)) * p.band_syms[0];
-        out.split_slices = slice_range(jobs[0], jobs[0].split_chunks);
     }
-    out.mma = jobs[0].mma;
     out.items = std::move(p.items);
     out.band_items = p.band_items[0];
     out.band_syms = p.band_syms[0];
@@ -624,17 +622,12 @@ void fill_info(const p2g_batch* b, p2g_batch_info* out) {
 
 using namespace p2g;
 
-extern "C" p2g_status p2g_plan_device_job(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count,
-                                          uint32_t file_count, uint32_t with_chains, uint32_t ctas,
-                                          p2g_plan_item* items, uint32_t cap, uint32_t* n_items,
-                                          uint32_t* zero_from_symbol, uint32_t* band_count) {
-    clear_error();
-    if (!ctas || !input_slices || input_slices > P2G_MAX_INPUT_BLOCKS || (cap && !items))
-        return set_error(P2G_ERR_INVALID_ARGUMENT, "plan needs ctas > 0, 1..32768 input slices and an item array");
+// The plan of one device job as run_device_job_persistent makes it, with device
+// slice checksums, a device set id and hash_full off the device;
+// P2G_TAIL_SPLIT=0 turns the tail split off there and here alike.
+static p2g_status plan_for_report(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count,
+                                  uint32_t file_count, bool with_chains, uint32_t ctas, SingleJobPlan* out) {
     P2G_TRY(check_common(std::max(1u, file_count), recovery_count, slice_size));
-    // as run_device_job_persistent plans a job with device slice checksums, a
-    // device set id and hash_full off the device; P2G_TAIL_SPLIT=0 turns the
-    // tail split off there and here alike
     const char* ts = getenv("P2G_TAIL_SPLIT");
     const bool split_tail = !(ts && !strcmp(ts, "0"));
     // the encode kernel the job would use (P2G_ENCODE_VARIANT, else the cost model)
@@ -642,35 +635,101 @@ extern "C" p2g_status p2g_plan_device_job(uint64_t slice_size, uint32_t input_sl
     const bool mma = ev && !strcmp(ev, "tensor") ? true
                      : ev && !strcmp(ev, "lut")  ? false
                                                  : prefer_mma(slice_size, input_slices, recovery_count);
-    const SingleJobPlan pl = plan_single_job(slice_size, input_slices, recovery_count, std::max(1u, file_count),
-                                             true, true, with_chains && recovery_count, ctas, 0, split_tail,
-                                             mma && recovery_count);
+    *out = plan_single_job(slice_size, input_slices, recovery_count, std::max(1u, file_count), true, true,
+                           with_chains && recovery_count, ctas, 0, split_tail, mma && recovery_count);
+    return P2G_OK;
+}
+
+extern "C" p2g_status p2g_plan_device_job(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count,
+                                          uint32_t file_count, uint32_t with_chains, uint32_t ctas,
+                                          p2g_plan_item* items, uint32_t cap, uint32_t* n_items,
+                                          uint32_t* zero_from_symbol, uint32_t* band_count) {
+    clear_error();
+    if (!ctas || !input_slices || input_slices > P2G_MAX_INPUT_BLOCKS || (cap && !items))
+        return set_error(P2G_ERR_INVALID_ARGUMENT, "plan needs ctas > 0, 1..32768 input slices and an item array");
+    SingleJobPlan pl;
+    P2G_TRY(plan_for_report(slice_size, input_slices, recovery_count, file_count, with_chains != 0, ctas, &pl));
+    const uint32_t Np = (uint32_t)(round_up(slice_size, 16) / 2), R = recovery_count, mrows = mma_rows(R);
+    // Tensor-core tiles, of other sizes, are reported in units of 16 rows x 240
+    // symbols of a band and slice range.  A unit is reported as often as the
+    // queued tiles cover it; one that they cover in part is not.
+    struct Piece {
+        uint32_t n0, rg, s0, sn, band, acc;
+        uint64_t cells;
+        auto unit() const { return std::tie(n0, rg, s0, sn, band, acc); }
+    };
+    std::vector<Piece> pieces;
     uint32_t n = 0;
-    if (pl.mma) {
-        // tensor-core plans are reported in the planner's units of 16 rows x
-        // 240 symbols of a band and slice range, which the kernel's tiles cover
-        const uint32_t Np = (uint32_t)(round_up(slice_size, 16) / 2);
-        const uint32_t RG = (recovery_count + kMmaUnitRows - 1) / kMmaUnitRows;
-        for (uint32_t n0 = 0; n0 < Np; n0 += kMmaUnitSymbols)
-            for (uint32_t rg = 0; rg < RG; ++rg)
-                for (uint32_t s0 = 0, cs = n0 >= pl.zero_from_sym ? pl.split_slices : input_slices; s0 < input_slices;
-                     s0 += cs, ++n)
-                    if (n < cap)
-                        items[n] = {rg, 0u, n0, std::min(kMmaUnitSymbols, Np - n0),
-                                    pl.band_syms ? n0 / pl.band_syms : 0u, s0, std::min(cs, input_slices - s0),
-                                    cs < input_slices ? 1u : 0u};
-    }
-    for (const BatchItem& it : pl.items) {
-        if ((it.kind_rg & kItemKindMask) != kItemEncode) continue;
-        if (n < cap)
-            items[n] = {(it.kind_rg >> 8) & 0xFFFFu, 1u << ((it.kind_rg >> 24) & 3u),
-                        it.a, it.b & 0xFFFFu, it.b >> 16, it.s0, it.sn ? it.sn : input_slices,
-                        (it.kind_rg & kItemAccumulate) ? 1u : 0u};
+    auto put = [&](const p2g_plan_item& it) {
+        if (n < cap) items[n] = it;
         ++n;
+    };
+    for (const BatchItem& it : pl.items) {
+        const uint32_t kind = it.kind_rg & kItemKindMask, at = (it.kind_rg >> 8) & 0xFFFFu, syms = it.b & 0xFFFFu;
+        const uint32_t acc = (it.kind_rg & kItemAccumulate) ? 1u : 0u, sn = it.sn ? it.sn : input_slices;
+        if (kind == kItemEncode)
+            put({at, 1u << ((it.kind_rg >> 24) & 3u), it.a, syms, it.b >> 16, it.s0, sn, acc});
+        if (kind != kItemEncodeMma) continue;
+        const uint32_t r0 = at * mrows, r1 = std::min(R, r0 + mrows), n1 = it.a + syms;
+        for (uint32_t u = it.a / kMmaUnitSymbols * kMmaUnitSymbols; u < n1; u += kMmaUnitSymbols)
+            for (uint32_t g = r0 / kMmaUnitRows; g * kMmaUnitRows < r1; ++g)
+                pieces.push_back({u, g, it.s0, sn, it.b >> 16, acc,
+                                  (uint64_t)(std::min(n1, u + kMmaUnitSymbols) - std::max(it.a, u)) *
+                                      (std::min(r1, (g + 1) * kMmaUnitRows) - std::max(r0, g * kMmaUnitRows))});
+    }
+    std::sort(pieces.begin(), pieces.end(), [](const Piece& a, const Piece& b) { return a.unit() < b.unit(); });
+    for (size_t i = 0; i < pieces.size();) {
+        const Piece& p = pieces[i];
+        const uint32_t syms = std::min(kMmaUnitSymbols, Np - p.n0);
+        const uint64_t whole = (uint64_t)syms * std::min(kMmaUnitRows, R - p.rg * kMmaUnitRows);
+        uint64_t cells = 0;
+        for (; i < pieces.size() && pieces[i].unit() == p.unit(); ++i) cells += pieces[i].cells;
+        for (; cells >= whole && cells % whole == 0; cells -= whole)
+            put({p.rg, 0u, p.n0, syms, p.band, p.s0, p.sn, p.acc});
     }
     if (n_items) *n_items = n;
     if (zero_from_symbol) *zero_from_symbol = pl.zero_from_sym;
     if (band_count) *band_count = (uint32_t)pl.band_items.size();
+    return P2G_OK;
+}
+
+static_assert((int)P2G_ITEM_SCAN == (int)kItemScan && (int)P2G_ITEM_ENCODE == (int)kItemEncode &&
+                  (int)P2G_ITEM_SET_ID == (int)kItemSetId && (int)P2G_ITEM_CRC == (int)kItemCrc &&
+                  (int)P2G_ITEM_ENCODE_TENSOR == (int)kItemEncodeMma && (int)P2G_ITEM_CHAIN == (int)kItemChain,
+              "the header's item kinds");
+extern "C" p2g_status p2g_plan_device_queue(uint64_t slice_size, uint32_t input_slices, uint32_t recovery_count,
+                                            uint32_t file_count, uint32_t with_chains, uint32_t ctas,
+                                            p2g_queue_item* items, uint32_t cap, uint32_t* n_items,
+                                            uint32_t* band_items, uint32_t band_cap, uint32_t* n_bands,
+                                            double* predicted_ms) {
+    clear_error();
+    if (!ctas || !input_slices || input_slices > P2G_MAX_INPUT_BLOCKS || (cap && !items) || (band_cap && !band_items))
+        return set_error(P2G_ERR_INVALID_ARGUMENT, "plan needs ctas > 0, 1..32768 input slices and the arrays");
+    SingleJobPlan pl;
+    P2G_TRY(plan_for_report(slice_size, input_slices, recovery_count, file_count, with_chains != 0, ctas, &pl));
+    for (size_t i = 0; i < std::min<size_t>(cap, pl.items.size()); ++i) {
+        const BatchItem& it = pl.items[i];
+        const uint32_t kind = it.kind_rg & kItemKindMask;
+        p2g_queue_item& q = items[i] = {kind, 0, 0, it.a, it.b, 0, 0, 0, 0};
+        if (kind == kItemEncode || kind == kItemEncodeMma) {
+            const uint32_t height = kind == kItemEncode ? (uint32_t)kRowsPerGroup : mma_rows(recovery_count);
+            q.row = ((it.kind_rg >> 8) & 0xFFFFu) * height;
+            q.rows = std::min(height, recovery_count - q.row);
+            q.count = it.b & 0xFFFFu;
+            q.band = it.b >> 16;
+            q.first_slice = it.s0;
+            q.slices = it.sn ? it.sn : input_slices;
+            q.accumulate = (it.kind_rg & kItemAccumulate) ? 1u : 0u;
+        } else if (kind == kItemChain) {
+            q.row = it.a * kChainRows;
+            q.rows = std::min(kChainRows, recovery_count - q.row);
+            q.first = q.count = 0;
+        }
+    }
+    for (size_t b = 0; b < std::min<size_t>(band_cap, pl.band_items.size()); ++b) band_items[b] = pl.band_items[b];
+    if (n_items) *n_items = (uint32_t)pl.items.size();
+    if (n_bands) *n_bands = (uint32_t)pl.band_items.size();
+    if (predicted_ms) *predicted_ms = pl.predicted_ms;
     return P2G_OK;
 }
 

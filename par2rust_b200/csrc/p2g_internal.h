@@ -154,9 +154,8 @@ constexpr uint32_t mma_row_tiles(uint32_t R) { return R ? (R + mma_rows(R) - 1) 
 // ~148 tiles at work are then about 8 x 19, and share their coefficients (6.6
 // KB a K-step, 19 ways) and source symbols (2 KB, 8 ways) in L2.
 constexpr uint32_t kMmaRowBlock = 8;
-// The planner's unit of tensor-core work: bands and slice ranges are cut, and
-// p2g_plan_device_job reports, in units of 16 rows x 240 symbols (one M = 256 x
-// N = 240 accumulator); 15 tiles' symbols make 16 units.
+// Bands of tensor-core work are cut, and p2g_plan_device_job reports it, in
+// units of 16 rows x 240 symbols; 15 tiles' symbols make 16 units.
 constexpr uint32_t kMmaUnitSymbols = 240;
 constexpr uint32_t kMmaUnitRows = 16;
 // K-steps (4 slices) per row tile in that image: whole 16-slice stages.
@@ -264,8 +263,6 @@ struct SingleJobPlan {
     // recovery columns [zero_from_sym, Np) are written by XOR-accumulating
     // items: the caller zeroes them first (Np: none)
     uint32_t zero_from_sym = 0;
-    uint32_t split_slices = 0;  // slices of each range there
-    bool mma = false;           // the encode items are tensor-core tiles
     double predicted_ms = 0;
 };
 // file_bytes: largest file (non-zero: whole-file MD5 items, kHashFiles files each);

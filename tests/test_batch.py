@@ -155,6 +155,66 @@ def test_device_job_plan_splits_the_538mb_job(p2g, monkeypatch):
     assert len(items) == 1093 * 13 and all(it["fold"] == 0 for it in items) and bands > 1
 
 
+@pytest.mark.parametrize("variant", ["lut", "tensor"])
+@pytest.mark.parametrize("slice_,S,R", SPLIT_SHAPES + [(4, 1, 1), (7680, 17, 13), (7696, 33, 14), (262160, 64, 27)])
+def test_device_job_queue_covers_every_row_symbol_and_slice_once(p2g, monkeypatch, variant, slice_, S, R):
+    """The items as they are queued: every recovery row and symbol gets every
+    slice exactly once (tiles in cells of 8 symbols), the bands follow one
+    another in the queue and in the symbols, and each counts its own items."""
+    monkeypatch.setenv("P2G_ENCODE_VARIANT", variant)
+    items, band_items, ms = p2g.plan_device_queue(slice_, S, R)
+    _, zero_from, bands = p2g.plan_device_job(slice_, S, R)
+    Np = (slice_ + 15) // 16 * 16 // 2
+    kind = p2g.ITEM_ENCODE_TENSOR if variant == "tensor" else p2g.ITEM_ENCODE
+    enc = [it for it in items if it["kind"] == kind]
+    assert enc and ms > 0 and {it["kind"] for it in items} <= {kind, p2g.ITEM_SCAN, p2g.ITEM_SET_ID, p2g.ITEM_CRC,
+                                                               p2g.ITEM_CHAIN}
+    edges = sorted({it["row"] for it in enc}) + [R]
+    got = np.zeros((len(edges) - 1, Np // 8), np.int64)  # slices added up per row tile and cell
+    starts = {}
+    for it in enc:
+        assert edges[edges.index(it["row"]) + 1] == it["row"] + it["rows"]
+        assert it["first"] % 8 == 0 and it["count"] % 8 == 0 and 0 < it["count"]
+        assert variant == "lut" or (it["rows"] <= 13 and it["count"] <= 256 and it["first_slice"] % 16 == 0)
+        assert it["accumulate"] == (it["slices"] != S) and (not it["accumulate"] or it["first"] >= zero_from)
+        got[edges.index(it["row"]), it["first"] // 8:(it["first"] + it["count"]) // 8] += it["slices"]
+        starts.setdefault((it["row"], it["first"], it["count"], it["band"]), []).append((it["first_slice"], it["slices"]))
+    assert (got == S).all()
+    for pieces in starts.values():
+        at = 0
+        for s0, sn in sorted(pieces):
+            assert s0 == at
+            at += sn
+        assert at == S
+    assert bands == len(band_items) and [sum(it["band"] == b for it in enc) for b in range(bands)] == band_items
+    order = [it["band"] for it in enc]
+    assert order == sorted(order)
+    ends = [(min(it["first"] for it in enc if it["band"] == b), max(it["first"] + it["count"] for it in enc
+                                                                    if it["band"] == b)) for b in range(bands)]
+    assert ends[0][0] == 0 and ends[-1][1] == Np and all(a[1] == b[0] for a, b in zip(ends, ends[1:]))
+    for k, n in ((p2g.ITEM_SCAN, S), (p2g.ITEM_CRC, S)):
+        at = 0
+        for it in sorted((it for it in items if it["kind"] == k), key=lambda it: it["first"]):
+            assert it["first"] == at
+            at += it["count"]
+        assert at == n
+
+
+def test_device_job_queues_chain_items_before_the_encode(p2g, monkeypatch):
+    """One CTA for each 128 rows' packet chains where these last more than half
+    as long as the encode, and never more than a quarter of the CTAs."""
+    monkeypatch.setenv("P2G_ENCODE_VARIANT", "tensor")
+    items, _, _ = p2g.plan_device_queue(524288, 1027, 200)
+    chains = [(i, it["row"], it["rows"]) for i, it in enumerate(items) if it["kind"] == p2g.ITEM_CHAIN]
+    assert [c[1:] for c in chains] == [(0, 128), (128, 72)]
+    assert chains[-1][0] < min(i for i, it in enumerate(items) if it["kind"] == p2g.ITEM_ENCODE_TENSOR)
+    assert not any(it["kind"] == p2g.ITEM_CHAIN for it in p2g.plan_device_queue(524288, 1027, 200, with_chains=False)[0])
+    monkeypatch.setenv("P2G_ENCODE_VARIANT", "lut")
+    for rows, want in ((4736, 37), (4737, 0)):  # 37 and 38 blocks of rows on 148 CTAs
+        items, _, _ = p2g.plan_device_queue(1 << 18, 1, rows)
+        assert sum(it["kind"] == p2g.ITEM_CHAIN for it in items) == want
+
+
 def test_staged_groups_cover_jobs_in_order(p2g):
     # equal jobs: the first group gets about half of the others' share
     r = p2g.staged_groups([10] * 70, 4)
