@@ -536,6 +536,8 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     d.ts = pl.ts;
     d.first_exp = j.first_exp;
     d.vec = j.slice % 16 == 0 ? 1u : 0u;
+    const char* polls = getenv("P2G_CHAIN_POLLS");
+    d.chain_polls = polls ? (uint32_t)std::min<unsigned long>(strtoul(polls, nullptr, 10), kChainPolls) : kChainPolls;
     if (mma) {
         d.mma = 1;
         d.aimg = c.aimg.as<uint8_t>();

@@ -196,6 +196,7 @@ constexpr uint32_t kScanSlices = 256;
 constexpr uint32_t kLoneScanSlices = 128;
 constexpr uint32_t kHashFiles = 128;         // files per whole-file MD5 item
 constexpr uint32_t kChainRows = 128;         // recovery rows per packet-MD5 chain token
+constexpr uint32_t kChainPolls = 1u << 20;   // polls of a chain item, ~0.5 us each
 constexpr uint32_t kCrcMaxSlices = 256;      // slices per CRC32 item
 
 // Encode item fields: kind_rg = kItemEncode | acc | rg << 8 | log2(fold) << 24;
@@ -249,6 +250,7 @@ struct BatchJob {
     uint32_t ts, first_exp;  // ts: tile width (sub-tile width of folded items)
     uint32_t vec;            // slices and file starts of src are 16-byte aligned
     uint32_t mma;            // encode items run on the tensor cores (kItemEncodeMma)
+    uint32_t chain_polls;    // polls of a chain item for the next band
     uint8_t* aimg;           // mma: the coefficient image (mma_aimg_bytes)
     uint32_t rows, ksteps;   // mma: recovery rows per row tile (mma_rows); the image's K-steps per tile
     CUtensorMap src_map;     // mma: esrc as a 2-D tensor (make_src_map); 64-byte aligned

@@ -1255,9 +1255,11 @@ __global__ void gather_host_kernel(const uint64_t* __restrict__ seg, uint32_t n_
 
 // ---------------------------------------------------------------------------
 // Batched create.  One CTA per SM pops work items off a device queue until
-// it is empty.  Items of one job never wait for one another: the CTA whose
-// encode item completes a job (counted with an atomic after a release fence)
-// runs that job's finish step itself, so the launch has no inter-CTA waits.
+// it is empty.  The CTA whose encode item completes a band of its job (counted
+// with an atomic after a release fence) advances the job's packet chains
+// itself, so no item has to wait for another, but for the chain items of a lone
+// job: each keeps one CTA, which polls a bounded number of times for the bands
+// that the others complete, and then leaves the chains to them.
 //
 // Shared memory: the encode region (tables, TMA ring, mbarriers), a cp.async
 // ring of kBatchRingLane bytes for each of the kHashThreadsWide MD5 lanes, the
@@ -1650,10 +1652,11 @@ __device__ uint32_t advance_ready(const BatchJob& J, uint32_t q, uint32_t ring, 
 // Take block q's chain token if it is free and advance its rows over every
 // band that is ready, in order; after releasing the token, look once more
 // (a band that became ready while the token was held was left to us).  Each
-// pass either advances at least one band or returns, so this ends.  No CTA
-// waits for another: a busy token means its holder will see the new band.
+// pass either advances at least one band or returns, so this ends.  A busy
+// token is not waited for: its holder will see the new band.
 // polls > 0: keep the token and look up to that many times, ~0.5 us apart, for
-// the next band, until the last one is done (the chain items).
+// the next band, until the last one is done (the chain items); when the polls
+// run out the block goes back to the CTAs that complete its bands.
 template <int UNITS, int AHEAD>
 __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32_t* misc, uint32_t polls = 0,
                             const int* err = nullptr) {
@@ -1694,10 +1697,6 @@ __device__ void try_advance(const BatchJob& J, uint32_t q, uint32_t ring, uint32
         if (!again) return;
     }
 }
-
-// Polls of a chain item (~1 s); when they run out the block goes back to the
-// CTAs that complete its bands.
-constexpr uint32_t kChainPolls = 1u << 20;
 
 // All row blocks, starting with block `first` mod Q: the CTAs that complete
 // neighbouring bands start on different blocks, so that the blocks advance
@@ -1811,7 +1810,7 @@ __global__ void __launch_bounds__(kEncThreads, 1)
         if (kind == kItemChain) {
             // this CTA keeps block it.a's chains until the last band (the
             // other MD5 items' ring: no tensor-core stage is in flight here)
-            try_advance<kRingUnits, kRingAhead>(J, it.a, ring, misc, kChainPolls, err);
+            try_advance<kRingUnits, kRingAhead>(J, it.a, ring, misc, J.chain_polls, err);
             continue;
         }
         if (kind == kItemPacket) {

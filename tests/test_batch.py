@@ -510,3 +510,33 @@ def test_planner_picks_the_encode_kernel_by_shape(p2g, monkeypatch, slice_, S, R
     items, _, _ = p2g.plan_device_job(slice_, S, R)
     got = "tensor" if items[0]["fold"] == 0 else "lut"
     assert got == want, (slice_, S, R, got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", ["lut", "tensor"])
+@pytest.mark.parametrize("polls", ["0", "1", "7", "300", None])
+def test_chain_items_that_stop_polling(p2g, gpu, monkeypatch, variant, polls):
+    """A chain item that gives up hands its rows' packet chains to the CTAs that
+    complete the bands, wherever the chains stand by then."""
+    import hashlib
+
+    import torch
+
+    monkeypatch.setenv("P2G_ENCODE_VARIANT", variant)
+    if polls is not None:
+        monkeypatch.setenv("P2G_CHAIN_POLLS", polls)
+    S, slice_, R = 64, 65536, 300  # three blocks of rows
+    items, band_items, _ = p2g.plan_device_queue(slice_, S, R)
+    assert sum(it["kind"] == p2g.ITEM_CHAIN for it in items) == 3 and len(band_items) > 4
+    src = torch.from_numpy(file_bytes(77, S * slice_).copy()).cuda()
+    bufs = p2g.run_device_job(src, [S * slice_], [b"f"], slice_, R, skip_hash_full=True)
+    torch.cuda.synchronize()
+    rec = bufs.recovery.view(-1, bufs.rec_stride)[:R, :slice_]
+    want = torch.zeros_like(rec)
+    p2g.encode_device(src.data_ptr(), slice_, S, slice_, R, want.data_ptr(), slice_,
+                      torch.cuda.current_stream().cuda_stream, wait=True)
+    assert torch.equal(rec, want)
+    sid, got = bufs.set_id, bufs.packet_md5.cpu().numpy().tobytes()
+    for r, row in enumerate(rec.cpu().numpy()):
+        head = sid + b"PAR 2.0\0RecvSlic" + r.to_bytes(4, "little")
+        assert got[16 * r:16 * r + 16] == hashlib.md5(head + row.tobytes()).digest(), r
