@@ -536,8 +536,6 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     d.ts = pl.ts;
     d.first_exp = j.first_exp;
     d.vec = j.slice % 16 == 0 ? 1u : 0u;
-    const char* polls = getenv("P2G_CHAIN_POLLS");
-    d.chain_polls = polls ? (uint32_t)std::min<unsigned long>(strtoul(polls, nullptr, 10), kChainPolls) : kChainPolls;
     if (mma) {
         d.mma = 1;
         d.aimg = c.aimg.as<uint8_t>();
@@ -581,9 +579,12 @@ static p2g_status run_device_job_persistent(Context& c, DeviceJob& j, cudaStream
     if (mma)
         P2G_CU(launch_a_image_batch(reinterpret_cast<const BatchJob*>(D + o_desc), 1, mma_aimg_bytes(j.S, j.R), st));
     if (esrc != j.d_src) P2G_CU(launch_realign(j.d_src, j.slice, c.src_al.as<uint8_t>(), estride, j.S, j.slice, st));
+    const char* polls = getenv("P2G_CHAIN_POLLS");
     P2G_CU(launch_batch(reinterpret_cast<const BatchJob*>(D + o_desc), reinterpret_cast<const BatchItem*>(D + o_items),
                         (uint32_t)pl.items.size(), reinterpret_cast<uint32_t*>(D + o_ctl), err,
-                        (uint32_t)device_sm_count(), st, mma));
+                        (uint32_t)device_sm_count(), st, mma,
+                        polls ? (uint32_t)std::min<unsigned long>(strtoul(polls, nullptr, 10), kChainPolls)
+                              : kChainPolls));
     P2G_CU(cudaMemcpyAsync(c.h_err.p, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     P2G_CU(cudaEventRecord(c.ev_scratch, st));
     c.scratch_pending = true;

@@ -250,7 +250,6 @@ struct BatchJob {
     uint32_t ts, first_exp;  // ts: tile width (sub-tile width of folded items)
     uint32_t vec;            // slices and file starts of src are 16-byte aligned
     uint32_t mma;            // encode items run on the tensor cores (kItemEncodeMma)
-    uint32_t chain_polls;    // polls of a chain item for the next band
     uint8_t* aimg;           // mma: the coefficient image (mma_aimg_bytes)
     uint32_t rows, ksteps;   // mma: recovery rows per row tile (mma_rows); the image's K-steps per tile
     CUtensorMap src_map;     // mma: esrc as a 2-D tensor (make_src_map); 64-byte aligned
@@ -307,9 +306,9 @@ double est_packet_item_ms(uint64_t slice, uint32_t rows);
 // Sets the batch kernel's shared-memory attribute (call before stream capture).
 cudaError_t prepare_batch_kernel();
 // mma: the batch has tensor-core encode items (the CTAs allocate TMEM) and no
-// lookup ones.
+// lookup ones.  chain_polls: of a chain item for the next band.
 cudaError_t launch_batch(const BatchJob* jobs, const BatchItem* items, uint32_t n_items, uint32_t* ctl, int* err,
-                         uint32_t ctas, cudaStream_t st, bool mma = false);
+                         uint32_t ctas, cudaStream_t st, bool mma = false, uint32_t chain_polls = kChainPolls);
 // One-time set-up of the tensor-core tables on this device.
 cudaError_t mma_prepare();
 // Fills every tensor-core job's coefficient image (blockIdx.y = job); max_bytes: the
