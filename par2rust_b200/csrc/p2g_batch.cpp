@@ -45,6 +45,7 @@ constexpr double kFoldCost = 1.15, kAccCost = 1.04;
 // simulation: the model is good to a few percent, and smaller pieces cost
 // more in ways it does not see.
 constexpr double kPlanMargin = 0.97;
+constexpr double kZeroMs = 0.01, kZeroRate = 7e9;  // zeroing the columns of split bands: a memset, bytes per ms
 constexpr double kItemMs = 0.003;          // pop, descriptor loads, pipeline fill
 
 inline uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
@@ -119,9 +120,11 @@ void job_bands(const PlanJob& j, uint32_t* band_tiles, uint32_t* n_bands) {
     *band_tiles = bt;
     *n_bands = (j.tiles + bt - 1) / bt;
 }
-// one chain segment of every kChainRows-row block over one band's bytes
-inline double chain_ms(const PlanJob& j, uint32_t band_syms) {
-    return ceil(j.R / (double)kChainRows) * md5_ms(2ull * band_syms) * 1.07 + kItemMs;
+// one chain segment of every kChainRows-row block over one band's bytes: the
+// blocks one after the other on the CTA that completed the band, or side by
+// side on the CTAs of the job's chain items (held)
+inline double chain_ms(const PlanJob& j, uint32_t band_syms, bool held = false) {
+    return (held ? 1.0 : ceil(j.R / (double)kChainRows)) * md5_ms(2ull * band_syms) * 1.07 + kItemMs;
 }
 
 // Slices of one of C ranges of a job; tensor-core ranges start on whole
@@ -253,7 +256,7 @@ double item_ms(const PlanJob& j, const BatchItem& it) {
     case kItemScan: return scan_ms(j, it.b);
     case kItemCrc: return est_crc_item_ms(j.slice, it.b);
     case kItemFileHash: return md5_ms(j.file_bytes) + kItemMs;
-    case kItemChain: return md5_ms(j.slice + 36) + kItemMs;
+    case kItemChain: return 0;  // its segments are counted band by band
     case kItemEncodeMma:
         return est_mma_item_ms(it.sn ? it.sn : j.S, mma_rows(j.R)) * ((it.kind_rg & kItemAccumulate) ? kAccCost : 1.0);
     case kItemEncode: {
@@ -268,20 +271,28 @@ double item_ms(const PlanJob& j, const BatchItem& it) {
 
 // List-scheduling simulation: each item goes to the CTA that frees first.
 // A job's packet chains advance band by band in order: band b's segment
-// starts when the band's last item ends and the previous segment is done.
+// starts when the band's last item ends and the previous segment is done, the
+// first one not before the set id, which the packets begin with.
 // (The advancing CTA's time is charged to it when the chain was waiting for
 // that band; a band that completes while the chain is busy is picked up by
-// the chain's holder.)
+// the chain's holder.)  The CTA of a chain item takes nothing else until the
+// last band, that is, to the end.
 double simulate(const std::vector<PlanJob>& jobs, const Plan& p, uint32_t ctas) {
     std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
     for (uint32_t c = 0; c < ctas; ++c) free_at.push(0.0);
     std::vector<std::vector<uint32_t>> left = p.band_items;
     std::vector<std::vector<double>> done(jobs.size());
     for (size_t ji = 0; ji < jobs.size(); ++ji) done[ji].assign(p.band_items[ji].size(), 0.0);
+    std::vector<bool> held(jobs.size(), false);
+    std::vector<double> sid(jobs.size(), 0.0);
     double end = 0;
     for (const BatchItem& it : p.items) {
         double t = free_at.top();
         free_at.pop();
+        if ((it.kind_rg & kItemKindMask) == kItemChain) {  // at most a quarter of the CTAs
+            held[it.job] = true;
+            continue;
+        }
         const PlanJob& j = jobs[it.job];
         t += item_ms(j, it);
         const uint32_t kd = it.kind_rg & kItemKindMask;
@@ -290,12 +301,13 @@ double simulate(const std::vector<PlanJob>& jobs, const Plan& p, uint32_t ctas) 
             done[it.job][b] = std::max(done[it.job][b], t);
             --left[it.job][b];
         }
+        if (kd == kItemSetId) sid[it.job] = t;
         end = std::max(end, t);
         free_at.push(t);
     }
     for (size_t ji = 0; ji < jobs.size(); ++ji) {
-        double chain = 0;
-        for (double d : done[ji]) chain = std::max(chain, d) + chain_ms(jobs[ji], p.band_syms[ji]);
+        double chain = sid[ji];
+        for (double d : done[ji]) chain = std::max(chain, d) + chain_ms(jobs[ji], p.band_syms[ji], held[ji]);
         end = std::max(end, chain);
     }
     return end;
@@ -328,7 +340,8 @@ Plan plan_batch(std::vector<PlanJob>& jobs, uint32_t ctas, uint32_t flags) {
             j.split_bands = std::min(bands, nb);
             j.split_chunks = chunks;
             Plan p = build_items(jobs, ctas);
-            p.makespan = simulate(jobs, p, ctas);
+            const uint32_t zero_from = (nb - j.split_bands) * p.band_syms[0];
+            p.makespan = simulate(jobs, p, ctas) + kZeroMs + 2.0 * (j.Np - std::min(j.Np, zero_from)) * j.R / kZeroRate;
             if (p.makespan < best.makespan * kPlanMargin) {
                 best = std::move(p);
                 bb = j.split_bands;
@@ -468,7 +481,7 @@ double est_scan_item_ms(uint64_t slice, uint32_t count) {
 // CRC32 streams from DRAM at ~35 GB/s per SM (16 warps)
 double est_crc_item_ms(uint64_t slice, uint32_t count) { return (double)slice * count / 3.5e7 + kItemMs; }
 double est_set_id_ms(uint32_t files) {
-    const double hashes = ceil(files / 256.0) * (md5_ms(P2G_HASH16K_LEN) * kWideChain + md5_ms(24 + 256));
+    const double hashes = ceil(files / 256.0) * (md5_ms(P2G_HASH16K_LEN) * (files > 128 ? kWideChain : 1.0) + md5_ms(24 + 256));
     const double sort = (double)files * files / 512.0 * 4e-6;
     return hashes + sort + md5_ms(12 + 16ull * files) + kItemMs;
 }

@@ -215,6 +215,19 @@ def test_device_job_queues_chain_items_before_the_encode(p2g, monkeypatch):
         assert sum(it["kind"] == p2g.ITEM_CHAIN for it in items) == want
 
 
+def test_chain_items_of_a_plan_run_side_by_side(p2g, monkeypatch):
+    """The planner's time for a job with chain items: their blocks of 128 rows
+    advance together, each on a CTA of its own (the 538 MB job takes 4.47 ms)."""
+    monkeypatch.setenv("P2G_ENCODE_VARIANT", "tensor")
+    one, two = (p2g.plan_device_queue(524288, 64, R)[2] for R in (128, 256))  # one chain: 3.6 ms
+    assert one > 3.6 and two - one < 0.5
+    assert abs(p2g.plan_device_queue(524288, 1027, 200)[2] - 4.47) < 0.45
+    # their CTAs encode nothing: 2 of 8 here, of a job bound by its encode
+    items, _, ms = p2g.plan_device_queue(524288, 16, 129, ctas=8)
+    assert sum(it["kind"] == p2g.ITEM_CHAIN for it in items) == 2
+    assert ms >= p2g.plan_device_queue(524288, 16, 129, ctas=6, with_chains=False)[2]
+
+
 def test_staged_groups_cover_jobs_in_order(p2g):
     # equal jobs: the first group gets about half of the others' share
     r = p2g.staged_groups([10] * 70, 4)
