@@ -10,7 +10,7 @@
 // Autotuning.  Items are popped in a fixed order by whichever CTA is free,
 // so the launch is list scheduling.  The planner simulates it with a cost
 // model (per-slice encode cost ~ tile + 384 shared-memory wavefronts at 78%
-// of peak, ~0.72 us per 64-byte MD5 block of a chain) for the queue order
+// of peak, kChainMs per 64-byte MD5 block of a chain) for the queue order
 // "longest item + tail first", then searches each large job's tile width
 // (1x, 2x, 4x, 8x its minimum tile count) for the shortest simulated makespan.
 #include <cuda_runtime.h>

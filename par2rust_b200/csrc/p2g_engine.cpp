@@ -670,14 +670,14 @@ static p2g_status run_device_job(Context& c, DeviceJob& j, cudaStream_t caller) 
             esrc = c.src_al.as<uint8_t>();
         }
         // slice-MD5 (and device whole-file MD5) blocks each hold an SM for
-        // about chain-length x 0.72 us per 64-byte block
+        // their longest chain
         uint32_t reserve = hash_blocks(j.d_checks ? j.S : 0) + hash_blocks(j.d_h16k ? n : 0);
-        double reserve_ms = j.d_checks ? (double)(j.slice / 64) * 7.2e-4 : 0.0;
+        double reserve_ms = j.d_checks ? est_md5_ms(j.slice) : 0.0;
         if (j.d_hfull) {
             uint64_t mx = 0;
             for (const auto& f : j.files) mx = std::max(mx, f.length);
             reserve += hash_blocks(n);
-            reserve_ms = std::max(reserve_ms, (double)(mx / 64) * 7.2e-4);
+            reserve_ms = std::max(reserve_ms, est_md5_ms(mx));
         }
         plan = plan_encode(j.slice, j.S, RG, j.d_pkt != nullptr, reserve, reserve_ms, tail_fold(j.R));
         if (plan.bands.size() > (size_t)Context::kBandEvents)

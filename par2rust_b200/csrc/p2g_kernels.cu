@@ -2091,7 +2091,7 @@ EncodePlan plan_encode(uint64_t slice_size, uint32_t S, uint32_t RG, bool banded
         if (unfolded.bands.size() > 1) return unfolded;
         return c;
     }
-    const double chain_ms_per_byte = 7.2e-4 / 64;  // one MD5 chain: ~0.72 us per 64-byte block
+    const double chain_ms_per_byte = est_md5_ms(1u << 20) / (1u << 20);
     const uint32_t waves1 = (uint32_t)((eff_ctas(t1, RG, fold) + sms - 1) / sms);
     const double ms_c = est_band_ms(S, ts1, waves1) + 2.0 * pl.Np * chain_ms_per_byte + reserve_ms;
     auto tail = [&](const EncodePlan& p) {  // last band's packet-MD5 step + per-band launch/drain
