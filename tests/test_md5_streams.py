@@ -77,6 +77,27 @@ def test_file_streams_of_mixed_lengths(p2g, gpu):
     assert got[16 * n:] == b"".join(hashlib.md5(d[:16384]).digest() for d in data)
 
 
+@pytest.mark.parametrize("pitch", [40960, 40976])
+def test_file_streams_that_all_start_16_byte_aligned(p2g, gpu, pitch):
+    """The unshifted ring of device-pointer file hashes, lanes of different lengths."""
+    import torch
+
+    lengths = [1, 63, 64, 65, 575, 576, 577, 767, 768, 16383, 16384, 16385, 40001] * 11
+    src = _device(len(lengths) * pitch, pitch)
+    n = len(lengths)
+    ptrs = (C.c_void_p * n)(*[src.data_ptr() + i * pitch for i in range(n)])
+    assert all(p % 16 == 0 for p in ptrs)
+    lens = (C.c_uint64 * n)(*lengths)
+    out = torch.zeros(32 * n, dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    assert p2g.lib().p2g_file_hashes(ptrs, lens, n, out.data_ptr(), out.data_ptr() + 16 * n, p2g.DEVICE_POINTERS,
+                                     st) == 0
+    host = src.cpu().numpy()
+    data = [host[i * pitch:i * pitch + k].tobytes() for i, k in enumerate(lengths)]
+    assert out.cpu().numpy().tobytes() == b"".join(hashlib.md5(d).digest() for d in data) + b"".join(
+        hashlib.md5(d[:16384]).digest() for d in data)
+
+
 # around 1, 2, 3, 4 and more fold groups of 1,024 B; around 2, 4, 8 and 16 parts of a slice (16 KiB each at least)
 CRC_SIZES = [(3, 1020), (3, 1024), (3, 1028), (2, 2048), (2, 2052), (5, 3076), (4, 4092), (4, 4100), (1, 32764),
              (17, 32768), (2, 32772), (3, 65540), (1, 131076), (9, 262144), (2, 262148), (1, 1048580), (2400, 1032)]
