@@ -1,11 +1,12 @@
 // p2g_batch.cpp -- batched create: many independent create jobs in one
 // persistent, graph-captured launch (p2g_batch_* in include/par2gpu.h).
 //
-// Planning.  Each job becomes work items: scan items (slice MD5 + CRC32 of
-// up to kScanSlices slices), encode items (one row group x one symbol tile
-// over all of the job's input slices) and, for a job without recovery rows,
-// one finish item.  A job's finish step (hash16k, file ids, set id, packet
-// MD5s) runs on the CTA that completes its last encode item.
+// Planning.  Each job becomes work items: a set-id item (hash16k, file ids, set
+// id), scan items (slice MD5 of up to kScanSlices slices), CRC32 items, whole-
+// file MD5 items where wanted, and encode items (one row group or row tile x one
+// symbol tile over the job's input slices or a range of them).  The packet-MD5
+// chains run band by band on the CTAs that complete the job's bands, or, for a
+// job alone, on the CTAs of its chain items.
 //
 // Autotuning.  Items are popped in a fixed order by whichever CTA is free,
 // so the launch is list scheduling.  The planner simulates it with a cost
@@ -829,11 +830,11 @@ extern "C" p2g_status p2g_batch_create(const p2g_batch_job* jobs, uint32_t n, ui
     }
     // One encode kernel for the whole launch: forced by the flags (or
     // P2G_ENCODE_VARIANT), else the one the cost model prefers for the
-    // batch's total encode work.  Lookup and tensor-core items are not mixed
-    // in one launch: mixed launches gave wrong recovery bytes for a few
-    // tensor-core tiles, and with the proxy fences between item kinds a
-    // 256-job mixed launch still ran into a bounded wait (each kind alone is
-    // bit-exact).
+    // batch's total encode work.  Lookup and tensor-core items are not mixed in
+    // one launch, whose shared memory is laid out for one kind: where an earlier
+    // form mixed them, a lookup item's mbarriers lay inside a tensor input stage
+    // and were not invalidated before copies went there, which gave wrong tiles
+    // and waits that ran out.
     const char* ev = getenv("P2G_ENCODE_VARIANT");
     bool use_mma, by_cost = false;
     if (flags & P2G_BATCH_TENSOR) {

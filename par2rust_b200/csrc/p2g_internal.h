@@ -220,9 +220,7 @@ struct BatchItem {
     uint32_t s0, sn;   // encode: input slices [s0, s0+sn) (sn == 0: all of the job's)
 };
 
-// Device descriptor of one job.  The CTA that completes a job's last encode
-// item (or runs its finish item) also derives the job's hash16k values, file
-// ids, set id and recovery-packet MD5s.
+// Device descriptor of one job.
 struct BatchJob {
     const uint8_t* src;        // files back to back, each on a slice boundary, zero-padded
     const uint8_t* esrc;       // encode source: src, or a copy with 16-byte aligned slices
@@ -277,8 +275,6 @@ SingleJobPlan plan_single_job(uint64_t slice, uint32_t S, uint32_t R, uint32_t n
 size_t batch_smem_bytes();
 // Fills every job's basis (one launch; blockIdx.y = job).
 cudaError_t launch_basis_batch(const BatchJob* jobs, uint32_t n_jobs, uint64_t max_words, cudaStream_t st);
-// The persistent kernel: `ctas` CTAs; ctl[0] queue head, ctl[1+j] completed
-// encode items of job j (zeroed before each launch).
 // Seeded synthetic files (3 words per file in `spans`: offset, length,
 // padded length; one seed per file), blockIdx.y = file.
 cudaError_t launch_seeded_fill(uint8_t* base, const uint64_t* spans, const uint64_t* seeds, uint32_t n_files,
@@ -305,6 +301,8 @@ double est_set_id_ms(uint32_t files);
 double est_packet_item_ms(uint64_t slice, uint32_t rows);
 // Sets the batch kernel's shared-memory attribute (call before stream capture).
 cudaError_t prepare_batch_kernel();
+// The persistent kernel on `ctas` CTAs.  ctl[0]: the queue head; the jobs' chain
+// state (bstate) and the error word follow, all zeroed before each launch.
 // mma: the batch has tensor-core encode items (the CTAs allocate TMEM) and no
 // lookup ones.  chain_polls: of a chain item for the next band.
 cudaError_t launch_batch(const BatchJob* jobs, const BatchItem* items, uint32_t n_items, uint32_t* ctl, int* err,
