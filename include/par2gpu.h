@@ -240,7 +240,8 @@ p2g_status p2g_gf_mul_xor(uint16_t coeff, const uint8_t *input, uint8_t *output,
  * call waits on `stream` for the previous device-pointer call's use of the
  * library's scratch (coefficient tables, error word), whatever its stream
  * (not while `stream` is being captured into a graph: captured calls must
- * not overlap other device-pointer encodes).
+ * not overlap other device-pointer encodes; the scratch they use stays
+ * allocated for the graph's replays).
  * Device rows are read and written in whole 16-byte units: bytes
  * [slice_size, round_up(slice_size, 16)) of every source row are read --
  * for the last row too, so src must be readable up to

@@ -53,15 +53,18 @@ constexpr uint64_t kGatherSegBytes = 4ull << 20;
 constexpr uint64_t kUploadChunk = 1ull << 20, kUploadSlots = 8;
 constexpr uint64_t kUploadMin = 1ull << 20;  // smaller ones: one copy of the driver's
 
-// Grow-only device buffer.
+// Grow-only device buffer.  One that a stream capture has used is not freed when
+// it grows: the graph may be replayed at any time.
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
+    bool captured = false;
     cudaError_t ensure(size_t n) {
         if (n <= cap && p) return cudaSuccess;
-        if (p) cudaFree(p);
+        if (p && !captured) cudaFree(p);
         p = nullptr;
         cap = 0;
+        captured = false;
         const size_t want = std::max<size_t>(round_up(n, 1 << 20), 1 << 20);
         cudaError_t e = cudaMalloc(&p, want);
         if (e == cudaSuccess) cap = want;
@@ -253,7 +256,7 @@ static p2g_status ensure_image(Context& c, size_t bytes, Forced forced, bool* ot
     size_t left = 0, total = 0;
     P2G_CU(cudaMemGetInfo(&left, &total));
     cudaError_t e = cudaErrorMemoryAllocation;
-    if (forced != Forced::No || left + c.aimg.cap >= bytes) e = c.aimg.ensure(bytes);
+    if (forced != Forced::No || left + (c.aimg.captured ? 0 : c.aimg.cap) >= bytes) e = c.aimg.ensure(bytes);
     if (e == cudaErrorMemoryAllocation && forced == Forced::No) {
         cudaGetLastError();
         *other = true;
@@ -1383,6 +1386,8 @@ extern "C" p2g_status p2g_encode(const p2g_encode_job* job) {
         if (order) {
             P2G_CU(cudaEventRecord(c.ev_scratch, s));
             c.scratch_pending = true;
+        } else {
+            (tensor ? c.aimg : c.basis).captured = true;
         }
         if (jb.flags & P2G_ENCODE_WAIT) {
             P2G_CU(cudaMemcpyAsync(c.h_err.p, c.err.p, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -89,6 +89,36 @@ def test_capture_after_one_kernel_ran(p2g, gpu, warm, S, size, rows):
     """ % (S, size, rows, warm))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", ["LUT", "TENSOR"])
+def test_replay_after_the_scratch_grew(p2g, gpu, kernel):
+    """A captured call's scratch outlives its growth by later calls: here it
+    grows twice, and what a free would have given back is overwritten."""
+    _run("""
+        S, size, rows = 64, 16384, 20
+        kw = dict(variant=p2g.ENCODE_%s)
+        data = file_bytes(2, S * size)
+        src = torch.from_numpy(data.copy()).cuda()
+        encode(src, S, size, rows, **kw)
+        g = torch.cuda.CUDAGraph()
+        rec = torch.zeros((rows, size), dtype=torch.uint8, device="cuda")
+        with torch.cuda.graph(g):
+            p2g.encode_device(src.data_ptr(), size, S, size, rows, rec.data_ptr(), size,
+                              torch.cuda.current_stream().cuda_stream, **kw)
+        want = oracle.encode_fast(data, S, size, rows)
+        for S2, rows2 in ((1024, 100), (2048, 200)):
+            big = file_bytes(3, S2 * 512)
+            got = encode(torch.from_numpy(big.copy()).cuda(), S2, 512, rows2, **kw)
+            hogs = [torch.full((1 << 20,), 0xAB, dtype=torch.uint8, device="cuda") for _ in range(64)]
+            rec.zero_()
+            g.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(rec.cpu().numpy().ravel(), want)
+            assert np.array_equal(got.cpu().numpy().ravel(), oracle.encode_fast(big, S2, 512, rows2))
+            assert all(bool((h == 0xAB).all()) for h in hogs)
+    """ % kernel)
+
+
 FULL = """
     S, size, rows = 32768, 64, 512  # image 2.2 GB, bases 0.5 GB
     data = file_bytes(2, S * size)
